@@ -1449,6 +1449,137 @@ int enqueue(gw_voxel_plan *P) {
 }  // namespace
 
 
+namespace {
+
+// Gather binning: where it applies and the pixel store fits the budget
+// (GW_GATHER_MAX_MB, default 8192), its tables and store.  The column and
+// row tables of the plan are made.
+int gather_setup(gw_voxel_plan *P) {
+  size_t &B = P->bytes;
+  const size_t g_bytes = (size_t)P->n_slices * P->Nf * P->Nr * sizeof(float);
+  const char *env = getenv("GW_GATHER_MAX_MB");
+  const size_t cap = (env ? (size_t)std::max(0L, atol(env)) : (size_t)8192) << 20;
+  // (and fewer than 2^31 pixels: the gather addresses them with 32 bits)
+  const bool can = !P->plain && P->p.accum == GW_ACCUM_FP64 && !P->fused_z &&
+                   g_bytes <= cap && g_bytes / sizeof(float) < ((size_t)1 << 31);
+  if (P->p.binning == GW_BINNING_GATHER && !can) {
+    return gw::fail(GW_ERR_ARG, "gw_voxel_plan_create: gather binning needs a batched, "
+                                "float64-accumulating plan without the fused column "
+                                "kernel, and a pixel store within GW_GATHER_MAX_MB");
+  }
+  // auto: gather for one structure on real grids whose float64 sum grid
+  // is larger than L2 -- each atomic is then a DRAM read-modify-write and
+  // the grid's clearing a DRAM pass, while each stored pixel serves two
+  // voxels (its mirror) -- measured faster there (si-100A) and slower
+  // with the grid in L2, several structures (the gather loops over the
+  // structures of every entry) or complex grids (lamellar-200A)
+  const size_t sum_bytes = P->sum_stride * P->n_out * sizeof(double);
+  const bool want = P->p.binning == GW_BINNING_GATHER ||
+                    (P->p.binning == GW_BINNING_AUTO && P->real && P->n_struct == 1 &&
+                     sum_bytes > P->ctx->l2_bytes);
+  if (want && can) {
+    // the line entries, in table order (phi, band column): counting sort
+    // by window line
+    std::vector<int> cof((size_t)P->n_phi * P->Nc), rowofs(P->Nr);
+    GW_CUDA(cudaMemcpy(cof.data(), P->d_colofs, cof.size() * sizeof(int),
+                       cudaMemcpyDeviceToHost));
+    GW_CUDA(cudaMemcpy(rowofs.data(), P->d_rowofs, rowofs.size() * sizeof(int),
+                       cudaMemcpyDeviceToHost));
+    const int W = P->W;
+    std::vector<int> lptr((size_t)W * W + 1, 0);
+    for (int co : cof)
+      if (co >= 0) ++lptr[co / W + 1];
+    for (size_t i = 1; i < lptr.size(); ++i) lptr[i] += lptr[i - 1];
+    std::vector<int2> lent(std::max(lptr.back(), 1));
+    std::vector<int> fill(lptr.begin(), lptr.end() - 1);
+    for (int q = 0; q < P->n_phi; ++q)
+      for (int m = 0; m < P->Nc; ++m) {
+        const int co = cof[(size_t)q * P->Nc + m];
+        if (co < 0) continue;
+        // F1 column of table column m: itself, or with real grids its
+        // mirror's (rows mirrored) below m_zero
+        int j = m, flip = 0;
+        if (P->real) {
+          if (m >= P->m_zero) j = m - P->m_zero;
+          else { j = P->m_zero - m; flip = 1; }
+        }
+        lent[fill[co / W]++] = make_int2(q, 2 * j + flip);
+      }
+    // output rows of every window z, ascending
+    std::vector<int> zptr((size_t)W + 1, 0);
+    for (int ro : rowofs)
+      if (ro >= 0) ++zptr[ro + 1];
+    for (int i = 1; i <= W; ++i) zptr[i] += zptr[i - 1];
+    std::vector<int> zrows(std::max(zptr.back(), 1));
+    std::vector<int> zfill(zptr.begin(), zptr.end() - 1);
+    for (int mr = 0; mr < P->Nr; ++mr)
+      if (rowofs[mr] >= 0) zrows[zfill[rowofs[mr]]++] = mr;
+    // window z with more than one output row
+    std::vector<int> zmulti;
+    for (int z = 0; z < W; ++z)
+      if (zptr[z + 1] - zptr[z] > 1) zmulti.push_back(z);
+    P->n_zmulti = (int)zmulti.size();
+    if (zmulti.empty()) zmulti.push_back(0);
+    // lines with more than kGatherHeavy pixels per voxel (entries times
+    // the structures each output sums; near the rotation axis)
+    const int per_entry = P->p.average == GW_STRUCTS_SEPARATE ? 1 : P->n_struct;
+    std::vector<int> heavy;
+    for (int l = 0; l < W * W; ++l)
+      if ((int64_t)(lptr[l + 1] - lptr[l]) * per_entry > kGatherHeavy) heavy.push_back(l);
+    P->n_heavy = (int)heavy.size();
+    P->h_heavy = heavy;
+    if (heavy.empty()) heavy.push_back(0);
+    GW_TRY(upload(&P->d_heavy, heavy, &B));
+    GW_TRY(upload(&P->d_zmulti, zmulti, &B));
+    GW_TRY(upload(&P->d_lptr, lptr, &B));
+    GW_TRY(upload(&P->d_lent, lent, &B));
+    GW_TRY(upload(&P->d_zptr, zptr, &B));
+    GW_TRY(upload(&P->d_zrows, zrows, &B));
+    GW_TRY(alloc(&P->d_G, g_bytes / sizeof(float), &B));
+    P->gather = true;
+  }
+  return GW_OK;
+}
+
+}  // namespace
+
+// Per-shell f values and the adjoint need the general path: a plan made with
+// real_grids refuses them where its window is at most half the transform
+// buffer.  A wider window takes them (such plans run them on the general
+// path): the plan leaves the real path for good.
+int gwv::leave_real(gw_voxel_plan *P, const char *who) {
+  if (!P->real) return GW_OK;
+  if (2 * P->Ly <= fft_ldm(P->My))
+    return gw::fail(GW_ERR_STATE, std::string(who) + ": the plan was made with real_grids; "
+                                  "per-shell f values and the adjoint need real_grids 0");
+  GW_CUDA(cudaSetDevice(P->ctx->device));
+  if (P->executed && gathering(P)) {
+    // the last execute's results that are made on request, from its pixels
+    GW_TRY(enqueue_finalize(P, true));
+    P->iq64_valid = true;
+    for (int t = 0; t < P->n_out; ++t) GW_TRY(enqueue_gather(P, 2, t));
+  }
+  GW_CUDA(cudaStreamSynchronize(P->ctx->stream));  // no pass reads the buffers
+  if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
+  if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
+  float2 *f1 = nullptr;
+  GW_TRY(alloc(&f1, (size_t)P->S * P->Lz * P->Nc, &P->bytes));
+  void *drop[] = {P->d_F1, P->d_pr, P->d_heavy, P->d_zmulti, P->d_lptr, P->d_lent,
+                  P->d_zptr, P->d_zrows, P->d_G};
+  for (void *q : drop) gw::dev_free(q);
+  P->d_F1 = f1;
+  P->d_pr = nullptr;
+  P->d_heavy = P->d_zmulti = P->d_lptr = P->d_zptr = P->d_zrows = nullptr;
+  P->d_lent = nullptr;
+  P->d_G = nullptr;
+  P->gather = false;
+  P->n_heavy = P->n_zmulti = 0;
+  P->real = false;
+  P->Nf = P->Nc;
+  GW_TRY(col_map_dispatch(P));
+  return gather_setup(P);
+}
+
 extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
                                     const gw_structure *structs,
                                     int32_t n_struct, const gw_phi *phis,
@@ -1638,10 +1769,13 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
     delete P;
     return gw::fail(GW_ERR_ARG, "gw_voxel_plan_create: fft_y/fft_z must be a supported length >= L+N-1");
   }
-  // real grids: two window rows share one row transform buffer (a window
-  // of at most half the buffer) and the Stockham kernels run both axes (a
-  // fused kernel asked for by name keeps the general path)
-  P->real = want_real && 2 * P->Ly <= fft_ldm(P->My) && P->My <= 2048 &&
+  // real grids: two window rows of floats share one row transform buffer of
+  // float2 (any window the length holds: Ly <= My) and the Stockham kernels
+  // run both axes (a fused kernel asked for by name keeps the general path).
+  // Measured against the general path for windows beyond half the buffer,
+  // whole voxel stage of 180 slices: Ly 754 of 1024 0.78 -> 0.515 ms, Ly 539
+  // of 768 0.378 -> 0.275 ms, Ly 359 of 512 0.235 -> 0.182 ms.
+  P->real = want_real && P->My <= 2048 &&
             p->transform_y != GW_TRANSFORM_FUSED && p->transform_z != GW_TRANSFORM_FUSED;
   P->Nf = P->real ? P->Nc - P->m_zero : P->Nc;
   // batch size: keep the per-batch intermediates near L2 size
@@ -1778,94 +1912,9 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       return gw::cuda_fail(e, "column tables", __FILE__, __LINE__);
     }
   }
-  // gather binning: where it applies and the pixel store fits the budget
-  // (GW_GATHER_MAX_MB, default 8192)
-  {
-    const size_t g_bytes = (size_t)P->n_slices * P->Nf * P->Nr * sizeof(float);
-    const char *env = getenv("GW_GATHER_MAX_MB");
-    const size_t cap = (env ? (size_t)std::max(0L, atol(env)) : (size_t)8192) << 20;
-    // (and fewer than 2^31 pixels: the gather addresses them with 32 bits)
-    const bool can = !P->plain && p->accum == GW_ACCUM_FP64 && !P->fused_z &&
-                     g_bytes <= cap && g_bytes / sizeof(float) < ((size_t)1 << 31);
-    if (p->binning == GW_BINNING_GATHER && !can) {
-      gw_voxel_plan_destroy(P);
-      return gw::fail(GW_ERR_ARG, "gw_voxel_plan_create: gather binning needs a batched, "
-                                  "float64-accumulating plan without the fused column "
-                                  "kernel, and a pixel store within GW_GATHER_MAX_MB");
-    }
-    // auto: gather for one structure on real grids whose float64 sum grid
-    // is larger than L2 -- each atomic is then a DRAM read-modify-write and
-    // the grid's clearing a DRAM pass, while each stored pixel serves two
-    // voxels (its mirror) -- measured faster there (si-100A) and slower
-    // with the grid in L2, several structures (the gather loops over the
-    // structures of every entry) or complex grids (lamellar-200A)
-    const size_t sum_bytes = P->sum_stride * P->n_out * sizeof(double);
-    const bool want = p->binning == GW_BINNING_GATHER ||
-                      (p->binning == GW_BINNING_AUTO && P->real && n_struct == 1 &&
-                       sum_bytes > ctx->l2_bytes);
-    if (want && can) {
-      // the line entries, in table order (phi, band column): counting sort
-      // by window line
-      std::vector<int> cof((size_t)n_phi * P->Nc);
-      cudaError_t e = cudaMemcpy(cof.data(), P->d_colofs, cof.size() * sizeof(int),
-                                 cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) {
-        gw_voxel_plan_destroy(P);
-        return gw::cuda_fail(e, "column tables", __FILE__, __LINE__);
-      }
-      const int W = P->W;
-      std::vector<int> lptr((size_t)W * W + 1, 0);
-      for (int co : cof)
-        if (co >= 0) ++lptr[co / W + 1];
-      for (size_t i = 1; i < lptr.size(); ++i) lptr[i] += lptr[i - 1];
-      std::vector<int2> lent(std::max(lptr.back(), 1));
-      std::vector<int> fill(lptr.begin(), lptr.end() - 1);
-      for (int q = 0; q < n_phi; ++q)
-        for (int m = 0; m < P->Nc; ++m) {
-          const int co = cof[(size_t)q * P->Nc + m];
-          if (co < 0) continue;
-          // F1 column of table column m: itself, or with real grids its
-          // mirror's (rows mirrored) below m_zero
-          int j = m, flip = 0;
-          if (P->real) {
-            if (m >= P->m_zero) j = m - P->m_zero;
-            else { j = P->m_zero - m; flip = 1; }
-          }
-          lent[fill[co / W]++] = make_int2(q, 2 * j + flip);
-        }
-      // output rows of every window z, ascending
-      std::vector<int> zptr((size_t)W + 1, 0);
-      for (int ro : rowofs)
-        if (ro >= 0) ++zptr[ro + 1];
-      for (int i = 1; i <= W; ++i) zptr[i] += zptr[i - 1];
-      std::vector<int> zrows(std::max(zptr.back(), 1));
-      std::vector<int> zfill(zptr.begin(), zptr.end() - 1);
-      for (int mr = 0; mr < P->Nr; ++mr)
-        if (rowofs[mr] >= 0) zrows[zfill[rowofs[mr]]++] = mr;
-      // window z with more than one output row
-      std::vector<int> zmulti;
-      for (int z = 0; z < W; ++z)
-        if (zptr[z + 1] - zptr[z] > 1) zmulti.push_back(z);
-      P->n_zmulti = (int)zmulti.size();
-      if (zmulti.empty()) zmulti.push_back(0);
-      // lines with more than kGatherHeavy pixels per voxel (entries times
-      // the structures each output sums; near the rotation axis)
-      const int per_entry = p->average == GW_STRUCTS_SEPARATE ? 1 : n_struct;
-      std::vector<int> heavy;
-      for (int l = 0; l < W * W; ++l)
-        if ((int64_t)(lptr[l + 1] - lptr[l]) * per_entry > kGatherHeavy) heavy.push_back(l);
-      P->n_heavy = (int)heavy.size();
-      P->h_heavy = heavy;
-      if (heavy.empty()) heavy.push_back(0);
-      if ((st = upload(&P->d_heavy, heavy, &B)) || (st = upload(&P->d_zmulti, zmulti, &B)) ||
-          (st = upload(&P->d_lptr, lptr, &B)) || (st = upload(&P->d_lent, lent, &B)) ||
-          (st = upload(&P->d_zptr, zptr, &B)) || (st = upload(&P->d_zrows, zrows, &B)) ||
-          (st = alloc(&P->d_G, g_bytes / sizeof(float), &B))) {
-        gw_voxel_plan_destroy(P);
-        return st;
-      }
-      P->gather = true;
-    }
+  if ((st = gather_setup(P))) {
+    gw_voxel_plan_destroy(P);
+    return st;
   }
   *out = P;
   return GW_OK;
@@ -1933,10 +1982,8 @@ extern "C" int gw_voxel_set_shells(gw_voxel_plan *P, int32_t n_shells,
                                    int32_t mode, const double *q_axis,
                                    const double *lower, const double *upper,
                                    const float *f, const double *avg_f) {
-  if (P && P->real)
-    return gw::fail(GW_ERR_STATE, "gw_voxel_set_shells: the plan was made with "
-                                  "real_grids (per-shell f values): make it with real_grids 0");
   if (!P) return gw::fail(GW_ERR_ARG, "gw_voxel_set_shells: null plan");
+  GW_TRY(gwv::leave_real(P, "gw_voxel_set_shells"));
   auto drop = [P]() {
     gw::dev_free(P->d_shell); gw::dev_free(P->d_f_shells);
     gw::dev_free(P->d_structs_shells);

@@ -162,10 +162,12 @@ typedef struct gw_voxel_params {
                            symmetry F(-k) = conj F(k) of a real grid); the
                            bands are made symmetric.  Used in batched,
                            nearest-bin plans with the Stockham kernels (not
-                           with GW_TRANSFORM_FUSED) when the window fits
-                           half a transform buffer; no shells, no backward.
-                           gw_voxel_info reports whether it runs.  0: the
-                           general path.                                   */
+                           with GW_TRANSFORM_FUSED) with row transforms up
+                           to 2048 points; no shells, no backward, but a
+                           plan whose window is wider than half a transform
+                           buffer takes them and goes on on the general
+                           path.  gw_voxel_info reports whether it runs.
+                           0: the general path.                            */
   int32_t binning;      /* how |F|^2 pixels reach the voxel sums.
                            GW_BINNING_ATOMIC: float64 atomic adds as the
                            column transforms produce them (the sum's

@@ -1,0 +1,88 @@
+"""Real-grid plans whose window is wider than half the transform buffer (two
+window rows of floats share one buffer of complex values) against the general
+path, at transform lengths from 128 to 2048, and what such plans still take
+that narrower real-grid plans refuse: per-shell f values and the adjoint."""
+import numpy as np
+import pytest
+
+from giwaxsim_gb300 import forward as F
+
+pytestmark = pytest.mark.gpu
+RTOL = 1e-5
+
+# (r, dq, max_q, box edge), transform length
+CASES = [((0.4, 0.1, 0.6), 22.0, 128), ((0.3, 0.08, 0.4), 45.0, 256),
+         ((0.2, 0.05, 0.3), 70.0, 640), ((0.15, 0.04, 0.3), 80.0, 1024),
+         ((0.12, 0.04, 0.3), 90.0, 1280), ((0.1, 0.04, 0.3), 100.0, 1536),
+         ((0.1, 0.035, 0.25), 130.0, 2048)]
+PHIS = np.array([0.0, 11.0, 45.0, 90.0, 133.5])
+
+
+def ldm(m):
+    return m + m // 16 + 4
+
+
+def atoms(box, seed, n=301):
+    rng = np.random.default_rng(seed)
+    xyz = rng.uniform(0.0, box, (n, 3)) * [1.0, 0.97, 0.3]
+    return xyz, np.where(rng.random(n) < 0.3, -0.5, 1.0) * (6.0 + 0.2j)
+
+
+def rel_l2(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("axes,box,m", CASES)
+@pytest.mark.parametrize("fill,smooth", [(False, 0), (True, 1.5)])
+def test_wide_window_vs_general(axes, box, m, fill, smooth):
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, m)
+    out = {}
+    for real in (None, False):
+        plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS, fill_bkg=fill,
+                           smooth=smooth, real=real)
+        try:
+            info = plan.info()
+            assert info["real"] == (real is None)
+            assert 2 * info["Ly"] > ldm(info["My"]) and info["My"] == m
+            plan.set_atoms()
+            plan.execute()
+            out[real] = plan.iq().copy()
+        finally:
+            plan.close()
+    assert rel_l2(out[None], out[False]) <= RTOL
+
+
+@pytest.mark.parametrize("binning", ["atomic", "gather"])
+@pytest.mark.parametrize("what", ["adjoint", "shells"])
+def test_wide_plan_takes_the_adjoint_and_shells(binning, what):
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    bound = 1.1 * np.sqrt(3) * geom.q[-1]
+    g_iq = np.random.default_rng(4).standard_normal((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    got = {}
+    for real in (None, False):
+        plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS, real=real, binning=binning)
+        try:
+            plan.set_atoms()
+            plan.execute()
+            assert plan.info()["real"] == (real is None)
+            if what == "adjoint":
+                got[real] = [plan.backward(g_iq)["g_f"].view(float)]
+                got[real].append(plan.iq().copy())  # of the execute before it
+            else:
+                avg = plan.structs["avg_f_re"][0] + 1j * plan.structs["avg_f_im"][0]
+                plan.set_shells(geom.q, np.array([0.0]), np.array([bound]), 1.5 * fv[None, :],
+                                np.full((1, 1), 1.5 * avg))
+                plan.execute()
+                got[real] = [plan.iq().copy()]
+                plan.set_shells(None, None, None, None, None)
+                plan.set_atoms()
+            assert plan.info()["real"] == 0
+            plan.execute()
+            got[real].append(plan.iq().copy())
+        finally:
+            plan.close()
+    for a, b in zip(got[None], got[False]):
+        assert rel_l2(a, b) <= RTOL
