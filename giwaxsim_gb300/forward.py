@@ -741,7 +741,7 @@ class PlaneCorners:
                           [x[-1, 0], y[-1, 0], z[-1, 0]]], dtype=np.float64)
         return c
 
-    def matrix(self, kind, angle):
+    def axis(self, kind):
         p1, p2, p3 = self.pts
         if kind == "psi":
             axis = np.cross(p2 - p1, p3 - p1)
@@ -752,12 +752,92 @@ class PlaneCorners:
         else:
             raise ValueError(kind)
         axis /= np.linalg.norm(axis)
-        return rotation_matrix(axis, np.radians(angle))
+        return axis
+
+    def matrix(self, kind, angle):
+        return rotation_matrix(self.axis(kind), np.radians(angle))
 
     def rotate(self, R):
         out = PlaneCorners.__new__(PlaneCorners)
         out.pts = N.rotate_points(R, self.pts)
         return out
+
+
+def _turns(axis, angles):
+    """rotation_matrix(axis, radians(angle)) of every angle, (n, 3, 3): the
+    same scalar trig and pow, and per element the same expression trees."""
+    ux, uy, uz = axis[0], axis[1], axis[2]
+    t = [np.radians(a) for a in angles]
+    c = np.array([np.cos(a) for a in t])
+    s = np.array([np.sin(a) for a in t])
+    k = 1 - c
+    R = np.empty((len(t), 3, 3))
+    R[:, 0, 0] = c + ux ** 2 * k
+    R[:, 0, 1] = ux * uy * k - uz * s
+    R[:, 0, 2] = ux * uz * k + uy * s
+    R[:, 1, 0] = uy * ux * k + uz * s
+    R[:, 1, 1] = c + uy ** 2 * k
+    R[:, 1, 2] = uy * uz * k - ux * s
+    R[:, 2, 0] = uz * ux * k - uy * s
+    R[:, 2, 1] = uz * uy * k + ux * s
+    R[:, 2, 2] = c + uz ** 2 * k
+    return R
+
+
+def _turn_corners(corners, R):
+    """corners.rotate(R[i]) for every i, as (n, 3 corners, 3): component j of
+    corner k is the fused chain of row j of R[i] with that corner, so one
+    native call over all the rows gives them (its products commute)."""
+    rows = N.rotate_points(corners.pts, R.reshape(-1, 3))
+    return rows.reshape(len(R), 3, 3).transpose(0, 2, 1)
+
+
+def orientation_matrices(corners, psis, psi_weights, phis, phi_weights, thetas,
+                         theta_weights):
+    """(rotations per orientation, their matrices (n, 3, 3) in order, weights)
+    of the psi x phi x theta list (comparison.py:836-841, detector.py:234-244).
+    An axis depends on the rotations before it only, so the matrices of one
+    axis are made for all its angles at once; identity matrices are left
+    out, which changes no bit."""
+    n1, n2, n3 = (min(len(a), len(w)) for a, w in
+                  ((psis, psi_weights), (phis, phi_weights), (thetas, theta_weights)))
+    psis, phis, thetas = psis[:n1], phis[:n2], thetas[:n3]
+    if n1 * n2 * n3 == 0:
+        return np.zeros(0, np.int32), np.zeros((0, 3, 3)), np.zeros(0)
+    a, b, c = (np.asarray(v)[:n] for v, n in ((psi_weights, n1), (phi_weights, n2),
+                                              (theta_weights, n3)))
+    if a.dtype == b.dtype == c.dtype == np.float64:
+        w = a[:, None, None] * b[None, :, None] * c[None, None, :]
+    else:  # other types multiply element by element in their own precision
+        w = np.array([p * h * t for p in psi_weights[:n1] for h in phi_weights[:n2]
+                      for t in theta_weights[:n3]], dtype=np.float64)
+    # a zero angle about an axis of finite direction is the identity exactly:
+    # the trailing axes whose angles are all zero need no corners
+    p = corners.pts
+    sound = (np.isfinite(p).all() and np.linalg.norm(p[1] - p[0]) > 0
+             and np.linalg.norm(p[2] - p[0]) > 0
+             and all(np.isfinite(np.asarray(a, dtype=np.float64)).all()
+                     for a in (psis, phis, thetas)))
+    no_theta = sound and all(a == 0 for a in thetas)
+    no_phi = no_theta and all(a == 0 for a in phis)
+    full = np.empty((n1, n2, n3, 3, 3, 3))
+    full[...] = _IDENTITY
+    R1 = _turns(corners.axis("psi"), psis)
+    full[..., 0, :, :] = R1[:, None, None]
+    for i in range(0 if no_phi else n1):
+        c1 = corners.rotate(R1[i])
+        R2 = _turns(c1.axis("phi"), phis)
+        full[i, :, :, 1] = R2[:, None]
+        if no_theta:
+            continue
+        c2 = _turn_corners(c1, R2)
+        for j in range(n2):
+            axis = c2[j, 1] - c2[j, 0]
+            axis /= np.linalg.norm(axis)
+            full[i, j, :, 2] = _turns(axis, thetas)
+    full = full.reshape(-1, 3, 3, 3)
+    turns = (full != _IDENTITY).any(axis=(2, 3))
+    return turns.sum(1).astype(np.int32), full[turns], w.reshape(-1)
 
 
 _IDENTITY = np.eye(3)
@@ -784,21 +864,9 @@ class DetectorPlan:
                 init.append(R)
         psis, phis, thetas = (np.atleast_1d(np.asarray(a)) for a in
                               (psis, phis, thetas))
-        n_rot, mats, weights = [], [], []
-        for ps, pw in zip(psis, psi_weights):
-            for ph, hw in zip(phis, phi_weights):
-                for th, tw in zip(thetas, theta_weights):
-                    c = corners
-                    k = 0
-                    for kind, ang in (("psi", ps), ("phi", ph), ("theta", th)):
-                        R = c.matrix(kind, ang)
-                        c = c.rotate(R)
-                        if not np.array_equal(R, _IDENTITY):
-                            mats.append(R)
-                            k += 1
-                    n_rot.append(k)
-                    weights.append(pw * hw * tw)
-        if not weights:
+        n_rot, mats, weights = orientation_matrices(
+            corners, psis, psi_weights, phis, phi_weights, thetas, theta_weights)
+        if not len(weights):
             raise ValueError("no detector orientation")
         self.n_orient = len(weights)
         self.iq_shape = tuple(int(s) for s in iq_shape)
@@ -816,10 +884,10 @@ class DetectorPlan:
         self._h = np.ascontiguousarray(h)
         self._v = np.ascontiguousarray(v)
         self._init = np.ascontiguousarray(np.array(init).reshape(-1, 9)) if init else None
-        self._nrot = np.ascontiguousarray(np.array(n_rot, dtype=np.int32))
-        self._mats = (np.ascontiguousarray(np.array(mats).reshape(-1, 9))
-                      if mats else None)
-        self._w = np.ascontiguousarray(np.array(weights, dtype=np.float64))
+        self._nrot = np.ascontiguousarray(n_rot, dtype=np.int32)
+        self._mats = (np.ascontiguousarray(mats.reshape(-1, 9))
+                      if len(mats) else None)
+        self._w = np.ascontiguousarray(weights, dtype=np.float64)
         hdl = ctypes.c_void_p()
         N.check(N.lib().gw_detector_plan_create(
             self.ctx.handle, ctypes.byref(p), N.ptr(self._h), N.ptr(self._v),
