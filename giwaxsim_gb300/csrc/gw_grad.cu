@@ -190,7 +190,9 @@ struct GradCol {
 // NB columns of one slice: recompute F along z from F1 (forward chirp-z),
 // form G_F = 2 F dL/dsum[bin] on the binned pixels, and transform G_F back
 // to the z window (adjoint chirp-z), leaving G1[col][z].
-template <int M>
+// HALF: window and band within M / 2 (pruned first and last passes, as in
+// the forward kernels).
+template <int M, bool HALF>
 __global__ void __launch_bounds__(FftShape<M>::NT, FftShape<M>::MINB)
 k_col_bwd(SliceArgs a, CztArgs cz, BinArgs bn, GradCol gc, int slice0, int nc,
           const float2 *F1) {
@@ -209,8 +211,8 @@ k_col_bwd(SliceArgs a, CztArgs cz, BinArgs bn, GradCol gc, int slice0, int nc,
   int first, rows;
   slice_rows(a, slice0, sl, first, rows);
   ColLoadF1 ld{F1 + (size_t)first * nc, cz.A, rows, nc, m0};
-  fft_run<M, NB, NT, false, 1, false, 0, true>(buf, tw, nullptr, ld, NoStore());
-  fft_run<M, NB, NT, true, 0, true, 0, false>(buf, tw, cz.H, NoLoad(), NoStore());
+  fft_run<M, NB, NT, false, 1, false, 0, true, HALF>(buf, tw, nullptr, ld, NoStore());
+  fft_run<M, NB, NT, true, 0, true, 0, false, false, HALF>(buf, tw, cz.H, NoLoad(), NoStore());
   const float2 cbg = slice_const(a, sl).cbg;
   for (int t = threadIdx.x; t < NB * M; t += NT) {
     const int f = t / M, mr = t - f * M;
@@ -237,9 +239,9 @@ k_col_bwd(SliceArgs a, CztArgs cz, BinArgs bn, GradCol gc, int slice0, int nc,
     buf[f * LDM + fft_pad(mr)] = out;
   }
   __syncthreads();
-  fft_run<M, NB, NT, false, 0, false, 0, false>(buf, tw, nullptr, NoLoad(), NoStore());
+  fft_run<M, NB, NT, false, 0, false, 0, false, HALF>(buf, tw, nullptr, NoLoad(), NoStore());
   ColStoreAdj st{gc.Ba, gc.G1 + (size_t)slot * a.Lz * nc, a.Lz, nc, m0};
-  fft_run<M, NB, NT, true, 0, true, 1, false>(buf, tw, gc.Ha, NoLoad(), st);
+  fft_run<M, NB, NT, true, 0, true, 1, false, false, HALF>(buf, tw, gc.Ha, NoLoad(), st);
 }
 
 // ------------------------------------------------------------ row stage
@@ -268,9 +270,31 @@ struct RowLoadAdj {
   }
 };
 
+__device__ __forceinline__ float warp_sum(float v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// v of every lane added to word f of rows of 7 words: one add for a warp
+// whose lanes share a row, else one a lane.
+__device__ __forceinline__ void row_add(float *word, int f, float v, int lane) {
+  if (__all_sync(0xffffffffu, f == __shfl_sync(0xffffffffu, f, 0))) {
+    v = warp_sum(v);
+    if (lane == 0 && v != 0.f) atomicAdd(word + 7 * f, v);
+  } else if (v != 0.f) {
+    atomicAdd(word + 7 * f, v);
+  }
+}
+
 // NB window rows: transform G1 back to the y window (G_D), then the atoms of
 // the rows gather G_D at their cells; per-row sums go to the slice scalars.
-template <int M, bool BIL>
+//
+// The row sums are taken in registers: a warp (or several, one part each)
+// goes over a row's window, then over the block's atoms 32 at a time, and
+// adds its lane sums to the row's shared words once (per-element shared
+// atomics on the same few words serialised the kernel: 150 slices of 230
+// rows at M = 512 took 1.67 ms, now 0.295 ms).
+template <int M, bool BIL, bool HALF>
 __global__ void __launch_bounds__(FftShape<M>::NT, FftShape<M>::MINB)
 k_row_bwd(SliceArgs a, GradRow gr, int slice0, int n_sl, int n_rows) {
   constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
@@ -305,93 +329,116 @@ k_row_bwd(SliceArgs a, GradRow gr, int slice0, int n_sl, int n_rows) {
   }
   __syncthreads();
   RowLoadAdj<M> ld{gr.G1, gr.Aa, gr.nc, a.Lz, r_slot, r_zz, row0, n_rows};
-  fft_run<M, NB, NT, false, 1, false, 0, true>(buf, tw, nullptr, ld, NoStore());
-  fft_run<M, NB, NT, true, 0, true, 0, false>(buf, tw, gr.Ha, NoLoad(), NoStore());
-  // G_D on the window, and the per-row sums of G_D m and G_D dm/dsigma
-  for (int t = threadIdx.x; t < NB * a.Ly; t += NT) {
-    const int f = t / a.Ly, yy = t - f * a.Ly;
-    const int row = row0 + f;
-    if (row >= n_rows) continue;
-    float2 *q = buf + f * LDM + fft_pad(yy);
-    const float2 v = conjf2(cmul(*q, __ldg(gr.Ba + yy)));
-    *q = v;
+  fft_run<M, NB, NT, false, 1, false, 0, true, HALF>(buf, tw, nullptr, ld, NoStore());
+  fft_run<M, NB, NT, true, 0, true, 0, false, false, HALF>(buf, tw, gr.Ha, NoLoad(), NoStore());
+  // G_D on the window, and the per-row sums of G_D m and G_D dm/dsigma:
+  // warps w, w + NB, .. take row w % NB (several rows a warp when there are
+  // fewer warps than rows)
+  const int lane = threadIdx.x & 31;
+  constexpr int NW = NT / 32, PARTS = NW / NB > 1 ? NW / NB : 1;
+  for (int u = threadIdx.x >> 5; u < NB * PARTS; u += NW) {
+    const int f = u % NB, part = u / NB;
+    if (row0 + f >= n_rows) continue;
+    const size_t yo = (size_t)r_slot[f] * a.Ly, zo = (size_t)r_slot[f] * a.Lz + r_zz[f];
+    const float mz = a.smooth_on ? a.mz[zo] : 0.f, dmz = a.smooth_on ? gr.dmz[zo] : 0.f;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int yy = part * 32 + lane; yy < a.Ly; yy += 32 * PARTS) {
+      float2 *q = buf + f * LDM + fft_pad(yy);
+      const float2 v = conjf2(cmul(*q, __ldg(gr.Ba + yy)));
+      *q = v;
+      if (a.smooth_on) {
+        const float my = a.my[yo + yy];
+        const float dm = dmz * my + mz * gr.dmy[yo + yy];
+        const float m = mz * my;
+        s[0] += v.x * m;
+        s[1] += v.y * m;
+        s[2] += v.x * dm;
+        s[3] += v.y * dm;
+      }
+    }
     if (a.smooth_on) {
-      const int slot = r_slot[f], zz = r_zz[f];
-      const float mz = a.mz[(size_t)slot * a.Lz + zz], my = a.my[(size_t)slot * a.Ly + yy];
-      const float dm = gr.dmz[(size_t)slot * a.Lz + zz] * my +
-                       mz * gr.dmy[(size_t)slot * a.Ly + yy];
-      const float m = mz * my;
-      atomicAdd(&racc[f][0], v.x * m);
-      atomicAdd(&racc[f][1], v.y * m);
-      atomicAdd(&racc[f][2], v.x * dm);
-      atomicAdd(&racc[f][3], v.y * dm);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        s[k] = warp_sum(s[k]);
+        if (lane == 0) atomicAdd(&racc[f][k], s[k]);
+      }
     }
   }
   __syncthreads();
   const int total = r_cnt[NB];
-  for (int i = threadIdx.x; i < total; i += NT) {
+  for (int i0 = threadIdx.x - lane; i0 < total; i0 += NT) {
+    const int i = i0 + lane;
     int f = 0;
     while (f + 1 < NB && i >= r_cnt[f + 1]) ++f;
+    float sig = 0.f, su = 0.f, sv = 0.f;  // the atom's terms of the row sums
     const int at = r_lo[f] + (i - r_cnt[f]);
     const int slot = r_slot[f], zz = r_zz[f];
     const int sl = slice0 + slot;
-    const float mz = a.smooth_on ? a.mz[(size_t)slot * a.Lz + zz] : 1.f;
-    const float dmz = a.smooth_on ? gr.dmz[(size_t)slot * a.Lz + zz] : 0.f;
-    const float4 q = a.xyf_s[at];
-    const float2 fs = make_float2(q.z, q.w);
     if constexpr (!BIL) {
       int yy;
-      if (!deposit_column(a, at, sl, yy) || yy >= a.Ly) continue;
-      const float2 G = buf[f * LDM + fft_pad(yy)];
-      float m = 1.f;
-      if (a.smooth_on) {
-        const float my = a.my[(size_t)slot * a.Ly + yy];
-        m = mz * my;
-        const float dm = dmz * my + mz * gr.dmy[(size_t)slot * a.Ly + yy];
-        atomicAdd(&racc[f][4], redot(G, fs) * dm);
-      }
-      atomicAdd(&gr.gacc[at].x, (double)(G.x * m));
-      atomicAdd(&gr.gacc[at].y, (double)(G.y * m));
-    } else {
-      int i0;
-      float fu;
-      if (!bilinear_column(a, at, sl, i0, fu)) continue;
-      const bool own = at >= r_mid[f];  // this row holds the atom's lower z corner
-      const float fz = a.fz_s[at];
-      const float wz = own ? 1.f - fz : fz;
-      float2 acc = make_float2(0.f, 0.f), du = acc, dv = acc;
-      float sig = 0.f;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int ic = i0 + c;
-        if (ic >= a.g) continue;
-        const int yy = window_col(a, ic);
-        if (yy >= a.Ly) continue;
+      if (i < total && deposit_column(a, at, sl, yy) && yy < a.Ly) {
+        const float4 q = a.xyf_s[at];
         const float2 G = buf[f * LDM + fft_pad(yy)];
         float m = 1.f;
         if (a.smooth_on) {
+          const float mz = a.mz[(size_t)slot * a.Lz + zz], dmz = gr.dmz[(size_t)slot * a.Lz + zz];
           const float my = a.my[(size_t)slot * a.Ly + yy];
           m = mz * my;
           const float dm = dmz * my + mz * gr.dmy[(size_t)slot * a.Ly + yy];
-          sig += (c ? fu : 1.f - fu) * dm * redot(G, fs);
+          sig = redot(G, make_float2(q.z, q.w)) * dm;
         }
-        const float wy = c ? fu : 1.f - fu, dwy = c ? 1.f : -1.f;
-        const float2 Gm = make_float2(G.x * m, G.y * m);
-        acc.x += wy * Gm.x; acc.y += wy * Gm.y;
-        du.x += dwy * Gm.x; du.y += dwy * Gm.y;
-        dv.x += wy * Gm.x; dv.y += wy * Gm.y;
+        atomicAdd(&gr.gacc[at].x, (double)(G.x * m));
+        atomicAdd(&gr.gacc[at].y, (double)(G.y * m));
       }
-      if (a.smooth_on) atomicAdd(&racc[f][4], wz * sig);
-      atomicAdd(&gr.gacc[at].x, (double)(wz * acc.x));
-      atomicAdd(&gr.gacc[at].y, (double)(wz * acc.y));
-      const gw_phi &ph = a.ph[sl % a.n_phi];
-      const double gyp = (double)(wz * redot(du, fs)) * a.inv_r;   // dL/dy'
-      const double gz = (double)((own ? -1.f : 1.f) * redot(dv, fs)) * a.inv_r;
-      atomicAdd(gr.gxyz + 3 * (size_t)at, gyp * ph.sin_phi);
-      atomicAdd(gr.gxyz + 3 * (size_t)at + 1, gyp * ph.cos_phi);
-      atomicAdd(gr.gxyz + 3 * (size_t)at + 2, gz);
-      atomicAdd(&racc[f][5], (float)gyp);
-      atomicAdd(&racc[f][6], (float)gz);
+    } else {
+      int i0c;
+      float fu;
+      if (i < total && bilinear_column(a, at, sl, i0c, fu)) {
+        const float mz = a.smooth_on ? a.mz[(size_t)slot * a.Lz + zz] : 1.f;
+        const float dmz = a.smooth_on ? gr.dmz[(size_t)slot * a.Lz + zz] : 0.f;
+        const float4 q = a.xyf_s[at];
+        const float2 fs = make_float2(q.z, q.w);
+        const bool own = at >= r_mid[f];  // this row holds the atom's lower z corner
+        const float fz = a.fz_s[at];
+        const float wz = own ? 1.f - fz : fz;
+        float2 acc = make_float2(0.f, 0.f), du = acc, dv = acc;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int ic = i0c + c;
+          if (ic >= a.g) continue;
+          const int yy = window_col(a, ic);
+          if (yy >= a.Ly) continue;
+          const float2 G = buf[f * LDM + fft_pad(yy)];
+          float m = 1.f;
+          const float wy = c ? fu : 1.f - fu, dwy = c ? 1.f : -1.f;
+          if (a.smooth_on) {
+            const float my = a.my[(size_t)slot * a.Ly + yy];
+            m = mz * my;
+            const float dm = dmz * my + mz * gr.dmy[(size_t)slot * a.Ly + yy];
+            sig += wy * dm * redot(G, fs);
+          }
+          const float2 Gm = make_float2(G.x * m, G.y * m);
+          acc.x += wy * Gm.x; acc.y += wy * Gm.y;
+          du.x += dwy * Gm.x; du.y += dwy * Gm.y;
+          dv.x += wy * Gm.x; dv.y += wy * Gm.y;
+        }
+        sig *= wz;
+        atomicAdd(&gr.gacc[at].x, (double)(wz * acc.x));
+        atomicAdd(&gr.gacc[at].y, (double)(wz * acc.y));
+        const gw_phi &ph = a.ph[sl % a.n_phi];
+        const double gyp = (double)(wz * redot(du, fs)) * a.inv_r;   // dL/dy'
+        const double gz = (double)((own ? -1.f : 1.f) * redot(dv, fs)) * a.inv_r;
+        atomicAdd(gr.gxyz + 3 * (size_t)at, gyp * ph.sin_phi);
+        atomicAdd(gr.gxyz + 3 * (size_t)at + 1, gyp * ph.cos_phi);
+        atomicAdd(gr.gxyz + 3 * (size_t)at + 2, gz);
+        su = (float)gyp;
+        sv = (float)gz;
+      }
+    }
+    if (a.smooth_on) row_add(&racc[0][4], f, sig, lane);
+    if constexpr (BIL) {
+      row_add(&racc[0][5], f, su, lane);
+      row_add(&racc[0][6], f, sv, lane);
     }
   }
   __syncthreads();
@@ -436,31 +483,40 @@ size_t fft_smem() {
   return (size_t)(FftShape<M>::NB * FftPlan<M>::LDM + FftPlan<M>::tw_len()) * sizeof(float2);
 }
 
-template <int M>
-int launch_col_bwd(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
-                   const BinArgs &bn, const GradCol &gc, int s0, int n) {
+template <int M, bool HALF>
+int launch_col_bwd_t(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
+                     const BinArgs &bn, const GradCol &gc, int s0, int n) {
   constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
   const size_t smem = fft_smem<M>();
   static gw::SmemRecord attr;
-  GW_TRY(gw::smem_limit(attr, k_col_bwd<M>, smem));
+  GW_TRY(gw::smem_limit(attr, k_col_bwd<M, HALF>, smem));
   dim3 grid((P->Nc + NB - 1) / NB, n);
   gw::KTimer tm(P->ctx, GW_K_COLBIN);
-  k_col_bwd<M><<<grid, NT, smem, P->ctx->stream>>>(a, cz, bn, gc, s0, P->Nc, P->d_F1);
+  k_col_bwd<M, HALF><<<grid, NT, smem, P->ctx->stream>>>(a, cz, bn, gc, s0, P->Nc, P->d_F1);
   GW_LAUNCHED(P->ctx);
   return GW_OK;
 }
 
-template <int M, bool BIL>
+template <int M>
+int launch_col_bwd(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
+                   const BinArgs &bn, const GradCol &gc, int s0, int n) {
+  if constexpr (M <= 2048) {
+    if (pruned<M>(cz)) return launch_col_bwd_t<M, true>(P, a, cz, bn, gc, s0, n);
+  }
+  return launch_col_bwd_t<M, false>(P, a, cz, bn, gc, s0, n);
+}
+
+template <int M, bool BIL, bool HALF>
 int launch_row_bwd_t(gw_voxel_plan *P, const SliceArgs &a, const GradRow &gr,
                      int s0, int n_sl) {
   const int n_rows = batch_rows(P, s0, n_sl);
   constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
   const size_t smem = fft_smem<M>();
   static gw::SmemRecord attr;
-  GW_TRY(gw::smem_limit(attr, k_row_bwd<M, BIL>, smem));
+  GW_TRY(gw::smem_limit(attr, k_row_bwd<M, BIL, HALF>, smem));
   gw::KTimer tm(P->ctx, GW_K_ROW);
-  k_row_bwd<M, BIL><<<(n_rows + NB - 1) / NB, NT, smem, P->ctx->stream>>>(a, gr, s0, n_sl,
-                                                                          n_rows);
+  k_row_bwd<M, BIL, HALF><<<(n_rows + NB - 1) / NB, NT, smem, P->ctx->stream>>>(
+      a, gr, s0, n_sl, n_rows);
   GW_LAUNCHED(P->ctx);
   return GW_OK;
 }
@@ -468,8 +524,13 @@ int launch_row_bwd_t(gw_voxel_plan *P, const SliceArgs &a, const GradRow &gr,
 template <int M>
 int launch_row_bwd(gw_voxel_plan *P, const SliceArgs &a, const GradRow &gr,
                    int s0, int n_sl) {
-  return a.bil ? launch_row_bwd_t<M, true>(P, a, gr, s0, n_sl)
-               : launch_row_bwd_t<M, false>(P, a, gr, s0, n_sl);
+  if constexpr (M <= 2048) {
+    if (a.Ly <= M / 2 && gr.nc <= M / 2)
+      return a.bil ? launch_row_bwd_t<M, true, true>(P, a, gr, s0, n_sl)
+                   : launch_row_bwd_t<M, false, true>(P, a, gr, s0, n_sl);
+  }
+  return a.bil ? launch_row_bwd_t<M, true, false>(P, a, gr, s0, n_sl)
+               : launch_row_bwd_t<M, false, false>(P, a, gr, s0, n_sl);
 }
 
 int col_bwd_dispatch(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
@@ -516,8 +577,8 @@ int grad_state_init(gw_voxel_plan *P) {
         (st = upload(&G->d_By, ty.B, &B)) || (st = upload(&G->d_Az, tz.A, &B)) ||
         (st = upload(&G->d_Hz, tz.H, &B)) || (st = upload(&G->d_Bz, tz.B, &B)) ||
         (st = upload(&G->d_dgw, dgw, &B)) ||
-        (st = alloc(&G->d_dmy, (size_t)P->S * P->Ly, &B)) ||
-        (st = alloc(&G->d_dmz, (size_t)P->S * P->Lz, &B)) ||
+        (st = alloc(&G->d_dmy, (size_t)P->n_slices * P->Ly, &B)) ||
+        (st = alloc(&G->d_dmz, (size_t)P->n_slices * P->Lz, &B)) ||
         (st = alloc(&G->d_gsum, W3, &B)) || (st = alloc(&G->d_giq, Qc3, &B)) ||
         (st = alloc(&G->d_G1, (size_t)P->S * P->Lz * P->Nc, &B)) ||
         (st = alloc(&G->d_sc, (size_t)P->n_slices * SC_N, &B)) ||
@@ -620,22 +681,31 @@ extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
              (float)((double)P->g * (double)P->g)};
   GradRow gr{G->d_Ay, G->d_Hy, G->d_By, P->d_twy, G->d_G1, G->d_dmy, G->d_dmz,
              G->d_gacc, G->d_gxyz, G->d_sc, P->Nc};
-  for (int s0 = 0; s0 < P->n_slices; s0 += P->S) {
-    const int nb = std::min(P->S, P->n_slices - s0);
-    GW_TRY(enqueue_slice_setup(P, a, s0, nb));
+  // the per-slice setup of every slice at once, as in the forward pass
+  for (int c0 = 0; c0 < P->n_slices; c0 += kSetupChunk) {
+    const int nb = std::min(kSetupChunk, P->n_slices - c0);
+    const SliceArgs ac = profile_view(a, c0);
+    GW_TRY(enqueue_slice_setup(P, ac, c0, nb));
     if (a.smooth_on) {
       gw::KTimer tm(ctx, GW_K_PROFILE);
-      k_dprofile<<<nb, 256, 0, st>>>(a, s0, G->d_dgw, G->d_dmy, G->d_dmz);
+      k_dprofile<<<nb, 256, 0, st>>>(ac, c0, G->d_dgw, G->d_dmy + (size_t)c0 * P->Ly,
+                                     G->d_dmz + (size_t)c0 * P->Lz);
       GW_LAUNCHED(ctx);
     }
     if (P->bil) {
       gw::KTimer tm(ctx, GW_K_MISC);
-      k_argmin_y<<<dim3(nblk_at, nb), 256, 0, st>>>(a, s0, P->d_perm, G->d_amy);
+      k_argmin_y<<<dim3(std::min(nblk_at, 16), nb), 256, 0, st>>>(a, c0, P->d_perm, G->d_amy);
       GW_LAUNCHED(ctx);
     }
-    GW_TRY(row_dispatch(P, a, cy, s0, nb));
-    GW_TRY(col_bwd_dispatch(P, a, cz, bn, gc, s0, nb));
-    GW_TRY(row_bwd_dispatch(P, a, gr, s0, nb));
+  }
+  for (int s0 = 0; s0 < P->n_slices; s0 += P->S) {
+    const int nb = std::min(P->S, P->n_slices - s0);
+    const SliceArgs ab = profile_view(a, s0);
+    gr.dmy = G->d_dmy + (size_t)s0 * P->Ly;
+    gr.dmz = G->d_dmz + (size_t)s0 * P->Lz;
+    GW_TRY(row_dispatch(P, ab, cy, s0, nb));
+    GW_TRY(col_bwd_dispatch(P, ab, cz, bn, gc, s0, nb));
+    GW_TRY(row_bwd_dispatch(P, ab, gr, s0, nb));
   }
   {
     gw::KTimer tm(ctx, GW_K_MISC);

@@ -1239,9 +1239,6 @@ int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n) {
   return GW_OK;
 }
 
-// Slices per launch of the setup kernels (their grids index slices in y).
-constexpr int kSetupChunk = 32768;
-
 // Average, crop and f0 factor of every I(q) grid the plan produces: the
 // float32 grid the detector reads (f64 false; part of every execute) or the
 // float64 grid (f64 true; made when a caller asks for float64 I(q)).

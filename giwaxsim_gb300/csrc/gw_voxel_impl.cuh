@@ -678,6 +678,10 @@ namespace gwv {
 SliceArgs slice_args(gw_voxel_plan *P);
 // Structure preparation: extents reset, z sort, column tables.
 int enqueue_prep(gw_voxel_plan *P);
+// Slice arguments whose profile arrays start at slice s0.
+SliceArgs profile_view(const SliceArgs &a, int s0);
+// Slices per launch of the setup kernels (their grids index slices in y).
+constexpr int kSetupChunk = 32768;
 // Per-slice min/max, extents and profiles of slices [s0, s0+n).
 int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n);
 // Row transforms of the window rows of slices [s0, s0+n_sl), into d_F1.
