@@ -87,24 +87,27 @@ k_row_czt(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
 // second; the window fits: L <= LDM), transforms the NB packed
 // rows, leaves the inverse transform in shared memory, and writes F1 for
 // the columns ky >= 0 only (the column stage needs no others):
-// F1[row][j] = u_row Y_row[m_zero + j], j < nf.
+// F1[row][j] = Y_row[m_zero + j], j < nf (in units of the phase u).
 template <int M>
 struct RowLoadPair {
-  RowValueArgs va;
+  const float2 *pr;       // k_profile's table (null: no fill, no smoothing)
   const float2 *A;        // forward chirp
   int L;                  // window length
   const float *rows;      // block row r: floats rows[r * LDM + n]
-  const RowConst *rc;     // per block row (shared memory)
-  int row0, n_rows;       // row0: the block's first window row
+  const float *mz;        // per block row: z factor (0 past the batch)
+  const int *slot;        // per block row
   __device__ float2 operator()(int f, int n) const {
     if (n >= L) return make_float2(0.f, 0.f);
     constexpr int LD = FftPlan<M>::LDM;
-    float re = 0.f, im = 0.f;
     const int ra = 2 * f, rb = 2 * f + 1;
-    // the deposit holds the real row's atom sum r (deposit_rows<.., REAL>):
-    // the grid value there is d_value_row of r u, projected back on u
-    if (row0 + ra < n_rows) re = d_value_row_real(va, rc[ra], n, rows[ra * LD + n]);
-    if (row0 + rb < n_rows) im = d_value_row_real(va, rc[rb], n, rows[rb * LD + n]);
+    float re = rows[ra * LD + n], im = rows[rb * LD + n];
+    if (pr) {
+      // the rows are mostly of one slice: one table entry for both
+      const float2 t = __ldg(pr + (size_t)slot[ra] * L + n);
+      const float2 u = slot[ra] == slot[rb] ? t : __ldg(pr + (size_t)slot[rb] * L + n);
+      re = d_value_row_real(t, mz[ra], re);
+      im = d_value_row_real(u, mz[rb], im);
+    }
     return cmul(make_float2(re, im), __ldg(A + n));
   }
 };
@@ -126,8 +129,11 @@ k_row_czt_real(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
   const int row0 = blockIdx.x * 2 * NB;
   deposit_rows<2 * NB, NT, false, true>(a, cz.L, slice0, n_sl, n_rows, row0, buf,
                                         LDM, rs);
-  RowLoadPair<M> ld{row_value_args(a), cz.A, cz.L, reinterpret_cast<const float *>(buf),
-                    rs.k, row0, n_rows};
+  __shared__ float mz[2 * NB];
+  if (threadIdx.x < 2 * NB) mz[threadIdx.x] = row_factor(row_value_args(a), rs.k[threadIdx.x]);
+  __syncthreads();
+  RowLoadPair<M> ld{a.fill || a.smooth_on ? a.pr : nullptr, cz.A, cz.L,
+                    reinterpret_cast<const float *>(buf), mz, rs.slot};
   fft_run<M, NB, NT, false, 1, false, 0, false, HALF, false>(buf, tw, nullptr, ld,
                                                             NoStore());
   // the inverse transform stays in shared memory (natural order; with HALF
@@ -145,8 +151,8 @@ k_row_czt_real(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
       const float2 ya = make_float2(0.5f * (X.x + Xm.x), 0.5f * (X.y - Xm.y));
       const float2 yb = make_float2(0.5f * (X.y + Xm.y), -0.5f * (X.x - Xm.x));
       const int ra = row0 + 2 * f, rb = ra + 1;
-      if (ra < n_rows) F1[(size_t)ra * nf + j] = cmul(rs.k[2 * f].u, ya);
-      if (rb < n_rows) F1[(size_t)rb * nf + j] = cmul(rs.k[2 * f + 1].u, yb);
+      if (ra < n_rows) F1[(size_t)ra * nf + j] = ya;
+      if (rb < n_rows) F1[(size_t)rb * nf + j] = yb;
     }
   }
 }

@@ -140,7 +140,7 @@ __global__ void k_zscatter(const double *xyz, const float2 *f,
                            const gw_structure *st, const int *zidx, int g,
                            const unsigned long long *zmin_ord, double inv_r,
                            int *cursor, double *xyz_s, float4 *xyf_s,
-                           int *perm, float *fz_s) {
+                           int *perm, float *fz_s, int real) {
   const gw_structure s = st[blockIdx.y];
   int *cur = cursor + (size_t)blockIdx.y * (g + 1);
   const double zmin = ord_dbl(zmin_ord[blockIdx.y]);
@@ -152,7 +152,12 @@ __global__ void k_zscatter(const double *xyz, const float2 *f,
     xyz_s[3 * (size_t)pos] = xyz[3 * a];
     xyz_s[3 * (size_t)pos + 1] = xyz[3 * a + 1];
     xyz_s[3 * (size_t)pos + 2] = xyz[3 * a + 2];
-    const float2 fa = f[a];
+    float2 fa = f[a];
+    if (real) {
+      // in units of the structure's phase (rounded once from float64)
+      const double mag = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im);
+      fa = make_float2((float)(((double)fa.x * s.avg_f_re + (double)fa.y * s.avg_f_im) / mag), 0.f);
+    }
     xyf_s[pos] = make_float4((float)xyz[3 * a], (float)xyz[3 * a + 1], fa.x, fa.y);
     perm[pos] = (int)a;
     if (fz_s) {
@@ -290,9 +295,16 @@ __global__ void k_yminmax(SliceArgs a, int slice0, int n) {
     // stays inside it
     const int sl = first + threadIdx.x;
     const gw_structure s = a.st[sl / a.n_phi];
-    const float2 c = make_float2((float)GW_DMUL(s.avg_f_re, s.max_voxels),
-                                 (float)GW_DMUL(s.avg_f_im, s.max_voxels));
+    double cr = GW_DMUL(s.avg_f_re, s.max_voxels), ci = GW_DMUL(s.avg_f_im, s.max_voxels);
+    if (a.real) {  // real grids are in units of the structure's phase
+      cr = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im) * s.max_voxels;
+      ci = 0.0;
+    }
+    const float2 c = make_float2((float)cr, (float)ci);
     const bool bg = !a.plain && (a.fill || a.smooth_on);
+    // the q = 0 pixel is by far the largest: rounded once
+    const double g2 = bg ? (double)a.g * (double)a.g : 0.0;
+    a.sdc[sl] = make_float2((float)(cr * g2), (float)(ci * g2));
     a.sconst[sl] = bg ? make_float4(c.x, c.y, 0.f, 0.f)
                       : make_float4(0.f, 0.f, c.x, c.y);
   }
@@ -412,31 +424,16 @@ __global__ void k_profile(SliceArgs a, int slice0) {
   const int i0 = blockIdx.y * blockDim.x + threadIdx.x;
   const int di = gridDim.y * blockDim.x;
   const bool lead = blockIdx.y == 0 && threadIdx.x == 0;
-  if (a.fill) {
-    const double base = a.clbase[sl];
-    for (int yy = i0; yy < a.Ly; yy += di) {
-      int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
-      const double x = GW_DMUL((double)yi, a.r);
-      const double len = collapse_length(ph, s.y_bound, s.x_bound, base, x);
-      const double nm = GW_DSUB(s.max_voxels, floor_div_exact(len, a.r, a.inv_r));
-      const double n_missing = (double)(long long)nm;
-      double re = GW_DMUL(n_missing, s.avg_f_re);
-      double im = GW_DMUL(n_missing, s.avg_f_im);
-      if (bg) { re -= cre; im -= cim; }
-      a.amo[(size_t)blockIdx.x * a.Ly + yy] = make_float2((float)re, (float)im);
-    }
-  }
+  // fill values: n_missing times the average voxel f, less the background
+  auto missing = [&](int yi) {
+    const double x = GW_DMUL((double)yi, a.r);
+    const double len = collapse_length(ph, s.y_bound, s.x_bound, a.clbase[sl], x);
+    const double nm = GW_DSUB(s.max_voxels, floor_div_exact(len, a.r, a.inv_r));
+    return (double)(long long)nm;
+  };
+  int ys = 0, ye = 0, zs = 0, ze = 0;
   if (a.smooth_on) {
-    int ys, ye, zs, ze;
     plateau(a, e, ys, ye, zs, ze);
-    for (int yy = i0; yy < a.Ly; yy += di) {
-      int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
-      a.my[(size_t)blockIdx.x * a.Ly + yy] = smooth_at(yi, ys, ye, a.g, a.radius, a.gw);
-    }
-    for (int zz = i0; zz < a.Lz; zz += di) {
-      int zi = a.z_lo + zz; if (zi < 0) zi += a.g; if (zi >= a.g) zi -= a.g;
-      a.mz[(size_t)blockIdx.x * a.Lz + zz] = smooth_at(zi, zs, ze, a.g, a.radius, a.gw);
-    }
     // the smoothing support must lie inside the transformed window
     if (lead && a.Ly < a.g) {
       int l = a.y_lo - 1; if (l < 0) l += a.g;
@@ -455,21 +452,39 @@ __global__ void k_profile(SliceArgs a, int slice0) {
     }
   }
   if (a.pr) {
-    // real grids: the row kernel's per-column table (d_value_row_real);
-    // this thread's own amo and my entries, written above
-    const float2 u = unit_phase(s);
-    const float nan = __int_as_float(0x7fc00000);
+    // one real function of y: the fill (or minus the background) in units
+    // of the structure's phase, and the factor of the deposited sums
+    const double mag = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im);
     for (int yy = i0; yy < a.Ly; yy += di) {
-      const size_t o = (size_t)blockIdx.x * a.Ly + yy;
-      float x = 0.f;
+      int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
+      float t = (float)(-mag * s.max_voxels), m = 1.f;
+      if (a.smooth_on) m = smooth_at(yi, ys, ye, a.g, a.radius, a.gw);
       if (a.fill) {
-        int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
-        const float2 am = a.amo[o];
-        x = (yi > e.x && yi < e.y) ? am.x * u.x + am.y * u.y : nan;
+        if (yi > e.x && yi < e.y) t = (float)((missing(yi) - s.max_voxels) * mag);
+        else t = m = 0.f;
       }
-      a.pr[o] = make_float2(x, a.smooth_on ? a.my[o] : 1.f);
+      a.pr[(size_t)blockIdx.x * a.Ly + yy] = make_float2(t, m);
+    }
+  } else if (a.fill) {
+    for (int yy = i0; yy < a.Ly; yy += di) {
+      int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
+      const double n_missing = missing(yi);
+      double re = GW_DMUL(n_missing, s.avg_f_re);
+      double im = GW_DMUL(n_missing, s.avg_f_im);
+      if (bg) { re -= cre; im -= cim; }
+      a.amo[(size_t)blockIdx.x * a.Ly + yy] = make_float2((float)re, (float)im);
     }
   }
+  if (a.smooth_on && !a.pr)
+    for (int yy = i0; yy < a.Ly; yy += di) {
+      int yi = a.y_lo + yy; if (yi < 0) yi += a.g; if (yi >= a.g) yi -= a.g;
+      a.my[(size_t)blockIdx.x * a.Ly + yy] = smooth_at(yi, ys, ye, a.g, a.radius, a.gw);
+    }
+  if (a.smooth_on)
+    for (int zz = i0; zz < a.Lz; zz += di) {
+      int zi = a.z_lo + zz; if (zi < 0) zi += a.g; if (zi >= a.g) zi -= a.g;
+      a.mz[(size_t)blockIdx.x * a.Lz + zz] = smooth_at(zi, zs, ze, a.g, a.radius, a.gw);
+    }
 }
 
 // ---------------------------------------------------------- geometry tables
@@ -950,6 +965,8 @@ __global__ void k_shell_double(const unsigned short *codes, int W, int off,
 // sorted arrays and index code the row kernel uses.
 __global__ void k_debug_window(SliceArgs a, int sl, float2 *win) {
   const int t = sl / a.n_phi;
+  // real grids keep their atoms' values in units of the structure's phase
+  const float2 u = a.real ? unit_phase(a.st[t]) : make_float2(1.f, 0.f);
   for (int zz = blockIdx.x; zz < a.Lz; zz += gridDim.x) {
     int lo, mid, hi;
     row_atoms(a, t, zz, lo, mid, hi);
@@ -958,8 +975,9 @@ __global__ void k_debug_window(SliceArgs a, int sl, float2 *win) {
       if (!a.bil) {
         int yy;
         if (deposit_column(a, at, sl, yy) && yy < a.Ly) {
-          atomicAdd(&row[yy].x, a.xyf_s[at].z);
-          atomicAdd(&row[yy].y, a.xyf_s[at].w);
+          const float2 fv = cmul(make_float2(a.xyf_s[at].z, a.xyf_s[at].w), u);
+          atomicAdd(&row[yy].x, fv.x);
+          atomicAdd(&row[yy].y, fv.y);
         }
       } else {
         int i0;
@@ -1133,13 +1151,13 @@ SliceArgs slice_args(gw_voxel_plan *P) {
   a.sigma = (float)P->p.smooth; a.radius = P->radius; a.plain = P->plain;
   a.xyz = P->d_xyz; a.f = P->d_f; a.zidx = P->d_zidx; a.st = P->d_structs;
   a.xyz_s = P->d_xyz_s; a.xyf_s = P->d_xyf_s; a.rowstart = P->d_rowstart;
-  a.fz_s = P->d_fz_s; a.bil = P->bil;
+  a.fz_s = P->d_fz_s; a.bil = P->bil; a.real = P->real;
   a.ybnd = P->d_ybnd;
   a.roff = P->d_roff;
   a.zstat = P->d_zstat; a.ymax_ord = P->d_ymax; a.extflag = P->d_extflag;
   a.ph = P->d_phis; a.clbase = P->d_clbase; a.ymin_ord = P->d_ymin;
   a.ext = P->d_ext; a.amo = P->d_amo; a.my = P->d_my; a.pr = P->d_pr;
-  a.mz = P->d_mz; a.gw = P->d_gw; a.sconst = P->d_sconst; a.err = P->ctx->d_err;
+  a.mz = P->d_mz; a.gw = P->d_gw; a.sconst = P->d_sconst; a.sdc = P->d_sdc; a.err = P->ctx->d_err;
   return a;
 }
 
@@ -1182,7 +1200,7 @@ int enqueue_prep(gw_voxel_plan *P) {
     gw::KTimer tm(ctx, GW_K_PREP);
     k_zscatter<<<dim3(nblk_at, P->n_struct), 256, 0, st>>>(
         P->d_xyz, P->d_f, P->d_structs, P->d_zidx, P->g, P->d_zmin, P->inv_r,
-        P->d_cursor, P->d_xyz_s, P->d_xyf_s, P->d_perm, P->d_fz_s);
+        P->d_cursor, P->d_xyz_s, P->d_xyf_s, P->d_perm, P->d_fz_s, P->real ? 1 : 0);
     GW_LAUNCHED(ctx);
   }
   return GW_OK;
@@ -1559,12 +1577,10 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   GW_CUDA(cudaStreamSynchronize(P->ctx->stream));  // no pass reads the buffers
   if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
   if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
-  float2 *f1 = nullptr;
-  GW_TRY(alloc(&f1, (size_t)P->S * P->Lz * P->Nc, &P->bytes));
   void *drop[] = {P->d_F1, P->d_pr, P->d_heavy, P->d_zmulti, P->d_lptr, P->d_lent,
                   P->d_zptr, P->d_zrows, P->d_G};
   for (void *q : drop) gw::dev_free(q);
-  P->d_F1 = f1;
+  P->d_F1 = nullptr;
   P->d_pr = nullptr;
   P->d_heavy = P->d_zmulti = P->d_lptr = P->d_zptr = P->d_zrows = nullptr;
   P->d_lent = nullptr;
@@ -1573,6 +1589,7 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   P->n_heavy = P->n_zmulti = 0;
   P->real = false;
   P->Nf = P->Nc;
+  GW_TRY(alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &P->bytes));
   GW_TRY(col_map_dispatch(P));
   return gather_setup(P);
 }
@@ -1867,6 +1884,7 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_ymin, P->n_slices, &B)) ||
       (st = alloc(&P->d_ext, P->n_slices, &B)) ||
       (st = alloc(&P->d_sconst, P->n_slices, &B)) ||
+      (st = alloc(&P->d_sdc, P->n_slices, &B)) ||
       (st = alloc(&P->d_colofs, (size_t)n_phi * P->Nc, &B)) ||
       (st = alloc(&P->d_C2, (size_t)P->W * P->W, &B)) ||
       (st = (p->accum == GW_ACCUM_KAHAN32
@@ -1881,12 +1899,12 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_rowstart, (size_t)n_struct * (g + 2), &B)) ||
       (st = alloc(&P->d_cursor, (size_t)n_struct * (g + 1), &B)) ||
       (st = alloc(&P->d_zstat, n_struct, &B)) ||
-      (st = alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &B)) ||
       (st = alloc(&P->d_amo, (size_t)P->n_slices * P->Ly, &B)) ||
       (P->real && (st = alloc(&P->d_pr, (size_t)P->n_slices * P->Ly, &B))) ||
       (st = alloc(&P->d_my, (size_t)P->n_slices * P->Ly, &B)) ||
       (st = alloc(&P->d_mz, (size_t)P->n_slices * P->Lz, &B)) ||
       (st = upload(&P->d_roff, P->roff_host, &B)) ||
+      (st = alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &B)) ||
       (st = col_map_dispatch(P))) {
     gw_voxel_plan_destroy(P);
     return st;
@@ -1928,7 +1946,7 @@ extern "C" int gw_voxel_plan_destroy(gw_voxel_plan *P) {
                   P->d_twz, P->d_gw, P->d_colofs, P->d_rowofs, P->d_C1,
                   P->d_C2, P->d_sum, P->d_sumk, P->d_f0, P->d_iq64,
                   P->d_iq32, P->d_F1, P->d_amo, P->d_my, P->d_mz,
-                  P->d_sconst, P->d_xyz_s, P->d_xyf_s, P->d_fz_s,
+                  P->d_sconst, P->d_sdc, P->d_xyz_s, P->d_xyf_s, P->d_fz_s,
                   P->d_perm, P->d_ybnd, P->d_roff, P->d_zhist, P->d_rowstart,
                   P->d_cursor, P->d_zstat, P->d_ymax, P->d_extflag,
                   P->d_shell, P->d_f_shells, P->d_structs_shells, P->d_zf0,

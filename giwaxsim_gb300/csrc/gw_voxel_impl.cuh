@@ -31,12 +31,14 @@ struct SliceArgs {
   int radius;
   int plain;
   int bil;             // bilinear deposit (two rows x two columns per atom)
+  int real;            // real grids
   // arrays
   const double *xyz;   // atoms in input order
   const float2 *f;
   const int *zidx;
   const double *xyz_s; // atoms sorted by z index within each structure
-  const float4 *xyf_s; // sorted atoms: float32 (x, y) and f (re, im)
+  const float4 *xyf_s; // sorted atoms: float32 (x, y) and f (re, im); real
+                       // grids: (Re(f conj(u)), 0), u the structure's phase
   const float *fz_s;   // bilinear: fractional z position of the sorted atoms
   unsigned *ybnd;      // per slice: float32 bounds on the y extremes (ordered)
   const int *roff;     // per slice: first window row (n_slices+1 entries),
@@ -51,12 +53,13 @@ struct SliceArgs {
   int4 *ext;  // y_min, y_max, z_min, z_max (valid atoms)
   float2 *amo;
   float *my, *mz;
-  // real grids: per slot and window column, (the fill value projected on
-  // the structure's phase, NaN outside the slice's y extent; the y
-  // smoothing factor, 1 without smoothing), made by k_profile
+  // real grids: per slot and window column (t, m), the grid value being
+  // (r + t) m mz for the deposited sum r: the fill (or minus the background)
+  // and the y smoothing factor; (0, 0) outside the slice's y extent
   float2 *pr;
   const float *gw;  // gaussian weights, 2*radius+1
   float4 *sconst;   // per slice: (Cbg.re, Cbg.im, Cd.re, Cd.im)
+  float2 *sdc;      // per slice: Cbg g^2, the background's DFT (at q = 0)
   int *err;
 };
 
@@ -229,8 +232,6 @@ struct RowConst {
   float mz;        // z smoothing factor of the row (1 when smoothing is off)
   int zin;         // the row's z lies inside [e.z, e.w)
   int slot;
-  float2 u;        // unit phase of the structure's average voxel f (real
-                   // grids: the row is u times a real row)
 };
 
 // Unit phase of a structure's average voxel f (real grids: its slice grids
@@ -252,7 +253,6 @@ __device__ __forceinline__ RowConst row_const(const SliceArgs &a, int slot,
   const int zi = window_row_to_z(a, zz);
   k.zin = zi >= k.e.z && zi < k.e.w;
   k.slot = slot;
-  k.u = unit_phase(a.st[sl / a.n_phi]);
   return k;
 }
 
@@ -296,26 +296,16 @@ __device__ __forceinline__ float2 d_value_row(const SliceArgs &a,
   return d_value_row(row_value_args(a), k, yy, dep);
 }
 
-// Real grids: Re(d_value_row(a, k, yy, r u) conj(u)) for the real row sum
-// r.  The fill and smoothing values (amo, cd, cbg) are multiples of u, so
-// the projection is taken term by term, in float32 (|u| = 1); the slot's
-// projected fill value, its y-extent test and the y smoothing factor come
-// as one 8-byte load of the k_profile table pr.
-__device__ __forceinline__ float d_value_row_real(const RowValueArgs &a,
-                                                  const RowConst &k, int yy,
-                                                  float r) {
-  const float cdr = k.cd.x * k.u.x + k.cd.y * k.u.y;
-  // (k_profile runs, and makes the table, with fill or smoothing only)
-  const float2 t = (a.fill || a.smooth_on) ? a.pr[(size_t)k.slot * a.Ly + yy]
-                                           : make_float2(0.f, 1.f);
-  float v;
-  if (a.fill) v = (k.zin && t.x == t.x) ? r + t.x : cdr;
-  else v = r - (k.cbg.x * k.u.x + k.cbg.y * k.u.y);
-  if (a.smooth_on) {
-    const float m = k.mz * t.y;
-    v = v * m + cdr * (1.f - m);
-  }
-  return v;
+// Real grids: the value of d_value_row in units of the structure's phase,
+// for the real row sum r.  The window excludes the background (batched
+// plans), so outside the slice's extents the value is 0: mz is the row's z
+// factor, 0 for rows outside them (fill).
+__device__ __forceinline__ float d_value_row_real(float2 t, float mz, float r) {
+  return (r + t.x) * (mz * t.y);
+}
+
+__device__ __forceinline__ float row_factor(const RowValueArgs &a, const RowConst &k) {
+  return a.fill && !k.zin ? 0.f : k.mz;
 }
 
 // Window column of sorted atom `at` in slice `sl` (nearest-bin deposit):
@@ -427,8 +417,8 @@ struct RowShared {
 // of the batch, row f into buf[f * ldm + 0 .. L) (zeroed first), by shared
 // atomics.  Sets up rs (slot, window row, atom range and constants of every
 // row) and leaves the block synchronised.  REAL (real grids, nearest bin):
-// each atom adds Re(f conj(u)) to the .x of its element only, u the row's
-// unit phase (the row is u times that real row): one shared atomic per atom.
+// float rows, one shared atomic per atom (the row is the structure's unit
+// phase u times that real row; |F|^2 does not see u).
 template <int NB, int NT, bool BIL, bool REAL = false>
 __device__ __forceinline__ void deposit_rows(const SliceArgs &a, int L,
                                              int slice0, int n_sl, int n_rows,
@@ -461,6 +451,9 @@ __device__ __forceinline__ void deposit_rows(const SliceArgs &a, int L,
     if (row < n_rows) {
       rs.k[f] = row_const(a, slot, slice0 + slot, zz);
       rs.d[f] = dep_row(a, slice0 + slot);
+    } else if (REAL) {
+      // a row past the batch: a zero factor at a valid slot
+      rs.k[f] = RowConst{};
     }
   }
   __syncthreads();
@@ -481,8 +474,7 @@ __device__ __forceinline__ void deposit_rows(const SliceArgs &a, int L,
       if (deposit_column(a, rs.d[f], make_float2(q.x, q.y), at, yy)) {
         if (yy < a.Ly) {
           if constexpr (REAL) {
-            const float2 u = rs.k[f].u;
-            atomicAdd(rbuf + f * ldm + yy, fmaf(q.z, u.x, q.w * u.y));
+            atomicAdd(rbuf + f * ldm + yy, q.z);
           } else {
             atomicAdd(&buf[f * ldm + yy].x, q.z);
             atomicAdd(&buf[f * ldm + yy].y, q.w);
@@ -665,6 +657,7 @@ struct gw_voxel_plan {
   int *d_extflag = nullptr;
   float *d_my = nullptr, *d_mz = nullptr;
   float4 *d_sconst = nullptr;
+  float2 *d_sdc = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int64_t graph_kernels = 0;
