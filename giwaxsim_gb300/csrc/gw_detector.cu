@@ -144,16 +144,16 @@ __global__ void k_det_debug(DetArgs a, int o, int64_t *idx) {
 // otherwise the (pixel, orientation) pair goes to a worklist that
 // k_detector_fix replays with the exact float64 chain.
 struct OrientFast {
+  // an axis whose coordinate is exactly +-0 for every pixel has A = 0, b =
+  // its (clipped) index + 0.5 and d = 0: it gathers that index, certainly
   float A[9];
   float b[3];
   float d[3];
   float w;
-  int fix[3];  // >= 0: the axis' coordinate is exactly +-0 for every pixel
-  int pad;     //       and its (clipped) index is this constant
 };
 constexpr int kOrientFloats = sizeof(OrientFast) / 4;
 
-constexpr int kDetThreads = 256, kDetPix = 2, kDetChunk = 128, kDetFlush = 16;
+constexpr int kDetThreads = 256, kDetChunk = 128, kDetFlush = 16;
 static_assert(kDetChunk % kDetFlush == 0, "orientation chunks hold whole flush groups");
 static_assert(kDetFlush * 2 <= 32, "a flush group's uncertain samples fit one 32-bit mask");
 
@@ -177,95 +177,10 @@ __device__ __forceinline__ bool fast_index(const OrientFast &T, const DetArgs &a
   const float ty = fmaf(T.A[3], x, fmaf(T.A[4], y, fmaf(T.A[5], z, T.b[1])));
   const float tz = fmaf(T.A[6], x, fmaf(T.A[7], y, fmaf(T.A[8], z, T.b[2])));
   int ix, iy, iz;
-  bool ok = fast_axis(tx, T.d[0], a.nx, ix) & fast_axis(ty, T.d[1], a.ny, iy) &
-            fast_axis(tz, T.d[2], a.nz, iz);
-  if (T.fix[0] >= 0 || T.fix[1] >= 0 || T.fix[2] >= 0) {
-    ok = (T.fix[0] >= 0 || fast_axis(tx, T.d[0], a.nx, ix)) &
-         (T.fix[1] >= 0 || fast_axis(ty, T.d[1], a.ny, iy)) &
-         (T.fix[2] >= 0 || fast_axis(tz, T.d[2], a.nz, iz));
-    if (T.fix[0] >= 0) ix = T.fix[0];
-    if (T.fix[1] >= 0) iy = T.fix[1];
-    if (T.fix[2] >= 0) iz = T.fix[2];
-  }
+  const bool ok = fast_axis(tx, T.d[0], a.nx, ix) & fast_axis(ty, T.d[1], a.ny, iy) &
+                  fast_axis(tz, T.d[2], a.nz, iz);
   idx = ((int64_t)iy * a.nx + ix) * a.nz + iz;
   return ok;
-}
-
-__global__ void __launch_bounds__(kDetThreads)
-k_detector_fast(DetArgs a, const OrientFast *ot, double *acc_out, int2 *wl,
-                int *wl_count, int wl_cap) {
-  __shared__ OrientFast s_ot[kDetChunk];
-  const int npx = a.nh * a.nv;
-  const int lane = threadIdx.x & 31;
-  int pix[kDetPix];
-  bool valid[kDetPix];
-  float xf[kDetPix], yf[kDetPix], zf[kDetPix];
-  double x0[kDetPix], y0[kDetPix], z0[kDetPix];
-  double acc[kDetPix];
-  float part[kDetPix], kc[kDetPix];
-#pragma unroll
-  for (int k = 0; k < kDetPix; ++k) {
-    pix[k] = blockIdx.x * (kDetThreads * kDetPix) + k * kDetThreads + threadIdx.x;
-    valid[k] = pix[k] < npx;
-    x0[k] = y0[k] = z0[k] = 0.0;
-    if (valid[k]) base_point(a, pix[k] / a.nh, pix[k] % a.nh, x0[k], y0[k], z0[k]);
-    xf[k] = (float)x0[k]; yf[k] = (float)y0[k]; zf[k] = (float)z0[k];
-    acc[k] = 0.0; part[k] = 0.f; kc[k] = 0.f;
-  }
-  for (int c0 = 0; c0 < a.n_orient; c0 += kDetChunk) {
-    const int nc = min(kDetChunk, a.n_orient - c0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < nc * kOrientFloats; t += kDetThreads)
-      reinterpret_cast<float *>(s_ot)[t] = reinterpret_cast<const float *>(ot + c0)[t];
-    __syncthreads();
-    for (int oo = 0; oo < nc; ++oo) {
-      const OrientFast &T = s_ot[oo];
-      const int o = c0 + oo;
-#pragma unroll
-      for (int k = 0; k < kDetPix; ++k) {
-        int64_t idx;
-        const bool ok = fast_index(T, a, xf[k], yf[k], zf[k], idx);
-        const bool need = valid[k] && !ok;
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        bool inline_exact = false;
-        if (m) {
-          int base = 0;
-          const int leader = __ffs(m) - 1;
-          if (lane == leader) base = atomicAdd(wl_count, __popc(m));
-          base = __shfl_sync(0xffffffffu, base, leader);
-          if (need) {
-            const int slot = base + __popc(m & ((1u << lane) - 1u));
-            if (slot < wl_cap) wl[slot] = make_int2(pix[k], o);
-            else inline_exact = true;
-          }
-        }
-        float v = 0.f;
-        if (valid[k] && ok) v = __ldg(a.iq + idx);
-        if (inline_exact) v = __ldg(a.iq + gather_index(a, o, x0[k], y0[k], z0[k]));
-        if (valid[k] && (ok || inline_exact)) {
-          if (!a.kahan) {
-            part[k] = fmaf(v, T.w, part[k]);
-          } else {
-            const float yv = v * T.w - kc[k];
-            const float t = part[k] + yv;
-            kc[k] = (t - part[k]) - yv;
-            part[k] = t;
-          }
-        }
-      }
-      // float32 partial sums of kDetFlush orientations, float64 across them
-      if (!a.kahan && ((o + 1) % kDetFlush == 0)) {
-#pragma unroll
-        for (int k = 0; k < kDetPix; ++k) { acc[k] += f2d_exact(part[k]); part[k] = 0.f; }
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kDetPix; ++k) {
-    if (!valid[k]) continue;
-    acc_out[pix[k]] = a.kahan ? f2d_exact(part[k]) - f2d_exact(kc[k])
-                              : acc[k] + f2d_exact(part[k]);
-  }
 }
 
 // ------------------------------------------------------------ plane mode
@@ -276,7 +191,7 @@ k_detector_fast(DetArgs a, const OrientFast *ot, double *acc_out, int2 *wl,
 // from shared memory when the plane fits, else from global memory through
 // L1.  Blocks own 16 x 32 pixel tiles, so that per orientation a block's
 // samples cover a compact patch of the plane.  Indices, worklist decisions
-// and the per-pixel accumulation order are those of k_detector_fast; only
+// and the per-pixel accumulation order are those of the general mode; only
 // the order in which k_detector_fix atomically adds the replayed samples
 // differs (it is scheduling order in both).
 struct PlaneArgs {
@@ -457,6 +372,146 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
     if (valid[k]) acc_out[pix[k]] = acc[k] + f2d_exact(part[k]);
 }
 
+// ------------------------------------------------------------ general mode
+// One orientation of the general gather, for two pixels a thread: (x, y)
+// pairs of the coefficients of those two axes, (z, z) pairs of the z axis',
+// so that an (x, y) pair of one pixel and a z pair of both pixels are each
+// one paired float32 instruction.  Six 16-byte words.
+struct __align__(16) GenOrient {
+  float2 ax, ay, az, c, d;       // x and y axes: of pixel x, y, z; constant; bound
+  float2 zx, zy, zz, zc, zd;     // z axis, twice
+  float2 w;                      // weight, -
+  float2 pad;
+};
+static_assert(sizeof(GenOrient) == 96, "six 16-byte words per orientation");
+
+// Every orientation's samples of a 32 x 32 pixel tile, two pixels a thread,
+// gathered from the whole I(q).  The indices, certainty tests and order of
+// the sums are those of fast_index with each floor taken by one addition
+// rounded toward minus infinity (as in plane_index); an index is the 32-bit
+// sum of the rounded additions' bit patterns less a constant, which is exact
+// modulo 2^32 (I(q) has fewer than 2^32 elements).  Tiles keep a block's
+// samples of one orientation within a small patch of the volume.
+// 2880 orientations of 500 x 500 pixels in 203^3: 4.75 ms with one axis at a
+// time, rows of 512 pixels a block and 64-bit indices, 1.37 ms so.
+template <bool ZX, bool KAHAN>
+__global__ void __launch_bounds__(kPlThreads)
+k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, int *wl_count,
+                   int wl_cap) {
+  constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+  constexpr int KP = 2;
+  static_assert(kPlTH * kPlTW == KP * kPlThreads, "two pixels a thread");
+  static_assert(kDetFlush * KP <= 32, "a group's uncertain samples fit one mask");
+  __shared__ GenOrient s_ot[kDetChunk];
+  const int tiles_x = (a.nh + kPlTW - 1) / kPlTW;
+  const int j = (blockIdx.x % tiles_x) * kPlTW + (threadIdx.x % kPlTW);
+  const int ib = (blockIdx.x / tiles_x) * kPlTH + threadIdx.x / kPlTW;
+  const float mx = (float)(a.nx - 1), my = (float)(a.ny - 1), mz = (float)(a.nz - 1);
+  const unsigned nx = a.nx, nz = a.nz;
+  const unsigned base = (0x4B400000u * nx + 0x4B400000u) * nz + 0x4B400000u;
+  int pix[KP];
+  bool valid[KP];
+  float xf[KP], yf[KP], zf[KP], part[KP], kc[KP];
+  double acc[KP];
+#pragma unroll
+  for (int k = 0; k < KP; ++k) {
+    const int i = ib + k * (kPlThreads / kPlTW);
+    valid[k] = i < a.nv && j < a.nh;
+    pix[k] = valid[k] ? i * a.nh + j : 0;
+    double x0 = 0.0, y0 = 0.0, z0 = 0.0;
+    if (valid[k]) base_point(a, i, j, x0, y0, z0);
+    xf[k] = (float)x0; yf[k] = (float)y0; zf[k] = (float)z0;
+    acc[k] = 0.0;
+    part[k] = kc[k] = 0.f;
+  }
+  const float2 px = make_float2(xf[0], xf[1]), py = make_float2(yf[0], yf[1]),
+               pz = make_float2(zf[0], zf[1]);
+  const float2 mg = make_float2(kMagic, kMagic);
+  auto add = [&](int k, float v, float w) {
+    if (!KAHAN) {
+      part[k] = fmaf(v, w, part[k]);
+    } else {
+      const float y = v * w - kc[k];
+      const float t = part[k] + y;
+      kc[k] = (t - part[k]) - y;
+      part[k] = t;
+    }
+  };
+  for (int c0 = 0; c0 < a.n_orient; c0 += kDetChunk) {
+    const int nc = min(kDetChunk, a.n_orient - c0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nc * 6; t += kPlThreads)
+      reinterpret_cast<float4 *>(s_ot)[t] = reinterpret_cast<const float4 *>(ot + c0)[t];
+    __syncthreads();
+    for (int g0 = 0; g0 < nc; g0 += kDetFlush) {
+      const int ge = min(g0 + kDetFlush, nc);
+      unsigned need = 0;  // bit (oo - g0) KP + k: an uncertain sample
+#pragma unroll 2
+      for (int oo = g0; oo < ge; ++oo) {
+        const float4 *q = reinterpret_cast<const float4 *>(s_ot + oo);
+        const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
+        const float w = s_ot[oo].w.x;
+        const float2 cx = make_float2(q0.x, q0.y), cy = make_float2(q0.z, q0.w),
+                     cz = make_float2(q1.x, q1.y), cc = make_float2(q1.z, q1.w),
+                     cd = make_float2(q2.x, q2.y);
+        // z axis of both pixels
+        float2 t = __ffma2_rn(make_float2(q3.x, q3.y), py,
+                              __ffma2_rn(make_float2(q3.z, q3.w), pz, make_float2(q4.x, q4.y)));
+        if (!ZX) t = __ffma2_rn(make_float2(q2.z, q2.w), px, t);
+        const float2 zd = make_float2(q4.z, q4.w);
+        const float2 zhi = __fadd2_rn(t, zd), zlo = f2_sub(t, zd);
+        const float2 zr = __fadd2_rd(
+            make_float2(fminf(fmaxf(zhi.x, 0.f), mz), fminf(fmaxf(zhi.y, 0.f), mz)), mg);
+        const float2 zfl = f2_sub(zr, mg);
+#pragma unroll
+        for (int k = 0; k < KP; ++k) {
+          const float2 yy = make_float2(yf[k], yf[k]), zz = make_float2(zf[k], zf[k]);
+          float2 u = __ffma2_rn(cy, yy, __ffma2_rn(cz, zz, cc));
+          if (!ZX) u = __ffma2_rn(cx, make_float2(xf[k], xf[k]), u);
+          const float2 hi = __fadd2_rn(u, cd), lo = f2_sub(u, cd);
+          const float2 r = __fadd2_rd(
+              make_float2(fminf(fmaxf(hi.x, 0.f), mx), fminf(fmaxf(hi.y, 0.f), my)), mg);
+          const float2 fl = f2_sub(r, mg);
+          const bool ok = (fmaxf(lo.x, 0.f) >= fl.x) & (fmaxf(lo.y, 0.f) >= fl.y) &
+                          (fmaxf(k ? zlo.y : zlo.x, 0.f) >= (k ? zfl.y : zfl.x));
+          const unsigned idx = (__float_as_uint(r.y) * nx + __float_as_uint(r.x)) * nz +
+                               __float_as_uint(k ? zr.y : zr.x) - base;
+          if (valid[k] && ok) add(k, __ldg(a.iq + idx), w);
+          need |= (unsigned)(valid[k] && !ok) << ((oo - g0) * KP + k);
+        }
+      }
+      // uncertain samples: to the worklist (k_detector_fix), or replayed
+      // here once it is full
+      if (__any_sync(0xffffffffu, need != 0)) {
+        while (need) {
+          const int b = __ffs(need) - 1;
+          need &= need - 1;
+          const int k = b % KP, o = c0 + g0 + b / KP, p = k ? pix[1] : pix[0];
+          const int slot = atomicAdd(wl_count, 1);
+          if (slot < wl_cap) {
+            wl[slot] = make_int2(p, o);
+          } else {
+            double x, y, z;
+            base_point(a, p / a.nh, p % a.nh, x, y, z);
+            const float v = __ldg(a.iq + gather_index(a, o, x, y, z));
+            if (k == 0) add(0, v, (float)a.w[o]);
+            else add(1, v, (float)a.w[o]);
+          }
+        }
+      }
+      // float32 partial sums of kDetFlush orientations, float64 across them
+      if (!KAHAN && ge - g0 == kDetFlush) {
+#pragma unroll
+        for (int k = 0; k < KP; ++k) { acc[k] += f2d_exact(part[k]); part[k] = 0.f; }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KP; ++k)
+    if (valid[k])
+      acc_out[pix[k]] = KAHAN ? f2d_exact(part[k]) - f2d_exact(kc[k]) : acc[k] + f2d_exact(part[k]);
+}
+
 // Exact float64 replay of the worklist's (pixel, orientation) pairs.
 __global__ void k_detector_fix(DetArgs a, const int2 *wl, const int *wl_count,
                                int wl_cap, double *acc) {
@@ -581,6 +636,7 @@ struct gw_detector_plan {
   bool plane_set = false;
   double *d_plane64 = nullptr;
   PlaneOrient *d_po = nullptr;
+  GenOrient *d_go = nullptr;    // general mode
   bool zero_x = false;  // every pixel's x is +-0 after the init rotations
   bool executed = false;
 };
@@ -697,6 +753,7 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
     }
     P->zero_x = zero0[0];
     std::vector<OrientFast> ot(n_orient);
+    std::vector<int> fix(3 * (size_t)n_orient);  // index of an exactly +-0 axis, or -1
     for (int o = 0; o < n_orient; ++o) {
       bool zero[3] = {zero0[0], zero0[1], zero0[2]};
       for (int r = 0; r < rn[o]; ++r) {
@@ -704,15 +761,6 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
         propagate(rot_R + 9 * (rs[o] + r), zero, nz);
         std::copy(nz, nz + 3, zero);
       }
-      for (int c = 0; c < 3; ++c) {
-        ot[o].fix[c] = -1;
-        if (zero[c]) {
-          double k = floor_div_exact(0.0 - qmin[c], p->dq, inv_dq);
-          k = std::min(std::max(k, 0.0), (double)(dims[c] - 1));
-          ot[o].fix[c] = (int)k;
-        }
-      }
-      ot[o].pad = 0;
       double M[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
       for (int r = 0; r < rn[o]; ++r) {
         const double *R = rot_R + 9 * (rs[o] + r);
@@ -730,6 +778,15 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
         }
         ot[o].b[c] = (float)(-qmin[c] * inv_dq);
         ot[o].d[c] = (float)(10.0 * std::ldexp(1.0, -24) * S + 1e-5);
+        fix[3 * o + c] = -1;
+        if (zero[c]) {
+          double k = floor_div_exact(0.0 - qmin[c], p->dq, inv_dq);
+          k = std::min(std::max(k, 0.0), (double)(dims[c] - 1));
+          fix[3 * o + c] = (int)k;
+          for (int j = 0; j < 3; ++j) ot[o].A[3 * c + j] = 0.f;
+          ot[o].b[c] = (float)k + 0.5f;
+          ot[o].d[c] = 0.f;
+        }
       }
       ot[o].w = (float)weights[o];
     }
@@ -753,14 +810,14 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
       for (int c = 0; c < 3 && P->plane.fa < 0; ++c) {
         bool same = true;
         for (int o = 0; o < n_orient && same; ++o)
-          same = ot[o].fix[c] >= 0 && ot[o].fix[c] == ot[0].fix[c];
+          same = fix[3 * o + c] >= 0 && fix[3 * o + c] == fix[c];
         if (!same) continue;
         // free axes in memory order (y, x, z)
         const int order[3] = {1, 0, 2};
         int fr[2], k = 0;
         for (int q : order)
           if (q != c) fr[k++] = q;
-        PlaneArgs pa{c, ot[0].fix[c], fr[0], fr[1], dims[fr[0]], dims[fr[1]], nullptr};
+        PlaneArgs pa{c, fix[c], fr[0], fr[1], dims[fr[0]], dims[fr[1]], nullptr};
         e = gw::dev_malloc((void **)&P->d_plane, (size_t)pa.nu * pa.nv * sizeof(float));
         if (e != cudaSuccess) {
           gw_detector_plan_destroy(P);
@@ -785,6 +842,21 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
         }
       }
     }
+    if (P->plane.fa < 0) {
+      auto two = [](float v) { return make_float2(v, v); };
+      std::vector<GenOrient> go(n_orient);
+      for (int o = 0; o < n_orient; ++o) {
+        const OrientFast &T = ot[o];
+        go[o] = GenOrient{make_float2(T.A[0], T.A[3]), make_float2(T.A[1], T.A[4]),
+                          make_float2(T.A[2], T.A[5]), make_float2(T.b[0], T.b[1]),
+                          make_float2(T.d[0], T.d[1]), two(T.A[6]), two(T.A[7]), two(T.A[8]),
+                          two(T.b[2]), two(T.d[2]), make_float2(T.w, 0.f), two(0.f)};
+      }
+      if ((st = up(&P->d_go, go.data(), go.size()))) {
+        gw_detector_plan_destroy(P);
+        return st;
+      }
+    }
   }
   *out = P;
   return GW_OK;
@@ -795,7 +867,7 @@ extern "C" int gw_detector_plan_destroy(gw_detector_plan *P) {
   void *ptrs[] = {P->d_h, P->d_v, P->d_init, P->d_rot, P->d_w, P->d_rs,
                   P->d_rn, P->d_iq_own, P->d_acc, P->d_out, P->d_ot, P->d_wl,
                   P->d_wl_count, P->d_gout, P->d_gpix, P->d_giq, P->d_plane,
-                  P->d_po, P->d_plane64};
+                  P->d_po, P->d_plane64, P->d_go};
   for (void *q : ptrs) gw::dev_free(q);
   delete P;
   return GW_OK;
@@ -918,9 +990,20 @@ extern "C" int gw_detector_execute(gw_detector_plan *P) {
       GW_LAUNCHED(P->ctx);
     } else {
       gw::KTimer tm(P->ctx, GW_K_DETECTOR);
-      const int per = kDetThreads * kDetPix;
-      k_detector_fast<<<(npx + per - 1) / per, kDetThreads, 0, P->ctx->stream>>>(
-          a, P->d_ot, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap);
+      const int tiles = ((P->p.n_h + kPlTW - 1) / kPlTW) * ((P->p.n_v + kPlTH - 1) / kPlTH);
+      const bool kh = P->p.accum == GW_ACCUM_KAHAN32;
+      // the 32-bit gather index holds volumes of up to 2^32 elements; larger
+      // ones replay every sample
+      if ((double)a.nx * a.ny * a.nz >= 4294967296.0)
+        k_detector<<<(npx + 127) / 128, 128, 0, P->ctx->stream>>>(a, P->d_acc);
+#define GW_GENERAL(ZX, KH)                                             \
+  k_detector_general<ZX, KH><<<tiles, kPlThreads, 0, P->ctx->stream>>>( \
+      a, P->d_go, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap)
+      else if (P->zero_x && kh) GW_GENERAL(true, true);
+      else if (P->zero_x) GW_GENERAL(true, false);
+      else if (kh) GW_GENERAL(false, true);
+      else GW_GENERAL(false, false);
+#undef GW_GENERAL
       GW_LAUNCHED(P->ctx);
     }
     gw::KTimer tm(P->ctx, GW_K_DET_FIX);

@@ -763,15 +763,21 @@ class PlaneCorners:
         return out
 
 
-def _turns(axis, angles):
-    """rotation_matrix(axis, radians(angle)) of every angle, (n, 3, 3): the
-    same scalar trig and pow, and per element the same expression trees."""
-    ux, uy, uz = axis[0], axis[1], axis[2]
+def _trig(angles):
+    """cos and sin of every angle in degrees, one scalar at a time as
+    rotation_matrix takes them."""
     t = [np.radians(a) for a in angles]
-    c = np.array([np.cos(a) for a in t])
-    s = np.array([np.sin(a) for a in t])
+    return np.array([np.cos(a) for a in t]), np.array([np.sin(a) for a in t])
+
+
+def _turns(axis, trig):
+    """rotation_matrix(axis, angle) of every angle (trig its cos and sin),
+    (n, 3, 3): the same scalar pow, and per element the same expression
+    trees."""
+    ux, uy, uz = axis[0], axis[1], axis[2]
+    c, s = trig
     k = 1 - c
-    R = np.empty((len(t), 3, 3))
+    R = np.empty((len(c), 3, 3))
     R[:, 0, 0] = c + ux ** 2 * k
     R[:, 0, 1] = ux * uy * k - uz * s
     R[:, 0, 2] = ux * uz * k + uy * s
@@ -822,11 +828,12 @@ def orientation_matrices(corners, psis, psi_weights, phis, phi_weights, thetas,
     no_phi = no_theta and all(a == 0 for a in phis)
     full = np.empty((n1, n2, n3, 3, 3, 3))
     full[...] = _IDENTITY
-    R1 = _turns(corners.axis("psi"), psis)
+    phi_trig, theta_trig = _trig(phis), _trig(thetas)
+    R1 = _turns(corners.axis("psi"), _trig(psis))
     full[..., 0, :, :] = R1[:, None, None]
     for i in range(0 if no_phi else n1):
         c1 = corners.rotate(R1[i])
-        R2 = _turns(c1.axis("phi"), phis)
+        R2 = _turns(c1.axis("phi"), phi_trig)
         full[i, :, :, 1] = R2[:, None]
         if no_theta:
             continue
@@ -834,7 +841,7 @@ def orientation_matrices(corners, psis, psi_weights, phis, phi_weights, thetas,
         for j in range(n2):
             axis = c2[j, 1] - c2[j, 0]
             axis /= np.linalg.norm(axis)
-            full[i, j, :, 2] = _turns(axis, thetas)
+            full[i, j, :, 2] = _turns(axis, theta_trig)
     full = full.reshape(-1, 3, 3, 3)
     turns = (full != _IDENTITY).any(axis=(2, 3))
     return turns.sum(1).astype(np.int32), full[turns], w.reshape(-1)
