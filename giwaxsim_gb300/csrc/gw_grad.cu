@@ -139,10 +139,10 @@ __global__ void k_argmin_y(SliceArgs a, int slice0, const int *perm, int *amy) {
   const gw_structure s = a.st[t];
   const unsigned long long mn = a.ymin_ord[sl];
   const double c = a.ph[p].cos_phi, sn = a.ph[p].sin_phi;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-       i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t pos = s.atom_begin + i;
-    if (dbl_ord(rot_y(a.xyz_s + 3 * pos, c, sn)) == mn) atomicMin(amy + sl, perm[pos]);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.ncand[t];
+       i += gridDim.x * blockDim.x) {
+    const int pos = a.cand[s.atom_begin + i];  // (the minimum is a candidate)
+    if (dbl_ord(rot_y(a.xyz_s + 3 * (size_t)pos, c, sn)) == mn) atomicMin(amy + sl, perm[pos]);
   }
 }
 
@@ -694,7 +694,7 @@ extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
     }
     if (P->bil) {
       gw::KTimer tm(ctx, GW_K_MISC);
-      k_argmin_y<<<dim3(std::min(nblk_at, 16), nb), 256, 0, st>>>(a, c0, P->d_perm, G->d_amy);
+      k_argmin_y<<<dim3(std::min(nblk_at, 2), nb), 256, 0, st>>>(a, c0, P->d_perm, G->d_amy);
       GW_LAUNCHED(ctx);
     }
   }

@@ -49,7 +49,7 @@ struct ColBin {
   BinArgs bn;       // by value: no reads through a pointer to the parameters
   const int *cofs;
   const float2 *B;
-  float2 dc;        // the background at q = 0 (SliceArgs.sdc)
+  const float4 *dc; // the background at q = 0 (SliceArgs.sdc)
   int nr, nc, j0, moff;
   int64_t soff;  // sum-grid offset of the slice's structure (separate mode)
   float *gcol;   // gather binning: the slice's pixels of F1 column j0, then
@@ -71,8 +71,9 @@ struct ColBin {
     if ((co < 0 || ro < 0) && (cm < 0 || rm < 0)) return;
     float2 X = cmul(v, __ldg(B + mr));
     if (bn.k0 + m == 0 && bn.kz0 + mr == 0) {
-      X.x += dc.x;
-      X.y += dc.y;
+      const float4 d = *dc;
+      X.x = (X.x + d.z) + d.x;
+      X.y = (X.y + d.w) + d.y;
     }
     const float I = X.x * X.x + X.y * X.y;
     if (gcol) {  // every pixel a voxel line will gather (its own or mirrored)
@@ -150,7 +151,7 @@ k_col_czt_bin(SliceArgs a, CztArgs cz, BinArgs bn, int slice0, int nc, int nf,
     fft_run<M, NB, NT, false, 1, false, 0, true, HALF, false>(buf, tw, nullptr, ld,
                                                              NoStore());
   }
-  ColBin st{bn, cofs, cz.B, a.sdc[sl], cz.N, nc, j0, moff,
+  ColBin st{bn, cofs, cz.B, a.sdc + sl, cz.N, nc, j0, moff,
             bn.sstride * (int64_t)(sl / a.n_phi),
             bn.G ? bn.G + ((size_t)sl * nf + j0) * cz.N : nullptr};
   fft_run<M, NB, NT, true, 0, true, 1, false, false, HALF>(buf, tw, cz.H, NoLoad(), st);

@@ -41,19 +41,129 @@ using namespace gwv;
 namespace {
 
 // ------------------------------------------------------------ structure prep
-__global__ void k_zmin(const double *xyz, const gw_structure *st,
-                       unsigned long long *zmin_ord) {
-  const gw_structure s = st[blockIdx.y];
-  unsigned long long best = ~0ULL;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-       i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
-    double z = xyz[3 * (s.atom_begin + i) + 2];
-    best = min(best, dbl_ord(z));
+// Per structure: the minimum z, and the atoms furthest out in kDirs
+// directions of the x-y plane.  Their convex polygon bounds the atoms that
+// can be at a slice's y extremes: an atom strictly inside it (by a margin far
+// above every rounding here) projects below one of its corners at every phi,
+// so only the others, the candidates, are looked at slice by slice.
+constexpr int kDirs = 8;
+
+__device__ __forceinline__ unsigned flt_ord(float f) {
+  const unsigned u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float ord_flt(unsigned o) {
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+
+// The block's minimum z and outermost atoms (ordered projection << 32 | index
+// in the structure), valid in threads 0 .. kDirs - 1 of the first warp (zbest
+// in thread 0).
+__device__ __forceinline__ void block_extremes(const double *xyz, const gw_structure &s,
+                                               int64_t i0, int64_t stride,
+                                               unsigned long long &zbest,
+                                               unsigned long long &out) {
+  __shared__ unsigned long long sh[kDirs + 1][32];
+  float best[kDirs];
+  unsigned at[kDirs];
+  gwd::sfor<kDirs>([&](auto j) { best[j] = -INFINITY; at[j] = 0u; });
+  unsigned long long z0 = ~0ULL;
+  for (int64_t i = i0; i < s.atom_count; i += stride) {
+    const double *p = xyz + 3 * (s.atom_begin + i);
+    z0 = min(z0, dbl_ord(p[2]));
+    const float x = (float)p[0], y = (float)p[1];
+    gwd::sfor<kDirs>([&](auto j) {
+      constexpr float c = (float)gwd::trig2pi(j, kDirs, false);
+      constexpr float n = (float)gwd::trig2pi(j, kDirs, true);
+      const float v = fmaf(y, n, x * c);
+      if (v > best[j]) { best[j] = v; at[j] = (unsigned)i; }
+    });
   }
-  for (int o = 16; o > 0; o >>= 1)
-    best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0 && best != ~0ULL)
-    atomicMin(zmin_ord + blockIdx.y, best);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) z0 = min(z0, __shfl_xor_sync(0xffffffffu, z0, o));
+  if (lane == 0) sh[kDirs][w] = z0;
+  gwd::sfor<kDirs>([&](auto j) {
+    unsigned long long k = ((unsigned long long)flt_ord(best[j]) << 32) | at[j];
+    for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+    if (lane == 0) sh[j][w] = k;
+  });
+  __syncthreads();
+  zbest = ~0ULL;
+  out = 0;
+  if (threadIdx.x < kDirs)
+    for (int k = 0; k < nw; ++k) out = max(out, sh[threadIdx.x][k]);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < nw; ++k) zbest = min(zbest, sh[kDirs][k]);
+}
+
+__global__ void k_extremes(const double *xyz, const gw_structure *st,
+                           unsigned long long *zmin_ord, unsigned long long *dirs) {
+  unsigned long long z, d;
+  block_extremes(xyz, st[blockIdx.y], blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
+                 (int64_t)gridDim.x * blockDim.x, z, d);
+  if (threadIdx.x < kDirs) atomicMax(dirs + kDirs * blockIdx.y + threadIdx.x, d);
+  if (threadIdx.x == 0) atomicMin(zmin_ord + blockIdx.y, z);
+}
+
+// Counters and minima before a pass's structure kernels.
+__global__ void k_prep_init(int n_struct, int64_t n_hist, int *hist, unsigned long long *zmin_ord,
+                            unsigned long long *dirs, int *ncand, int *any_ext) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t di = (int64_t)gridDim.x * blockDim.x;
+  if (i0 == 0) *any_ext = 0;
+  for (int64_t i = i0; i < n_hist; i += di) hist[i] = 0;
+  for (int64_t i = i0; i < n_struct; i += di) {
+    zmin_ord[i] = ~0ULL;
+    ncand[i] = 0;
+  }
+  for (int64_t i = i0; i < (int64_t)n_struct * kDirs; i += di) dirs[i] = 0;
+}
+
+// The polygon's edges as half planes n . p > c (c holds the margin) in shared
+// memory; without three edges every atom is a candidate.  All threads call.
+struct HullEdges {
+  float4 e[kDirs];  // (n.x, n.y, c, -); a repeated corner: c = -infinity
+};
+__device__ __forceinline__ void hull_edges(const double *xyz, const gw_structure &s,
+                                           const unsigned long long *dirs, HullEdges &h) {
+  __shared__ float2 v[kDirs];
+  __shared__ float reach[kDirs];
+  if (threadIdx.x < kDirs) {
+    const unsigned long long k = dirs[threadIdx.x];
+    const double *p = xyz + 3 * (s.atom_begin + (int64_t)(k & 0xffffffffu));
+    v[threadIdx.x] = make_float2((float)p[0], (float)p[1]);
+    reach[threadIdx.x] = fabsf(ord_flt((unsigned)(k >> 32)));
+  }
+  __syncthreads();
+  if (threadIdx.x < kDirs) {
+    float R = 0.f;
+    int edges = 0;
+    for (int j = 0; j < kDirs; ++j) {
+      const float2 a = v[j], b = v[(j + 1) % kDirs];
+      R = reach[j] > R || reach[j] != reach[j] ? reach[j] : R;
+      edges += a.x != b.x || a.y != b.y;
+    }
+    const float2 a = v[threadIdx.x], b = v[(threadIdx.x + 1) % kDirs];
+    const float ex = b.x - a.x, ey = b.y - a.y, len = sqrtf(ex * ex + ey * ey);
+    // float32 coordinates and products are off by at most about 1e-6 R
+    float2 n = make_float2(0.f, 0.f);
+    float c = edges < 3 ? INFINITY : -INFINITY;
+    if (edges >= 3 && !(len == 0.f)) {
+      n = make_float2(-ey / len, ex / len);
+      c = n.x * a.x + n.y * a.y + 1e-5f * R;
+    }
+    h.e[threadIdx.x] = make_float4(n.x, n.y, c, 0.f);
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ bool hull_inside(const HullEdges &h, float x, float y) {
+  bool in = true;
+#pragma unroll
+  for (int j = 0; j < kDirs; ++j) {
+    const float4 e = h.e[j];
+    in = in & (fmaf(e.x, x, e.y * y) > e.z);
+  }
+  return in;
 }
 
 // z index is phi independent: rotation about z leaves z unchanged
@@ -77,11 +187,10 @@ __global__ void k_zidx_hist(const double *xyz, const gw_structure *st,
 
 // Per structure: exclusive scan of the row histogram into absolute offsets
 // rowstart[0..g+1], scatter cursors, and (largest occupied row, all valid).
-__global__ void __launch_bounds__(1024)
-k_zscan(const gw_structure *st, int g, const int *hist, int *rowstart,
-        int *cursor, int2 *zstat) {
+__device__ __forceinline__ void zscan_block(const gw_structure *st, int t, int g,
+                                            const int *hist, int *rowstart, int *cursor,
+                                            int2 *zstat) {
   __shared__ int warp_sum[32];
-  const int t = blockIdx.x;
   const int *h = hist + (size_t)t * (g + 1);
   int *rs = rowstart + (size_t)t * (g + 2);
   int *cur = cursor + (size_t)t * (g + 1);
@@ -92,8 +201,9 @@ k_zscan(const gw_structure *st, int g, const int *hist, int *rowstart,
   for (int k = 0; k < per; ++k) {
     const int b = b0 + k;
     if (b < nb) {
-      local += h[b];
-      if (b < g && h[b] > 0) zmax = b;
+      const int c = __ldcg(h + b);  // (counted by atomics)
+      local += c;
+      if (b < g && c > 0) zmax = b;
     }
   }
   // block exclusive scan of `local`
@@ -120,7 +230,7 @@ k_zscan(const gw_structure *st, int g, const int *hist, int *rowstart,
     if (b < nb) {
       rs[b] = run;
       cur[b] = run;
-      run += h[b];
+      run += __ldcg(h + b);
     }
   }
   if (threadIdx.x == blockDim.x - 1) rs[nb] = (int)(st[t].atom_begin + st[t].atom_count);
@@ -130,62 +240,138 @@ k_zscan(const gw_structure *st, int g, const int *hist, int *rowstart,
   __syncthreads();
   if (lane == 0) atomicMax(&zm, zmax);
   __syncthreads();
-  if (threadIdx.x == 0) zstat[t] = make_int2(zm, h[g] == 0);
+  if (threadIdx.x == 0) zstat[t] = make_int2(zm, __ldcg(h + g) == 0);
+}
+
+__global__ void __launch_bounds__(1024)
+k_zscan(const gw_structure *st, int g, const int *hist, int *rowstart,
+        int *cursor, int2 *zstat) {
+  zscan_block(st, blockIdx.x, g, hist, rowstart, cursor, zstat);
 }
 
 // Counting-sort scatter by z index.  Also records the permutation (sorted
-// position -> input index) and, for the bilinear deposit, the fractional z
-// position (z - zmin)/r - zi of each atom.
-__global__ void k_zscatter(const double *xyz, const float2 *f,
-                           const gw_structure *st, const int *zidx, int g,
-                           const unsigned long long *zmin_ord, double inv_r,
-                           int *cursor, double *xyz_s, float4 *xyf_s,
-                           int *perm, float *fz_s, int real) {
+// position -> input index), for the bilinear deposit the fractional z
+// position (z - zmin)/r - zi of each atom, and the sorted positions of the
+// candidates for the y extremes (any order).
+struct Scatter {
+  const double *xyz;
+  const float2 *f;
+  const int *zidx;
+  int g, real;
+  double inv_r;
+  int *cursor;
+  double *xyz_s;
+  float4 *xyf_s;
+  int *perm;
+  float *fz_s;
+  int *cand;
+};
+// one atom a warp lane (i < atom_count), all lanes call; h null: every atom
+// is a candidate
+__device__ __forceinline__ void scatter_atom(const Scatter &k, const gw_structure &s, int t,
+                                             double zmin, const HullEdges *h, int64_t i,
+                                             int *ncand) {
+  const bool live = i < s.atom_count;
+  const int64_t a = s.atom_begin + (live ? i : 0);
+  const double x = k.xyz[3 * a], y = k.xyz[3 * a + 1], z = k.xyz[3 * a + 2];
+  const int zi = k.zidx[a];
+  // one count of candidates per warp
+  const bool cand = live && !(h && hull_inside(*h, (float)x, (float)y));
+  const unsigned m = __ballot_sync(0xffffffffu, cand);
+  const int lane = threadIdx.x & 31;
+  int base = 0, pos = 0;
+  if (m && lane == __ffs(m) - 1) base = atomicAdd(ncand, __popc(m));
+  if (live)
+    pos = atomicAdd(k.cursor + (size_t)t * (k.g + 1) + (zi >= 0 && zi < k.g ? zi : k.g), 1);
+  if (m) base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+  if (!live) return;
+  if (cand) k.cand[s.atom_begin + base + __popc(m & ((1u << lane) - 1u))] = pos;
+  k.xyz_s[3 * (size_t)pos] = x;
+  k.xyz_s[3 * (size_t)pos + 1] = y;
+  k.xyz_s[3 * (size_t)pos + 2] = z;
+  float2 fa = k.f[a];
+  if (k.real) {
+    // in units of the structure's phase (rounded once from float64)
+    const double mag = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im);
+    fa = make_float2((float)(((double)fa.x * s.avg_f_re + (double)fa.y * s.avg_f_im) / mag), 0.f);
+  }
+  k.xyf_s[pos] = make_float4((float)x, (float)y, fa.x, fa.y);
+  k.perm[pos] = (int)a;
+  if (k.fz_s) {
+    const double v = GW_DMUL(GW_DSUB(z, zmin), k.inv_r);
+    k.fz_s[pos] = fminf(fmaxf((float)(v - (double)zi), 0.f), 1.f);
+  }
+}
+
+__global__ void k_zscatter(Scatter k, const gw_structure *st, const unsigned long long *zmin_ord,
+                           const unsigned long long *dirs, int *ncand) {
+  __shared__ HullEdges h;
   const gw_structure s = st[blockIdx.y];
-  int *cur = cursor + (size_t)blockIdx.y * (g + 1);
+  hull_edges(k.xyz, s, dirs + kDirs * blockIdx.y, h);
   const double zmin = ord_dbl(zmin_ord[blockIdx.y]);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-       i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
+       i - (threadIdx.x & 31) < s.atom_count; i += stride)
+    scatter_atom(k, s, blockIdx.y, zmin, &h, i, ncand + blockIdx.y);
+}
+
+// The whole structure preparation in one block per structure, every atom a
+// candidate, for structures of at most kPrepSmall atoms: there the five
+// launches cost more than their work (264 atoms: 7.8 us), and above it one
+// block's passes over the atoms do (with the line at 8192 atoms a whole pass
+// over 2,387 atoms at 159 angles took 139 us, with the many-block kernels 120).
+constexpr int kPrepSmall = 2048;
+__global__ void __launch_bounds__(1024)
+k_prep_small(Scatter k, const gw_structure *st, double r, int *zidx, int *hist, int *rowstart,
+             int2 *zstat, unsigned long long *zmin_ord, int *ncand, int *any_ext) {
+  __shared__ unsigned long long s_z[32];
+  __shared__ int s_n;
+  const int t = blockIdx.x;
+  const gw_structure s = st[t];
+  int *hs = hist + (size_t)t * (k.g + 1);
+  for (int b = threadIdx.x; b <= k.g; b += blockDim.x) __stcg(hs + b, 0);
+  unsigned long long z = ~0ULL;
+  for (int64_t i = threadIdx.x; i < s.atom_count; i += blockDim.x)
+    z = min(z, dbl_ord(k.xyz[3 * (s.atom_begin + i) + 2]));
+  for (int o = 16; o > 0; o >>= 1) z = min(z, __shfl_xor_sync(0xffffffffu, z, o));
+  if ((threadIdx.x & 31) == 0) s_z[threadIdx.x >> 5] = z;
+  if (threadIdx.x == 0) {
+    s_n = 0;
+    if (t == 0) *any_ext = 0;
+  }
+  __syncthreads();
+  z = s_z[threadIdx.x & 31];
+  for (int o = 16; o > 0; o >>= 1) z = min(z, __shfl_xor_sync(0xffffffffu, z, o));
+  const double zmin = ord_dbl(z);
+  for (int64_t i = threadIdx.x; i < s.atom_count; i += blockDim.x) {
     const int64_t a = s.atom_begin + i;
-    const int zi = zidx[a];
-    const int pos = atomicAdd(cur + (zi >= 0 && zi < g ? zi : g), 1);
-    xyz_s[3 * (size_t)pos] = xyz[3 * a];
-    xyz_s[3 * (size_t)pos + 1] = xyz[3 * a + 1];
-    xyz_s[3 * (size_t)pos + 2] = xyz[3 * a + 2];
-    float2 fa = f[a];
-    if (real) {
-      // in units of the structure's phase (rounded once from float64)
-      const double mag = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im);
-      fa = make_float2((float)(((double)fa.x * s.avg_f_re + (double)fa.y * s.avg_f_im) / mag), 0.f);
-    }
-    xyf_s[pos] = make_float4((float)xyz[3 * a], (float)xyz[3 * a + 1], fa.x, fa.y);
-    perm[pos] = (int)a;
-    if (fz_s) {
-      const double v = GW_DMUL(GW_DSUB(xyz[3 * a + 2], zmin), inv_r);
-      fz_s[pos] = fminf(fmaxf((float)(v - (double)zi), 0.f), 1.f);
-    }
+    const int zi = (int)floor_div_exact(GW_DSUB(k.xyz[3 * a + 2], zmin), r, k.inv_r);
+    zidx[a] = zi;
+    atomicAdd(hs + (zi >= 0 && zi < k.g ? zi : k.g), 1);
+  }
+  __threadfence_block();
+  __syncthreads();
+  zscan_block(st, t, k.g, hist, rowstart, k.cursor, zstat);
+  __threadfence_block();
+  __syncthreads();
+  for (int64_t i = threadIdx.x; i - (threadIdx.x & 31) < s.atom_count; i += blockDim.x)
+    scatter_atom(k, s, t, zmin, nullptr, i, &s_n);
+  if (threadIdx.x == 0) {
+    ncand[t] = (int)s.atom_count;
+    zmin_ord[t] = z;
   }
 }
 
 // ------------------------------------------------------------ per slice
-// Per slice: min and max of the rotated y over all atoms (the shift to the
-// minimum, voxelgrids.py:323), and the slice's background constants.
 // Per-slice extremes of the rotated y' = x sin(phi) + y cos(phi) over all
 // atoms of the structure (voxelgrids.py:325-330: np.min / np.max of
-// rot[:, 1]), exact in float64, in two passes over the z-sorted atoms.
-// Pass 1 (k_ybound) evaluates y' in float32 with a rigorous error bound d
-// (10 u (|x s| + |y c|), u = 2^-24: input, product and fma roundings total
+// rot[:, 1]), exact in float64, over the structure's candidates (block_extremes)
+// in two passes.  Pass 1 evaluates y' in float32 with a rigorous error bound
+// d (10 u (|x s| + |y c|), u = 2^-24: input, product and fma roundings total
 // about 4.1 u of that sum) and keeps lo = min(y' + d) and hi = max(y' - d),
-// rounded outward.  Pass 2 (k_yminmax) evaluates the float64 chain only for
-// the atoms whose interval reaches below lo or above hi: every other atom's
-// exact value is above lo >= the exact minimum (below hi <= the maximum).
-__device__ __forceinline__ unsigned flt_ord(float f) {
-  const unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_flt(unsigned o) {
-  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
+// rounded outward.  Pass 2 evaluates the float64 chain only for the atoms
+// whose interval reaches below lo or above hi: every other atom's exact value
+// is above lo >= the exact minimum (below hi <= the maximum).
 __device__ __forceinline__ void y_interval(const float4 q, float cs, float sn,
                                            float &lo, float &hi) {
   const float xs = q.x * sn, yc = q.y * cs;
@@ -195,21 +381,10 @@ __device__ __forceinline__ void y_interval(const float4 q, float cs, float sn,
   hi = __fadd_ru(t, d);
 }
 
-// lo bounds to the largest ordered value, hi bounds to the smallest
-__global__ void k_yreset(unsigned *ybnd, int s0, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    ybnd[2 * (size_t)(s0 + i)] = ~0u;
-    ybnd[2 * (size_t)(s0 + i) + 1] = 0u;
-  }
-}
-
-// Both passes give a block kYS consecutive slices of the batch: a thread
-// loads an atom once and evaluates it for each of them (the atoms stay in
-// L2; one load per atom and slice made the passes L2-bound).  Slices of
-// different structures in one block are taken as runs of the same
-// structure, each over its own atoms.
-constexpr int kYS = 4;
+// A block takes S consecutive slices of the batch: a thread loads an atom
+// once and evaluates it for each of them.  Slices of different structures in
+// one block are taken as runs of the same structure, each over its own
+// candidates.
 
 // Run [kb, ke) of the block's slices k0 + k that share one structure.
 __device__ __forceinline__ int y_run_end(const SliceArgs &a, int first, int kb,
@@ -220,13 +395,13 @@ __device__ __forceinline__ int y_run_end(const SliceArgs &a, int first, int kb,
   return ke;
 }
 
-// Block reduction of kYS (min, max) pairs; thread 0 gets the results.
-template <typename T>
-__device__ __forceinline__ void y_block_reduce(T (&lo)[kYS], T (&hi)[kYS]) {
-  __shared__ T s_lo[kYS][32], s_hi[kYS][32];
+// Block reduction of S (min, max) pairs; thread 0 gets the results.
+template <int S, typename T>
+__device__ __forceinline__ void y_block_reduce(T (&lo)[S], T (&hi)[S]) {
+  __shared__ T s_lo[S][32], s_hi[S][32];
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-  for (int k = 0; k < kYS; ++k) {
+  for (int k = 0; k < S; ++k) {
     for (int o = 16; o > 0; o >>= 1) {
       lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
       hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
@@ -236,7 +411,7 @@ __device__ __forceinline__ void y_block_reduce(T (&lo)[kYS], T (&hi)[kYS]) {
   __syncthreads();
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int k = 0; k < kYS; ++k)
+    for (int k = 0; k < S; ++k)
       for (int j = 1; j < nw; ++j) {
         lo[k] = min(lo[k], s_lo[k][j]);
         hi[k] = max(hi[k], s_hi[k][j]);
@@ -244,98 +419,78 @@ __device__ __forceinline__ void y_block_reduce(T (&lo)[kYS], T (&hi)[kYS]) {
   }
 }
 
-__global__ void k_ybound(SliceArgs a, int slice0, int n) {
-  const int first = slice0 + blockIdx.y * kYS;
-  const int ns = min(kYS, slice0 + n - first);
-  float cs[kYS], sn[kYS];
-  unsigned lo[kYS], hi[kYS];  // ordered: min of (y'+d), max of (y'-d)
+// The extremes of the block's slices, then, per slice, its background
+// constants and the extents of the valid atoms (voxelgrids.py:346-349): y
+// indices grow with y (the floor division is monotone), so when every atom is
+// valid the extents are (0, index of max y, 0, largest occupied z row);
+// otherwise k_ext_exact computes them atom by atom.  Bound by the candidates'
+// gathers from L2.  Over all atoms, with a reset and the extents in launches
+// of their own, 16 boxes of 57,000 atoms at 180 angles each took 389 us, one of
+// 13,713 at 180 angles 27 us and one of 264,424 at 720 angles 332 us; this and
+// k_ext_exact take 31, 7 and 14 us (the candidate test costs k_zscatter 2-6 us
+// a box of these).
+template <int S>
+__global__ void __launch_bounds__(256) k_yext(SliceArgs a, int slice0, int n) {
+  __shared__ float s_lo[S], s_hi[S];
+  const int first = slice0 + blockIdx.x * S;
+  const int ns = min(S, slice0 + n - first);
+  double c[S], sn[S];
+  unsigned flo[S], fhi[S];  // ordered: min of (y'+d), max of (y'-d)
 #pragma unroll
-  for (int k = 0; k < kYS; ++k) {
+  for (int k = 0; k < S; ++k) {
     const int p = (first + min(k, ns - 1)) % a.n_phi;
-    cs[k] = (float)a.ph[p].cos_phi;
-    sn[k] = (float)a.ph[p].sin_phi;
-    lo[k] = ~0u;
-    hi[k] = 0u;
+    c[k] = a.ph[p].cos_phi;
+    sn[k] = a.ph[p].sin_phi;
+    flo[k] = ~0u;
+    fhi[k] = 0u;
   }
   for (int kb = 0; kb < ns;) {
     const int ke = y_run_end(a, first, kb, ns);
-    const gw_structure s = a.st[(first + kb) / a.n_phi];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-         i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
-      const float4 q = a.xyf_s[s.atom_begin + i];
+    const int t = (first + kb) / a.n_phi;
+    const int *cand = a.cand + a.st[t].atom_begin;
+    const int nc = a.ncand[t];
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+      const float4 q = a.xyf_s[cand[i]];
 #pragma unroll
-      for (int k = 0; k < kYS; ++k) {
+      for (int k = 0; k < S; ++k) {
         if (k < kb || k >= ke) continue;
         float l, h;
-        y_interval(q, cs[k], sn[k], l, h);
-        lo[k] = min(lo[k], flt_ord(h));
-        hi[k] = max(hi[k], flt_ord(l));
+        y_interval(q, (float)c[k], (float)sn[k], l, h);
+        flo[k] = min(flo[k], flt_ord(h));
+        fhi[k] = max(fhi[k], flt_ord(l));
       }
     }
     kb = ke;
   }
-  // block reduction, then one atomic per block, slice and bound
-  y_block_reduce(lo, hi);
-  if (threadIdx.x == 0) {
+  y_block_reduce<S>(flo, fhi);
+  if (threadIdx.x == 0)
 #pragma unroll
-    for (int k = 0; k < kYS; ++k) {
-      if (k >= ns || lo[k] == ~0u) continue;
-      atomicMin(a.ybnd + 2 * (size_t)(first + k), lo[k]);
-      atomicMax(a.ybnd + 2 * (size_t)(first + k) + 1, hi[k]);
+    for (int k = 0; k < S; ++k) {
+      s_lo[k] = ord_flt(flo[k]);
+      s_hi[k] = ord_flt(fhi[k]);
     }
-  }
-}
-
-__global__ void k_yminmax(SliceArgs a, int slice0, int n) {
-  const int first = slice0 + blockIdx.y * kYS;
-  const int ns = min(kYS, slice0 + n - first);
-  if (blockIdx.x == 0 && threadIdx.x < ns) {
-    // background constant C = avg_voxel_f * max_voxels (voxelgrids.py:358,365):
-    // Cbg is what the transformed window excludes (batched mode), Cd what
-    // stays inside it
-    const int sl = first + threadIdx.x;
-    const gw_structure s = a.st[sl / a.n_phi];
-    double cr = GW_DMUL(s.avg_f_re, s.max_voxels), ci = GW_DMUL(s.avg_f_im, s.max_voxels);
-    if (a.real) {  // real grids are in units of the structure's phase
-      cr = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im) * s.max_voxels;
-      ci = 0.0;
-    }
-    const float2 c = make_float2((float)cr, (float)ci);
-    const bool bg = !a.plain && (a.fill || a.smooth_on);
-    // the q = 0 pixel is by far the largest: rounded once
-    const double g2 = bg ? (double)a.g * (double)a.g : 0.0;
-    a.sdc[sl] = make_float2((float)(cr * g2), (float)(ci * g2));
-    a.sconst[sl] = bg ? make_float4(c.x, c.y, 0.f, 0.f)
-                      : make_float4(0.f, 0.f, c.x, c.y);
-  }
-  double c[kYS], sn[kYS];
-  float blo[kYS], bhi[kYS];
-  unsigned long long lo[kYS], hi[kYS];
+  __syncthreads();
+  unsigned long long lo[S], hi[S];
 #pragma unroll
-  for (int k = 0; k < kYS; ++k) {
-    const int sl = first + min(k, ns - 1);
-    const int p = sl % a.n_phi;
-    c[k] = a.ph[p].cos_phi;
-    sn[k] = a.ph[p].sin_phi;
-    blo[k] = ord_flt(a.ybnd[2 * (size_t)sl]);
-    bhi[k] = ord_flt(a.ybnd[2 * (size_t)sl + 1]);
+  for (int k = 0; k < S; ++k) {
     lo[k] = ~0ULL;
     hi[k] = 0ULL;
   }
   for (int kb = 0; kb < ns;) {
     const int ke = y_run_end(a, first, kb, ns);
-    const gw_structure s = a.st[(first + kb) / a.n_phi];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-         i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
-      const float4 q = a.xyf_s[s.atom_begin + i];
+    const int t = (first + kb) / a.n_phi;
+    const int *cand = a.cand + a.st[t].atom_begin;
+    const int nc = a.ncand[t];
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+      const int pos = cand[i];
+      const float4 q = a.xyf_s[pos];
 #pragma unroll
-      for (int k = 0; k < kYS; ++k) {
+      for (int k = 0; k < S; ++k) {
         if (k < kb || k >= ke) continue;
         float l, h;
         y_interval(q, (float)c[k], (float)sn[k], l, h);
-        if (l <= blo[k] || h >= bhi[k]) {
-          const unsigned long long v =
-              dbl_ord(rot_y(a.xyz_s + 3 * (s.atom_begin + i), c[k], sn[k]));
+        if (l <= s_lo[k] || h >= s_hi[k]) {
+          const unsigned long long v = dbl_ord(rot_y(a.xyz_s + 3 * (size_t)pos, c[k], sn[k]));
           lo[k] = min(lo[k], v);
           hi[k] = max(hi[k], v);
         }
@@ -343,41 +498,44 @@ __global__ void k_yminmax(SliceArgs a, int slice0, int n) {
     }
     kb = ke;
   }
-  y_block_reduce(lo, hi);
-  if (threadIdx.x == 0) {
+  y_block_reduce<S>(lo, hi);
+  if (threadIdx.x != 0) return;
 #pragma unroll
-    for (int k = 0; k < kYS; ++k) {
-      if (k >= ns || lo[k] == ~0ULL) continue;
-      atomicMin(a.ymin_ord + first + k, lo[k]);
-      atomicMax(a.ymax_ord + first + k, hi[k]);
+  for (int k = 0; k < S; ++k) {
+    if (k >= ns) continue;
+    const int sl = first + k, t = sl / a.n_phi;
+    a.ymin_ord[sl] = lo[k];
+    // background constant C = avg_voxel_f * max_voxels (voxelgrids.py:358,365):
+    // Cbg is what the transformed window excludes (batched mode), Cd what
+    // stays inside it
+    const gw_structure s = a.st[t];
+    double cr = GW_DMUL(s.avg_f_re, s.max_voxels), ci = GW_DMUL(s.avg_f_im, s.max_voxels);
+    if (a.real) {  // real grids are in units of the structure's phase
+      cr = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im) * s.max_voxels;
+      ci = 0.0;
+    }
+    const float2 cf = make_float2((float)cr, (float)ci);
+    const bool bg = !a.plain && (a.fill || a.smooth_on);
+    // the q = 0 pixel is by far the largest
+    const double g2 = (double)a.g * (double)a.g;
+    const double dr = bg ? cr * g2 : 0.0, di = bg ? ci * g2 : 0.0;
+    a.sdc[sl] = make_float4((float)dr, (float)di, (float)(dr - (float)dr), (float)(di - (float)di));
+    a.sconst[sl] = bg ? make_float4(cf.x, cf.y, 0.f, 0.f) : make_float4(0.f, 0.f, cf.x, cf.y);
+    const double Y = floor_div_exact(GW_DSUB(ord_dbl(hi[k]), ord_dbl(lo[k])), a.r, a.inv_r);
+    const int2 zs = a.zstat[t];
+    if (Y < (double)a.g && zs.y) {
+      a.ext[sl] = make_int4(0, (int)Y, 0, zs.x);
+      a.extflag[sl] = 0;
+    } else {
+      a.ext[sl] = make_int4(INT_MAX, -1, INT_MAX, -1);
+      a.extflag[sl] = 1;
+      *a.any_ext = 1;
     }
   }
 }
 
-// Per slice extents of the valid atoms (voxelgrids.py:346-349).  y indices
-// grow with y (the floor division is monotone), so when every atom is valid
-// the extents are (0, index of max y, 0, largest occupied z row); otherwise
-// k_ext_exact computes them atom by atom.
-__global__ void k_ext(SliceArgs a, int slice0, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int sl = slice0 + i;
-  const int t = sl / a.n_phi;
-  const double ymin = ord_dbl(a.ymin_ord[sl]), ymax = ord_dbl(a.ymax_ord[sl]);
-  const double Y = floor_div_exact(GW_DSUB(ymax, ymin), a.r, a.inv_r);
-  const int2 zs = a.zstat[t];
-  if (Y < (double)a.g && zs.y) {
-    a.ext[sl] = make_int4(0, (int)Y, 0, zs.x);
-    a.extflag[sl] = 0;
-  } else {
-    a.ext[sl] = make_int4(INT_MAX, -1, INT_MAX, -1);
-    a.extflag[sl] = 1;
-  }
-}
-
-__global__ void k_ext_exact(SliceArgs a, int slice0) {
-  const int sl = slice0 + blockIdx.y;
-  if (!a.extflag[sl]) return;
+// The extents of slice sl's valid atoms, this block's share of the atoms.
+__device__ __forceinline__ void ext_exact(const SliceArgs &a, int sl) {
   const int t = sl / a.n_phi, p = sl % a.n_phi;
   const gw_structure s = a.st[t];
   const double c = a.ph[p].cos_phi, sn = a.ph[p].sin_phi;
@@ -403,6 +561,14 @@ __global__ void k_ext_exact(SliceArgs a, int slice0) {
     atomicMin(&e->x, ymn); atomicMax(&e->y, ymx);
     atomicMin(&e->z, zmn); atomicMax(&e->w, zmx);
   }
+}
+
+// Rarely needed (a slice with atoms outside the grid): a small grid over the
+// slices that exits at once otherwise.
+__global__ void k_ext_exact(SliceArgs a, int slice0, int n) {
+  if (!*a.any_ext) return;
+  for (int sl = slice0 + blockIdx.y; sl < slice0 + n; sl += gridDim.y)
+    if (a.extflag[sl]) ext_exact(a, sl);
 }
 
 // Per-slice profiles: fill_bkg column term (minus the background) and the
@@ -1000,12 +1166,6 @@ __global__ void k_debug_window(SliceArgs a, int sl, float2 *win) {
   }
 }
 
-// per-slice extents start empty: min fields INT_MAX, max fields -1
-__global__ void k_ext_init(int4 *ext, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) ext[i] = make_int4(INT_MAX, -1, INT_MAX, -1);
-}
-
 __global__ void k_debug_deposit(SliceArgs a, int sl, int *yo, int *zo) {
   const int t = sl / a.n_phi, p = sl % a.n_phi;
   const gw_structure s = a.st[t];
@@ -1152,9 +1312,9 @@ SliceArgs slice_args(gw_voxel_plan *P) {
   a.xyz = P->d_xyz; a.f = P->d_f; a.zidx = P->d_zidx; a.st = P->d_structs;
   a.xyz_s = P->d_xyz_s; a.xyf_s = P->d_xyf_s; a.rowstart = P->d_rowstart;
   a.fz_s = P->d_fz_s; a.bil = P->bil; a.real = P->real;
-  a.ybnd = P->d_ybnd;
+  a.cand = P->d_cand; a.ncand = P->d_ncand; a.any_ext = P->d_any_ext;
   a.roff = P->d_roff;
-  a.zstat = P->d_zstat; a.ymax_ord = P->d_ymax; a.extflag = P->d_extflag;
+  a.zstat = P->d_zstat; a.extflag = P->d_extflag;
   a.ph = P->d_phis; a.clbase = P->d_clbase; a.ymin_ord = P->d_ymin;
   a.ext = P->d_ext; a.amo = P->d_amo; a.my = P->d_my; a.pr = P->d_pr;
   a.mz = P->d_mz; a.gw = P->d_gw; a.sconst = P->d_sconst; a.sdc = P->d_sdc; a.err = P->ctx->d_err;
@@ -1171,16 +1331,31 @@ int atom_blocks(gw_voxel_plan *P) {
 int enqueue_prep(gw_voxel_plan *P) {
   gw_ctx *ctx = P->ctx;
   cudaStream_t st = ctx->stream;
-  k_ext_init<<<(P->n_slices + 255) / 256, 256, 0, st>>>(P->d_ext, P->n_slices);
-  GW_LAUNCHED(ctx);
-  GW_CUDA(cudaMemsetAsync(P->d_zmin, 0xff, P->n_struct * sizeof(unsigned long long), st));
-  GW_CUDA(cudaMemsetAsync(P->d_ymin, 0xff, P->n_slices * sizeof(unsigned long long), st));
-  GW_CUDA(cudaMemsetAsync(P->d_ymax, 0, P->n_slices * sizeof(unsigned long long), st));
-  GW_CUDA(cudaMemsetAsync(P->d_zhist, 0, (size_t)P->n_struct * (P->g + 1) * sizeof(int), st));
+  const Scatter sc{P->d_xyz, P->d_f, P->d_zidx, P->g, P->real ? 1 : 0, P->inv_r, P->d_cursor,
+                   P->d_xyz_s, P->d_xyf_s, P->d_perm, P->d_fz_s, P->d_cand};
+  int64_t max_atoms = 0;
+  for (auto &s : P->structs) max_atoms = std::max(max_atoms, s.atom_count);
+  if (max_atoms <= kPrepSmall) {
+    gw::KTimer tm(ctx, GW_K_PREP);
+    k_prep_small<<<P->n_struct, 1024, 0, st>>>(sc, P->d_structs, P->r, P->d_zidx, P->d_zhist,
+                                               P->d_rowstart, P->d_zstat, P->d_zmin,
+                                               P->d_ncand, P->d_any_ext);
+    GW_LAUNCHED(ctx);
+    return GW_OK;
+  }
   const int nblk_at = atom_blocks(P);
+  const int64_t n_hist = (int64_t)P->n_struct * (P->g + 1);
   {
     gw::KTimer tm(ctx, GW_K_PREP);
-    k_zmin<<<dim3(nblk_at, P->n_struct), 256, 0, st>>>(P->d_xyz, P->d_structs, P->d_zmin);
+    k_prep_init<<<(int)std::min<int64_t>((n_hist + 255) / 256, 2 * ctx->sm_count), 256, 0, st>>>(
+        P->n_struct, n_hist, P->d_zhist, P->d_zmin, P->d_dirs, P->d_ncand, P->d_any_ext);
+    GW_LAUNCHED(ctx);
+  }
+  {
+    gw::KTimer tm(ctx, GW_K_PREP);
+    // (one atomic per block and direction)
+    const int nb = std::min(nblk_at, std::max(1, 2 * ctx->sm_count / P->n_struct));
+    k_extremes<<<dim3(nb, P->n_struct), 256, 0, st>>>(P->d_xyz, P->d_structs, P->d_zmin, P->d_dirs);
     GW_LAUNCHED(ctx);
   }
   {
@@ -1198,9 +1373,10 @@ int enqueue_prep(gw_voxel_plan *P) {
   }
   {
     gw::KTimer tm(ctx, GW_K_PREP);
-    k_zscatter<<<dim3(nblk_at, P->n_struct), 256, 0, st>>>(
-        P->d_xyz, P->d_f, P->d_structs, P->d_zidx, P->g, P->d_zmin, P->inv_r,
-        P->d_cursor, P->d_xyz_s, P->d_xyf_s, P->d_perm, P->d_fz_s, P->real ? 1 : 0);
+    // (each block sets the polygon's edges up: no more blocks than fill the GPU)
+    const int nb = std::min(nblk_at, std::max(1, 8 * ctx->sm_count / P->n_struct));
+    k_zscatter<<<dim3(nb, P->n_struct), 256, 0, st>>>(sc, P->d_structs, P->d_zmin, P->d_dirs,
+                                                           P->d_ncand);
     GW_LAUNCHED(ctx);
   }
   return GW_OK;
@@ -1220,31 +1396,17 @@ SliceArgs profile_view(const SliceArgs &a, int s0) {
 int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n) {
   gw_ctx *ctx = P->ctx;
   cudaStream_t st = ctx->stream;
-  const int nblk_at = atom_blocks(P);
   {
     gw::KTimer tm(ctx, GW_K_DEPOSIT);
-    // bounds of slice s live at ybnd[2s], ybnd[2s+1]: reset this range
-    k_yreset<<<(n + 255) / 256, 256, 0, st>>>(P->d_ybnd, s0, n);
-    GW_LAUNCHED(ctx);
-    // a few blocks per slice (grid-stride over the atoms), one atomic per
-    // block: the slice's two words are the only targets
-    const int nblk_y = std::min(nblk_at, 16);
-    const int ngrp = (n + kYS - 1) / kYS;
-    k_ybound<<<dim3(nblk_y, ngrp), 256, 0, st>>>(a, s0, n);
-    GW_LAUNCHED(ctx);
-    k_yminmax<<<dim3(nblk_y, ngrp), 256, 0, st>>>(a, s0, n);
+    // four slices a block reuse each candidate, once there are blocks enough
+    // (180 slices: 12.3 us at four a block, 5.3 at one; 2880: 29.7 at four)
+    if (n > 4 * ctx->sm_count) k_yext<4><<<(n + 3) / 4, 256, 0, st>>>(a, s0, n);
+    else k_yext<1><<<n, 256, 0, st>>>(a, s0, n);
     GW_LAUNCHED(ctx);
   }
   {
     gw::KTimer tm(ctx, GW_K_DEPOSIT);
-    k_ext<<<(n + 127) / 128, 128, 0, st>>>(a, s0, n);
-    GW_LAUNCHED(ctx);
-  }
-  {
-    gw::KTimer tm(ctx, GW_K_DEPOSIT);
-    // rarely needed (a slice with atoms outside the grid): a small grid
-    // that exits at once otherwise
-    k_ext_exact<<<dim3(std::min(nblk_at, 16), n), 256, 0, st>>>(a, s0);
+    k_ext_exact<<<dim3(std::min(atom_blocks(P), 16), std::min(n, 64)), 256, 0, st>>>(a, s0, n);
     GW_LAUNCHED(ctx);
   }
   if (a.fill || a.smooth_on) {
@@ -1892,8 +2054,8 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
                  : alloc(&P->d_sum, P->sum_stride * P->n_out, &B))) ||
       (st = alloc(&P->d_iq64, P->iq_stride * P->n_out, &B)) ||
       (st = alloc(&P->d_iq32, P->iq_stride * P->n_out, &B)) ||
-      (st = alloc(&P->d_ymax, P->n_slices, &B)) ||
-      (st = alloc(&P->d_ybnd, 2 * (size_t)P->n_slices, &B)) ||
+      (st = alloc(&P->d_dirs, (size_t)n_struct * kDirs, &B)) ||
+      (st = alloc(&P->d_ncand, n_struct, &B)) || (st = alloc(&P->d_any_ext, 1, &B)) ||
       (st = alloc(&P->d_extflag, P->n_slices, &B)) ||
       (st = alloc(&P->d_zhist, (size_t)n_struct * (g + 1), &B)) ||
       (st = alloc(&P->d_rowstart, (size_t)n_struct * (g + 2), &B)) ||
@@ -1947,8 +2109,8 @@ extern "C" int gw_voxel_plan_destroy(gw_voxel_plan *P) {
                   P->d_C2, P->d_sum, P->d_sumk, P->d_f0, P->d_iq64,
                   P->d_iq32, P->d_F1, P->d_amo, P->d_my, P->d_mz,
                   P->d_sconst, P->d_sdc, P->d_xyz_s, P->d_xyf_s, P->d_fz_s,
-                  P->d_perm, P->d_ybnd, P->d_roff, P->d_zhist, P->d_rowstart,
-                  P->d_cursor, P->d_zstat, P->d_ymax, P->d_extflag,
+                  P->d_perm, P->d_cand, P->d_dirs, P->d_ncand, P->d_any_ext, P->d_roff, P->d_zhist, P->d_rowstart,
+                  P->d_cursor, P->d_zstat, P->d_extflag,
                   P->d_shell, P->d_f_shells, P->d_structs_shells, P->d_zf0,
                   P->d_fty, P->d_ftz, P->d_G, P->d_lptr, P->d_lent, P->d_zptr,
                   P->d_zrows, P->d_heavy, P->d_zmulti, P->d_pr};
@@ -1966,11 +2128,11 @@ extern "C" int gw_voxel_set_atoms(gw_voxel_plan *P, const double *xyz,
       return gw::fail(GW_ERR_ARG, "gw_voxel_set_atoms: structure atom range outside the atom arrays");
   if (n != P->n_atoms) {
     void *old[] = {P->d_xyz, P->d_f, P->d_zidx, P->d_xyz_s, P->d_xyf_s,
-                   P->d_perm, P->d_fz_s};
+                   P->d_perm, P->d_fz_s, P->d_cand};
     for (void *q : old) gw::dev_free(q);
     P->d_xyz = nullptr; P->d_f = nullptr; P->d_zidx = nullptr;
     P->d_xyz_s = nullptr; P->d_xyf_s = nullptr;
-    P->d_perm = nullptr; P->d_fz_s = nullptr;
+    P->d_perm = nullptr; P->d_fz_s = nullptr; P->d_cand = nullptr;
     P->n_atoms = -1;
     if (n > INT_MAX / 4)
       return gw::fail(GW_ERR_ARG, "gw_voxel_set_atoms: more than 2^29 atoms");
@@ -1980,6 +2142,7 @@ extern "C" int gw_voxel_set_atoms(gw_voxel_plan *P, const double *xyz,
     GW_CUDA(gw::dev_malloc((void **)&P->d_xyz_s, (size_t)n * 3 * sizeof(double)));
     GW_CUDA(gw::dev_malloc((void **)&P->d_xyf_s, (size_t)n * sizeof(float4)));
     GW_CUDA(gw::dev_malloc((void **)&P->d_perm, (size_t)n * sizeof(int)));
+    GW_CUDA(gw::dev_malloc((void **)&P->d_cand, (size_t)n * sizeof(int)));
     if (P->bil)
       GW_CUDA(gw::dev_malloc((void **)&P->d_fz_s, (size_t)n * sizeof(float)));
     P->n_atoms = n;

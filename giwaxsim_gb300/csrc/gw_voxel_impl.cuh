@@ -40,7 +40,9 @@ struct SliceArgs {
   const float4 *xyf_s; // sorted atoms: float32 (x, y) and f (re, im); real
                        // grids: (Re(f conj(u)), 0), u the structure's phase
   const float *fz_s;   // bilinear: fractional z position of the sorted atoms
-  unsigned *ybnd;      // per slice: float32 bounds on the y extremes (ordered)
+  // per structure: sorted positions of the atoms that may be at a slice's y
+  // extremes (from atom_begin on), and their number
+  const int *cand, *ncand;
   const int *roff;     // per slice: first window row (n_slices+1 entries),
                        // when structures have their own z windows; else null
   const int *rowstart; // per structure: g+2 offsets into the sorted arrays
@@ -48,8 +50,9 @@ struct SliceArgs {
   const gw_structure *st;
   const gw_phi *ph;
   const double *clbase;  // per slice
-  unsigned long long *ymin_ord, *ymax_ord;
+  unsigned long long *ymin_ord;
   int *extflag;          // per slice: 1 = extents need the exact pass
+  int *any_ext;          // some slice of the pass needs it
   int4 *ext;  // y_min, y_max, z_min, z_max (valid atoms)
   float2 *amo;
   float *my, *mz;
@@ -59,7 +62,9 @@ struct SliceArgs {
   float2 *pr;
   const float *gw;  // gaussian weights, 2*radius+1
   float4 *sconst;   // per slice: (Cbg.re, Cbg.im, Cd.re, Cd.im)
-  float2 *sdc;      // per slice: Cbg g^2, the background's DFT (at q = 0)
+  // per slice: Cbg g^2, the background's DFT (at q = 0), and what its rounding
+  // to float32 leaves (re, im, re, im)
+  float4 *sdc;
   int *err;
 };
 
@@ -648,16 +653,17 @@ struct gw_voxel_plan {
   float4 *d_xyf_s = nullptr;
   float *d_fz_s = nullptr;
   int *d_perm = nullptr;   // sorted position -> input atom index
-  unsigned *d_ybnd = nullptr;  // 2 per slice (see k_ybound)
+  int *d_cand = nullptr;       // candidates for the y extremes (sorted positions)
+  int *d_ncand = nullptr, *d_any_ext = nullptr;
+  unsigned long long *d_dirs = nullptr;  // per structure: outermost atoms
   std::vector<int> roff_host;  // per-slice first window row (n_slices+1)
   int *d_roff = nullptr;       // null when every slice has Lz rows
   int *d_zhist = nullptr, *d_rowstart = nullptr, *d_cursor = nullptr;
   int2 *d_zstat = nullptr;
-  unsigned long long *d_ymax = nullptr;
   int *d_extflag = nullptr;
   float *d_my = nullptr, *d_mz = nullptr;
   float4 *d_sconst = nullptr;
-  float2 *d_sdc = nullptr;
+  float4 *d_sdc = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int64_t graph_kernels = 0;
