@@ -681,6 +681,90 @@ __global__ void k_col_tables(const gw_phi *ph, int g, int k0, int nc,
   }
 }
 
+// The gather's line table from the counts per window line: lptr, its entries
+// and the heavy lines, so that a plan's creation neither reads the column
+// tables back nor sorts them on the host (403^3 at 360 angles: @HOST@ against
+// @DEV@ us).  Two launches of a block scan each (line_sums: a block's totals;
+// line_ptrs: the totals before it, then its own lines), kLineBlock lines a
+// block.  line_ptrs leaves line l's start in lptr[l + 1]; line_scatter counts
+// it up to the line's end while it takes the keys phi Nc + m in any order, and
+// line_entries puts each entry at its key's rank in the line: table order.
+constexpr int kLineBlock = 1024;
+
+// inclusive scan of v over the block's kLineBlock threads (all call)
+__device__ __forceinline__ int2 line_scan(int2 v) {
+  __shared__ int2 ws[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) { v.x += x; v.y += y; }
+  }
+  if (lane == 31) ws[w] = v;
+  __syncthreads();
+  int2 b = make_int2(0, 0);
+  for (int j = 0; j < w; ++j) { b.x += ws[j].x; b.y += ws[j].y; }
+  __syncthreads();
+  return make_int2(v.x + b.x, v.y + b.y);
+}
+__device__ __forceinline__ int2 line_count(const unsigned *C2, int l, int n, int per_entry,
+                                           int heavy) {
+  const int c = l < n ? (int)C2[l] : 0;
+  return make_int2(c, (int64_t)c * per_entry > heavy);
+}
+__global__ void __launch_bounds__(kLineBlock)
+k_line_sums(const unsigned *C2, int n, int per_entry, int heavy, int2 *part) {
+  const int2 v = line_scan(
+      line_count(C2, blockIdx.x * kLineBlock + threadIdx.x, n, per_entry, heavy));
+  if (threadIdx.x == kLineBlock - 1) part[blockIdx.x] = v;
+}
+// total[0]: (entries, heavy lines)
+__global__ void __launch_bounds__(kLineBlock)
+k_line_ptrs(const unsigned *C2, int n, int per_entry, int heavy_above, const int2 *part,
+            int *lptr, int *heavy, int2 *total) {
+  __shared__ int2 s_base;
+  int2 b = make_int2(0, 0);
+  for (int j = threadIdx.x; j < (int)blockIdx.x; j += kLineBlock) {
+    b.x += part[j].x;
+    b.y += part[j].y;
+  }
+  b = line_scan(b);
+  if (threadIdx.x == kLineBlock - 1) s_base = b;
+  __syncthreads();
+  b = s_base;
+  const int l = blockIdx.x * kLineBlock + threadIdx.x;
+  const int2 c = line_count(C2, l, n, per_entry, heavy_above);
+  const int2 v = line_scan(c);
+  if (l < n) {
+    lptr[l + 1] = b.x + v.x - c.x;
+    if (c.y) heavy[b.y + v.y - 1] = l;
+  }
+  if (l == 0) lptr[0] = 0;
+  if (l == n - 1) *total = make_int2(b.x + v.x, b.y + v.y);
+}
+__global__ void k_line_scatter(const int *colofs, int nc, int W, int *lptr, unsigned *keys) {
+  for (int m = threadIdx.x; m < nc; m += blockDim.x) {
+    const int co = colofs[(size_t)blockIdx.x * nc + m];
+    if (co >= 0) keys[atomicAdd(lptr + co / W + 1, 1)] = blockIdx.x * (unsigned)nc + m;
+  }
+}
+// real: table column m of F1 column j = m - m_zero, or its mirror's below
+// m_zero (rows mirrored)
+__global__ void k_line_entries(const int *colofs, int nc, int W, const int *lptr,
+                               const unsigned *keys, int real, int m_zero, int2 *lent) {
+  const int q = blockIdx.x;
+  for (int m = threadIdx.x; m < nc; m += blockDim.x) {
+    const int co = colofs[(size_t)q * nc + m];
+    if (co < 0) continue;
+    const unsigned key = q * (unsigned)nc + m;
+    const int e0 = lptr[co / W], e1 = lptr[co / W + 1];
+    int pos = e0;
+    for (int e = e0; e < e1; ++e) pos += keys[e] < key;
+    const int flip = real && m < m_zero;
+    const int j = real ? (flip ? m_zero - m : m - m_zero) : m;
+    lent[pos] = make_int2(q, 2 * j + flip);
+  }
+}
+
 // I = sum / count (0 where count == 0), crop, f0 factor (comparison.py:765-786,
 // voxelgrids.py:16-48, :828-857).  Output in crop coordinates (qy,qx,qz).
 // One warp per (qy, qx) line, lanes along qz (the contiguous axis), lines
@@ -1628,6 +1712,53 @@ int enqueue(gw_voxel_plan *P) {
 
 namespace {
 
+// The gather's line table (window line -> entries in (phi, band column) order)
+// and its heavy lines: those with more than kGatherHeavy pixels per voxel
+// (entries times the structures each output sums; near the rotation axis).
+int gather_lines(gw_voxel_plan *P) {
+  gw_ctx *ctx = P->ctx;
+  cudaStream_t st = ctx->stream;
+  size_t &B = P->bytes;
+  struct Tmp {
+    void *p = nullptr;
+    cudaStream_t st;
+    // (the launches that use it have finished before it is given back)
+    ~Tmp() { if (p) { cudaStreamSynchronize(st); gw::dev_free(p); } }
+  };
+  const int n = P->W * P->W, nb = (n + kLineBlock - 1) / kLineBlock;
+  const int per_entry = P->p.average == GW_STRUCTS_SEPARATE ? 1 : P->n_struct;
+  const int64_t heavy_max = std::min<int64_t>(
+      n, (int64_t)P->n_phi * P->Nc * per_entry / (kGatherHeavy + 1) + 1);
+  GW_TRY(alloc(&P->d_lptr, (size_t)n + 1, &B));
+  GW_TRY(alloc(&P->d_heavy, (size_t)heavy_max, &B));
+  Tmp part{nullptr, st}, keys{nullptr, st};
+  GW_CUDA(gw::dev_malloc(&part.p, (size_t)(nb + 1) * sizeof(int2)));
+  int2 *sums = (int2 *)part.p, *total = sums + nb;
+  k_line_sums<<<nb, kLineBlock, 0, st>>>(P->d_C2, n, per_entry, kGatherHeavy, sums);
+  GW_LAUNCHED(ctx);
+  k_line_ptrs<<<nb, kLineBlock, 0, st>>>(P->d_C2, n, per_entry, kGatherHeavy, sums, P->d_lptr,
+                                         P->d_heavy, total);
+  GW_LAUNCHED(ctx);
+  int2 tot;
+  GW_CUDA(cudaMemcpyAsync(&tot, total, sizeof(tot), cudaMemcpyDeviceToHost, st));
+  GW_CUDA(cudaStreamSynchronize(st));
+  GW_TRY(alloc(&P->d_lent, (size_t)std::max(tot.x, 1), &B));
+  GW_CUDA(gw::dev_malloc(&keys.p, (size_t)std::max(tot.x, 1) * sizeof(unsigned)));
+  k_line_scatter<<<P->n_phi, 256, 0, st>>>(P->d_colofs, P->Nc, P->W, P->d_lptr,
+                                           (unsigned *)keys.p);
+  GW_LAUNCHED(ctx);
+  k_line_entries<<<P->n_phi, 256, 0, st>>>(P->d_colofs, P->Nc, P->W, P->d_lptr,
+                                           (unsigned *)keys.p, P->real ? 1 : 0, P->m_zero,
+                                           P->d_lent);
+  GW_LAUNCHED(ctx);
+  P->n_heavy = tot.y;
+  P->h_heavy.resize(tot.y);
+  if (tot.y)
+    GW_CUDA(cudaMemcpyAsync(P->h_heavy.data(), P->d_heavy, tot.y * sizeof(int),
+                            cudaMemcpyDeviceToHost, st));
+  return GW_OK;
+}
+
 // Gather binning: where it applies and the pixel store fits the budget
 // (GW_GATHER_MAX_MB, default 8192), its tables and store.  The column and
 // row tables of the plan are made.
@@ -1655,33 +1786,9 @@ int gather_setup(gw_voxel_plan *P) {
                     (P->p.binning == GW_BINNING_AUTO && P->real && P->n_struct == 1 &&
                      sum_bytes > P->ctx->l2_bytes);
   if (want && can) {
-    // the line entries, in table order (phi, band column): counting sort
-    // by window line
-    std::vector<int> cof((size_t)P->n_phi * P->Nc), rowofs(P->Nr);
-    GW_CUDA(cudaMemcpy(cof.data(), P->d_colofs, cof.size() * sizeof(int),
-                       cudaMemcpyDeviceToHost));
-    GW_CUDA(cudaMemcpy(rowofs.data(), P->d_rowofs, rowofs.size() * sizeof(int),
-                       cudaMemcpyDeviceToHost));
+    GW_TRY(gather_lines(P));
+    const std::vector<int> &rowofs = P->h_rowofs;
     const int W = P->W;
-    std::vector<int> lptr((size_t)W * W + 1, 0);
-    for (int co : cof)
-      if (co >= 0) ++lptr[co / W + 1];
-    for (size_t i = 1; i < lptr.size(); ++i) lptr[i] += lptr[i - 1];
-    std::vector<int2> lent(std::max(lptr.back(), 1));
-    std::vector<int> fill(lptr.begin(), lptr.end() - 1);
-    for (int q = 0; q < P->n_phi; ++q)
-      for (int m = 0; m < P->Nc; ++m) {
-        const int co = cof[(size_t)q * P->Nc + m];
-        if (co < 0) continue;
-        // F1 column of table column m: itself, or with real grids its
-        // mirror's (rows mirrored) below m_zero
-        int j = m, flip = 0;
-        if (P->real) {
-          if (m >= P->m_zero) j = m - P->m_zero;
-          else { j = P->m_zero - m; flip = 1; }
-        }
-        lent[fill[co / W]++] = make_int2(q, 2 * j + flip);
-      }
     // output rows of every window z, ascending
     std::vector<int> zptr((size_t)W + 1, 0);
     for (int ro : rowofs)
@@ -1697,19 +1804,7 @@ int gather_setup(gw_voxel_plan *P) {
       if (zptr[z + 1] - zptr[z] > 1) zmulti.push_back(z);
     P->n_zmulti = (int)zmulti.size();
     if (zmulti.empty()) zmulti.push_back(0);
-    // lines with more than kGatherHeavy pixels per voxel (entries times
-    // the structures each output sums; near the rotation axis)
-    const int per_entry = P->p.average == GW_STRUCTS_SEPARATE ? 1 : P->n_struct;
-    std::vector<int> heavy;
-    for (int l = 0; l < W * W; ++l)
-      if ((int64_t)(lptr[l + 1] - lptr[l]) * per_entry > kGatherHeavy) heavy.push_back(l);
-    P->n_heavy = (int)heavy.size();
-    P->h_heavy = heavy;
-    if (heavy.empty()) heavy.push_back(0);
-    GW_TRY(upload(&P->d_heavy, heavy, &B));
     GW_TRY(upload(&P->d_zmulti, zmulti, &B));
-    GW_TRY(upload(&P->d_lptr, lptr, &B));
-    GW_TRY(upload(&P->d_lent, lent, &B));
     GW_TRY(upload(&P->d_zptr, zptr, &B));
     GW_TRY(upload(&P->d_zrows, zrows, &B));
     GW_TRY(alloc(&P->d_G, g_bytes / sizeof(float), &B));
@@ -1851,7 +1946,8 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
   }
   P->kz0 = r0 - g / 2;
   P->Nr = r1 - r0 + 1;
-  std::vector<int> rowofs(P->Nr);
+  std::vector<int> &rowofs = P->h_rowofs;
+  rowofs.resize(P->Nr);
   for (int i = 0; i < P->Nr; ++i) {
     rowofs[i] = rowofs_all[r0 + i];
     if (rowofs[i] >= 0) P->C1host[rowofs[i]]++;

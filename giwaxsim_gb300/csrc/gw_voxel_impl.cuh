@@ -592,6 +592,7 @@ struct gw_voxel_plan {
   int64_t n_atoms = -1;
   size_t bytes = 0;
   std::vector<int> C1host;
+  std::vector<int> h_rowofs;  // the output rows' window z (host copy)
   // device
   double *d_xyz = nullptr;
   float2 *d_f = nullptr;

@@ -188,3 +188,30 @@ def test_chunked_result_copy(monkeypatch):
         assert np.array_equal(outs[k].view(np.uint64), outs["1"].view(np.uint64)), k
     assert not outs["1"][counts == 0].any()
     assert (outs["1"] >= 0).all()
+
+
+@pytest.mark.parametrize("max_q,n_phi", [(0.5, 5), (1.5, 7), (2.3, 180), (2.4, 361),
+                                         (3.0, 90)])
+def test_line_table(max_q, n_phi):
+    """The line table made on the device, from grids of less than one of its
+    blocks of lines to several: the same I(q) bits from every plan (entries in
+    table order whatever the order they were counted in), and the atomic
+    binning's to the accuracy of the compensated float32 sums."""
+    xyz = slab("C", 38, (12.0, 11.0, 13.0))
+    fv = np.full(len(xyz), 6.0 + 0.2j)
+    geom = F.VoxelGeometry(GEOM[0], GEOM[1], max_q)
+    phis = np.linspace(0.0, 180.0, n_phi, endpoint=False)
+    out = {}
+    for real in (None, False):
+        for k, binning in enumerate(("gather", "gather", "atomic")):
+            plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=phis, fill_bkg=True,
+                               binning=binning, real=real)
+            try:
+                plan.set_atoms()
+                plan.execute()
+                assert plan.info()["gather"] == (binning == "gather")
+                out[k] = plan.iq().copy()
+            finally:
+                plan.close()
+        assert np.array_equal(out[0].view(np.uint64), out[1].view(np.uint64))
+        assert rel_l2(out[0], out[2]) <= 1e-6
