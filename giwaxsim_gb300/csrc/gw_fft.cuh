@@ -20,6 +20,19 @@
 // the odd stride R-1, conflict-free) and tw[(r-1)*Ns + k] for odd R (lanes
 // read consecutive k).  No pass evaluates a transcendental.
 //
+// The inverse transform runs the passes transposed, in reverse order: the
+// transpose of a pass reads the strided slots, does the (conjugate) DFT,
+// multiplies by the same table's conjugates and writes j + r*(M/R), and the
+// DFT matrix is symmetric.  So its first pass takes exactly the values that
+// the last forward pass leaves in a thread's registers, and the two and the
+// multiplication by the filter between them are one pass over shared memory
+// without an exchange (fft_middle): four reads and four
+// writes instead of five at three passes, and two barriers fewer.  (Kernels
+// that are bound by these trips, their barriers and the twiddle reads: rows of
+// 640 / 1024 / 2048 points 74 -> 70 us, 3.15 -> 2.90 ms, 11.6 -> 11.0 ms;
+// columns of 384 / 640 / 1536 points 80 -> 60 us, 1.69 -> 1.37 ms, 3.10 -> 2.68
+// ms.)
+//
 // The first pass of a transform can read its inputs from a functor (global
 // memory) and the last pass can hand its outputs to a functor, so the
 // transform's input and output need no shared-memory round trip.
@@ -110,23 +123,41 @@ __host__ __device__ constexpr int tw_offset(int p) {
   return t;
 }
 
-// Generic pass.  SRC: 0 = shared memory (optionally multiplied by pre[n]),
-// 1 = load(f, n).  DST: 0 = shared memory, 1 = store(f, m, value).
+// v[r] times W_{NS R}^{r k} (conjugated with CONJ).
+template <int R, int NS, bool CONJ>
+__device__ __forceinline__ void fft_twiddle(float2 (&v)[R], const float2 *tw, int k) {
+  if constexpr (R & 1) {
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], conj_if<CONJ>(tw[(r - 1) * NS + k]));
+  } else {
+    const float2 *t = tw + k * (R - 1) - 1;
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], conj_if<CONJ>(t[r]));
+  }
+}
+
+// Slot of output r of butterfly j of the forward pass (R, NS) in sequence f.
+template <int M, int R, int NS>
+__device__ __forceinline__ float2 *fft_strided(float2 *buf, int f, int j, int r) {
+  const int base = (j / NS) * NS * R + j % NS;
+  // NS a multiple of 16: fft_pad(base + r NS) = fft_pad(base) + r (NS + NS/16);
+  // NS = 1 and R = 16 with base = 16 j: + r
+  constexpr bool kStride = NS % 16 == 0 || (NS == 1 && R == 16);
+  constexpr int kStep = NS == 1 ? 1 : NS + NS / 16;
+  float2 *p = buf + f * FftPlan<M>::LDM;
+  return kStride ? p + fft_pad(base) + r * kStep : p + fft_pad(base + r * NS);
+}
+
+// Forward pass into shared memory.  SRC: 0 = shared memory, 1 = load(f, n).
 // FFAST maps the sequence index f fastest across threads (column loads from
 // global memory); otherwise the butterfly index j is fastest.
-// Pruning (the chirp-z window and band are shorter than M): HIN, in a first
-// pass (NS = 1), reads only the inputs r < R/2 of each butterfly (the
-// others, n >= M/2, are zero) and transforms them with the pruned register
-// DFT; HOUT, in a last pass, produces only the outputs r < ceil(R/2) (the
-// others, m >= M/2, are not wanted), the rest being dead code.
-template <int M, int R, int NS, int NB, int NT, bool INV, int SRC, bool PREMUL,
-          int DST, bool FFAST, bool HIN = false, bool HOUT = false, class Load,
-          class Store>
-__device__ __forceinline__ void fft_pass(float2 *buf, const float2 *tw,
-                                         const float2 *pre, Load load,
-                                         Store store) {
+// HIN (a first pass, NS = 1; the chirp-z window is within M/2): reads only
+// the inputs r < R/2 of each butterfly (the others, n >= M/2, are zero) and
+// transforms them with the pruned register DFT.
+template <int M, int R, int NS, int NB, int NT, int SRC, bool FFAST, bool HIN, class Load>
+__device__ __forceinline__ void fft_pass(float2 *buf, const float2 *tw, Load load) {
   static_assert(!HIN || NS == 1, "input pruning is for a first pass");
-  constexpr int KIN = HIN ? R / 2 : R, KOUT = HOUT ? (R + 1) / 2 : R;
+  constexpr int KIN = HIN ? R / 2 : R;
   constexpr int Q = M / R;
   constexpr int BF = NB * Q;
   constexpr int PER = (BF + NT - 1) / NT;
@@ -144,60 +175,107 @@ __device__ __forceinline__ void fft_pass(float2 *buf, const float2 *tw,
 #pragma unroll
       for (int r = 0; r < KIN; ++r) {
         const int n = j + r * Q;
-        if (SRC == 0) {
-          float2 x = Q % 16 == 0 ? src[r * (Q + Q / 16)] : buf[f * LDM + fft_pad(n)];
-          if (PREMUL) x = cmul(x, __ldg(pre + n));
-          v[e][r] = x;
-        } else {
+        if (SRC == 0)
+          v[e][r] = Q % 16 == 0 ? src[r * (Q + Q / 16)] : buf[f * LDM + fft_pad(n)];
+        else
           v[e][r] = load(f, n);
-        }
       }
-      if (NS > 1) {
-        const int k = j % NS;
-        if constexpr (R & 1) {
-#pragma unroll
-          for (int r = 1; r < R; ++r)
-            v[e][r] = cmul(v[e][r], conj_if<INV>(tw[(r - 1) * NS + k]));
-        } else {
-          const float2 *t = tw + k * (R - 1) - 1;
-#pragma unroll
-          for (int r = 1; r < R; ++r) v[e][r] = cmul(v[e][r], conj_if<INV>(t[r]));
-        }
-      }
-      if constexpr (HIN) gwd::dft_prefix<R, KIN, INV>(v[e]);
-      else dft<R, INV>(v[e]);
+      if constexpr (NS > 1) fft_twiddle<R, NS, false>(v[e], tw, j % NS);
+      if constexpr (HIN) gwd::dft_prefix<R, KIN, false>(v[e]);
+      else dft<R, false>(v[e]);
     }
   }
   // The writes wait for every thread's reads (passes are in place; a first
-  // pass may read inputs that alias its shared destination), except in a
-  // last pass (NS R = M): there Q = NS, so base = j and a butterfly writes
-  // exactly the slots j + r Q it read, which no other thread touches.
-  constexpr bool kOwnSlots = NS * R == M && SRC == 0;
-  if (DST == 0 && !kOwnSlots) __syncthreads();
+  // pass may read inputs that alias its shared destination).
+  __syncthreads();
 #pragma unroll
   for (int e = 0; e < PER; ++e) {
     const int b = threadIdx.x + e * NT;
     if (BF % NT == 0 || b < BF) {
       const int f = FFAST ? b % NB : b / Q;
       const int j = FFAST ? b / NB : b % Q;
-      const int k = j % NS;
-      const int base = (j / NS) * NS * R + k;
-      // NS a multiple of 16: fft_pad(base + r NS) = fft_pad(base) + r (NS + NS/16);
-      // NS = 1 and R <= 16 with base = j R a multiple of 16 (R = 16): + r
-      constexpr bool kStride = NS % 16 == 0 || (NS == 1 && R == 16);
-      constexpr int kStep = NS == 1 ? 1 : NS + NS / 16;
-      float2 *dst = buf + f * LDM + fft_pad(base);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        // dft_prefix leaves natural order, dft its out_slot order
+        *fft_strided<M, R, NS>(buf, f, j, r) = HIN ? v[e][r] : v[e][out_slot<R>(r)];
+    }
+  }
+  __syncthreads();
+}
+
+// The last forward pass (NS R = M), the multiplication by H and the first
+// inverse pass, which take and leave the same slots j + r NS: one read and one
+// write of the buffer, nothing exchanged between threads.
+template <int M, int R, int NS, int NB, int NT>
+__device__ __forceinline__ void fft_middle(float2 *buf, const float2 *tw, const float2 *H) {
+  static_assert(NS * R == M && NS % 16 == 0, "last pass");
+  constexpr int BF = NB * NS;
+  constexpr int PER = (BF + NT - 1) / NT;
+  constexpr int LDM = FftPlan<M>::LDM, STEP = NS + NS / 16;
+#pragma unroll
+  for (int e = 0; e < PER; ++e) {
+    const int b = threadIdx.x + e * NT;
+    if (BF % NT == 0 || b < BF) {
+      const int f = b / NS, j = b % NS;
+      float2 *p = buf + f * LDM + fft_pad(j);
+      float2 v[R], w[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[r * STEP];
+      fft_twiddle<R, NS, false>(v, tw, j);
+      dft<R, false>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = cmul(v[out_slot<R>(r)], __ldg(H + j + r * NS));
+      dft<R, true>(w);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = w[out_slot<R>(r)];
+      fft_twiddle<R, NS, true>(v, tw, j);
+#pragma unroll
+      for (int r = 0; r < R; ++r) p[r * STEP] = v[r];
+    }
+  }
+  __syncthreads();
+}
+
+// Inverse pass: the forward pass (R, NS) transposed.  DST: 0 = shared memory,
+// 1 = store(f, m, value).  HOUT (the last one, NS = 1; the band is within
+// M/2): produces only the outputs r < R/2 (the others, m >= M/2, are not
+// wanted), the rest being dead code.
+template <int M, int R, int NS, int NB, int NT, int DST, bool HOUT, class Store>
+__device__ __forceinline__ void fft_pass_inv(float2 *buf, const float2 *tw, Store store) {
+  static_assert((!HOUT && !DST) || NS == 1, "outputs leave a last pass");
+  constexpr int KOUT = HOUT ? (R + 1) / 2 : R;
+  constexpr int Q = M / R;
+  constexpr int BF = NB * Q;
+  constexpr int PER = (BF + NT - 1) / NT;
+  constexpr int LDM = FftPlan<M>::LDM;
+  float2 v[PER][R];
+#pragma unroll
+  for (int e = 0; e < PER; ++e) {
+    const int b = threadIdx.x + e * NT;
+    if (BF % NT == 0 || b < BF) {
+      const int f = b / Q, j = b % Q;
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[e][r] = *fft_strided<M, R, NS>(buf, f, j, r);
+      dft<R, true>(v[e]);
+    }
+  }
+  if (DST == 0) __syncthreads();
+#pragma unroll
+  for (int e = 0; e < PER; ++e) {
+    const int b = threadIdx.x + e * NT;
+    if (BF % NT == 0 || b < BF) {
+      const int f = b / Q, j = b % Q;
+      float2 w[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = v[e][out_slot<R>(r)];
+      if constexpr (NS > 1) fft_twiddle<R, NS, true>(w, tw, j % NS);
+      float2 *dst = buf + f * LDM + fft_pad(j);
 #pragma unroll
       for (int r = 0; r < KOUT; ++r) {
-        const int m = base + r * NS;
-        // dft_prefix leaves natural order, dft its out_slot order
-        const float2 val = HIN ? v[e][r] : v[e][out_slot<R>(r)];
-        if (DST == 0) {
-          if (kStride) dst[r * kStep] = val;
-          else buf[f * LDM + fft_pad(m)] = val;
-        } else {
-          store(f, m, val);
-        }
+        const int m = j + r * Q;
+        if (DST == 1) store(f, m, w[r]);
+        else if (Q % 16 == 0) dst[r * (Q + Q / 16)] = w[r];
+        else buf[f * LDM + fft_pad(m)] = w[r];
       }
     }
   }
@@ -211,45 +289,38 @@ struct NoStore {
   __device__ void operator()(int, int, float2) const {}
 };
 
-// Whole transform.  The first pass reads shared memory (SRC=0, times pre[n]
-// when PREMUL) or load(f, n) (SRC=1); the last pass writes shared memory
-// (DST=0) or calls store(f, m, value) (DST=1).  Middle passes stay in shared
-// memory.  A transform ending in shared memory leaves the block synchronised.
+// Whole chirp-z convolution: forward transform, times H, inverse transform
+// (not scaled).  The first pass reads shared memory (SRC = 0) or load(f, n)
+// (SRC = 1); the last one writes shared memory in natural order (DST = 0; the
+// block is synchronised afterwards) or calls store(f, m, value) (DST = 1).
 // HIN / HOUT: the first pass reads only the first half of its inputs / the
-// last pass produces only the first half of its outputs (fft_pass).
-template <int M, int NB, int NT, bool INV, int SRC, bool PREMUL, int DST,
-          bool FFAST_FIRST, bool HIN = false, bool HOUT = false, class Load,
-          class Store>
-__device__ __forceinline__ void fft_run(float2 *buf, const float2 *tw,
-                                        const float2 *pre, Load load,
-                                        Store store) {
+// last pass produces only the first half of its outputs.
+template <int M, int NB, int NT, int SRC, int DST, bool FFAST_FIRST, bool HIN, bool HOUT,
+          class Load, class Store>
+__device__ __forceinline__ void czt_run(float2 *buf, const float2 *tw, const float2 *H,
+                                        Load load, Store store) {
   using Pl = FftPlan<M>;
-  static_assert(Pl::N16 >= 1, "M >= 16");
-  if constexpr (Pl::NPASS == 1) {
-    fft_pass<M, 16, 1, NB, NT, INV, SRC, PREMUL, DST, FFAST_FIRST, HIN, HOUT>(
-        buf, tw, pre, load, store);
-  } else {
-    fft_pass<M, 16, 1, NB, NT, INV, SRC, PREMUL, 0, FFAST_FIRST, HIN, false>(
-        buf, tw, pre, load, NoStore());
-    if constexpr (Pl::N16 >= 2) {
-      constexpr int dst = Pl::NPASS == 2 ? DST : 0;
-      fft_pass<M, 16, 16, NB, NT, INV, 0, false, dst, false, false,
-               HOUT && Pl::NPASS == 2>(buf, tw + tw_offset<M>(1), nullptr, NoLoad(), store);
-    }
-    if constexpr (Pl::N16 >= 3) {
-      constexpr int dst = Pl::NPASS == 3 ? DST : 0;
-      fft_pass<M, 16, 256, NB, NT, INV, 0, false, dst, false, false,
-               HOUT && Pl::NPASS == 3>(buf, tw + tw_offset<M>(2), nullptr, NoLoad(), store);
-    }
-    if constexpr (Pl::R2 > 1) {
-      constexpr int NS2 = 1 << (4 * Pl::N16);
-      constexpr int dst = Pl::F == 1 ? DST : 0;
-      fft_pass<M, Pl::R2, NS2, NB, NT, INV, 0, false, dst, false, false,
-               HOUT && Pl::F == 1>(buf, tw + Pl::tw_r2(), nullptr, NoLoad(), store);
-    }
-    if constexpr (Pl::F > 1) {
-      fft_pass<M, Pl::F, Pl::P2, NB, NT, INV, 0, false, DST, false, false, HOUT>(
-          buf, tw + Pl::tw_f(), nullptr, NoLoad(), store);
-    }
-  }
+  static_assert(Pl::NPASS >= 2, "M >= 32");
+  constexpr int N16 = Pl::N16, R2 = Pl::R2, F = Pl::F, P16 = 1 << (4 * N16);
+  fft_pass<M, 16, 1, NB, NT, SRC, FFAST_FIRST, HIN>(buf, tw, load);
+  // the passes between the first and the last, there and back
+  constexpr bool k16 = N16 >= 3 || (N16 == 2 && (R2 > 1 || F > 1));
+  constexpr bool k256 = N16 == 3 && (R2 > 1 || F > 1);
+  constexpr bool kR2 = R2 > 1 && F > 1;
+  if constexpr (k16)
+    fft_pass<M, 16, 16, NB, NT, 0, false, false>(buf, tw + tw_offset<M>(1), NoLoad());
+  if constexpr (k256)
+    fft_pass<M, 16, 256, NB, NT, 0, false, false>(buf, tw + tw_offset<M>(2), NoLoad());
+  if constexpr (kR2)
+    fft_pass<M, R2, P16, NB, NT, 0, false, false>(buf, tw + Pl::tw_r2(), NoLoad());
+  if constexpr (F > 1) fft_middle<M, F, Pl::P2, NB, NT>(buf, tw + Pl::tw_f(), H);
+  else if constexpr (R2 > 1) fft_middle<M, R2, P16, NB, NT>(buf, tw + Pl::tw_r2(), H);
+  else fft_middle<M, 16, P16 / 16, NB, NT>(buf, tw + tw_offset<M>(N16 - 1), H);
+  if constexpr (kR2)
+    fft_pass_inv<M, R2, P16, NB, NT, 0, false>(buf, tw + Pl::tw_r2(), NoStore());
+  if constexpr (k256)
+    fft_pass_inv<M, 16, 256, NB, NT, 0, false>(buf, tw + tw_offset<M>(2), NoStore());
+  if constexpr (k16)
+    fft_pass_inv<M, 16, 16, NB, NT, 0, false>(buf, tw + tw_offset<M>(1), NoStore());
+  fft_pass_inv<M, 16, 1, NB, NT, DST, HOUT>(buf, tw, store);
 }

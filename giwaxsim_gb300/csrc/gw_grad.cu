@@ -211,8 +211,7 @@ k_col_bwd(SliceArgs a, CztArgs cz, BinArgs bn, GradCol gc, int slice0, int nc,
   int first, rows;
   slice_rows(a, slice0, sl, first, rows);
   ColLoadF1 ld{F1 + (size_t)first * nc, cz.A, rows, nc, m0};
-  fft_run<M, NB, NT, false, 1, false, 0, true, HALF>(buf, tw, nullptr, ld, NoStore());
-  fft_run<M, NB, NT, true, 0, true, 0, false, false, HALF>(buf, tw, cz.H, NoLoad(), NoStore());
+  czt_run<M, NB, NT, 1, 0, true, HALF, HALF>(buf, tw, cz.H, ld, NoStore());
   const float2 cbg = slice_const(a, sl).cbg;
   for (int t = threadIdx.x; t < NB * M; t += NT) {
     const int f = t / M, mr = t - f * M;
@@ -239,9 +238,8 @@ k_col_bwd(SliceArgs a, CztArgs cz, BinArgs bn, GradCol gc, int slice0, int nc,
     buf[f * LDM + fft_pad(mr)] = out;
   }
   __syncthreads();
-  fft_run<M, NB, NT, false, 0, false, 0, false, HALF>(buf, tw, nullptr, NoLoad(), NoStore());
   ColStoreAdj st{gc.Ba, gc.G1 + (size_t)slot * a.Lz * nc, a.Lz, nc, m0};
-  fft_run<M, NB, NT, true, 0, true, 1, false, false, HALF>(buf, tw, gc.Ha, NoLoad(), st);
+  czt_run<M, NB, NT, 0, 1, false, HALF, HALF>(buf, tw, gc.Ha, NoLoad(), st);
 }
 
 // ------------------------------------------------------------ row stage
@@ -329,8 +327,7 @@ k_row_bwd(SliceArgs a, GradRow gr, int slice0, int n_sl, int n_rows) {
   }
   __syncthreads();
   RowLoadAdj<M> ld{gr.G1, gr.Aa, gr.nc, a.Lz, r_slot, r_zz, row0, n_rows};
-  fft_run<M, NB, NT, false, 1, false, 0, true, HALF>(buf, tw, nullptr, ld, NoStore());
-  fft_run<M, NB, NT, true, 0, true, 0, false, false, HALF>(buf, tw, gr.Ha, NoLoad(), NoStore());
+  czt_run<M, NB, NT, 1, 0, true, HALF, HALF>(buf, tw, gr.Ha, ld, NoStore());
   // G_D on the window, and the per-row sums of G_D m and G_D dm/dsigma:
   // warps w, w + NB, .. take row w % NB (several rows a warp when there are
   // fewer warps than rows)

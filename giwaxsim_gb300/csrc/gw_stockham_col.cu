@@ -134,6 +134,9 @@ k_col_czt_bin(SliceArgs a, CztArgs cz, BinArgs bn, int slice0, int nc, int nf,
   }
   for (int t = threadIdx.x; t < TWL; t += NT) tw[t] = cz.tw[t];
   __syncthreads();
+  ColBin st{bn, cofs, cz.B, a.sdc + sl, cz.N, nc, j0, moff,
+            bn.sstride * (int64_t)(sl / a.n_phi),
+            bn.G ? bn.G + ((size_t)sl * nf + j0) * cz.N : nullptr};
   if constexpr (TMA) {
     // one decision for the whole block: every thread goes on, or none
     if (!__syncthreads_and(mbar_wait_bounded(&tile_bar, 0, bn.wait_polls))) {
@@ -144,17 +147,11 @@ k_col_czt_bin(SliceArgs a, CztArgs cz, BinArgs bn, int slice0, int nc, int nf,
       return;
     }
     ColTileLoad<NB> ld{tile, cz.A, rows, nf, j0};
-    fft_run<M, NB, NT, false, 1, false, 0, true, HALF, false>(buf, tw, nullptr, ld,
-                                                             NoStore());
+    czt_run<M, NB, NT, 1, 1, true, HALF, HALF>(buf, tw, cz.H, ld, st);
   } else {
     ColLoad ld{F1 + (size_t)first * nf, cz.A, rows, nf, j0};
-    fft_run<M, NB, NT, false, 1, false, 0, true, HALF, false>(buf, tw, nullptr, ld,
-                                                             NoStore());
+    czt_run<M, NB, NT, 1, 1, true, HALF, HALF>(buf, tw, cz.H, ld, st);
   }
-  ColBin st{bn, cofs, cz.B, a.sdc + sl, cz.N, nc, j0, moff,
-            bn.sstride * (int64_t)(sl / a.n_phi),
-            bn.G ? bn.G + ((size_t)sl * nf + j0) * cz.N : nullptr};
-  fft_run<M, NB, NT, true, 0, true, 1, false, false, HALF>(buf, tw, cz.H, NoLoad(), st);
 }
 
 }  // namespace

@@ -19,8 +19,8 @@ namespace {
 // z-sorted arrays) into shared-memory row buffers with shared atomics
 // (voxelgrids.py:328-341: shift, floor division, valid mask, np.add.at).
 // The forward FFT's first pass reads those rows with the fill/smoothing
-// transform and the chirp A; the inverse FFT's first pass multiplies by the
-// filter spectrum H, and its last pass writes F1 = B * result to global
+// transform and the chirp A; the middle pass multiplies by the filter
+// spectrum H, and the inverse FFT's last pass writes F1 = B * result to global
 // memory.  The row buffers share storage with the FFT buffer: the first pass
 // reads all its inputs before it writes.
 template <int M>
@@ -69,10 +69,8 @@ k_row_czt(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
   const int row0 = blockIdx.x * NB;
   deposit_rows<NB, NT, BIL>(a, cz.L, slice0, n_sl, n_rows, row0, buf, LDM, rs);
   RowLoad<M> ld{row_value_args(a), cz.A, cz.L, buf, rs.k, row0, n_rows};
-  fft_run<M, NB, NT, false, 1, false, 0, false, HALF, false>(buf, tw, nullptr, ld,
-                                                            NoStore());
   RowStore stv{cz.B, F1, row0, n_rows, nc_out};
-  fft_run<M, NB, NT, true, 0, true, 1, false, false, HALF>(buf, tw, cz.H, NoLoad(), stv);
+  czt_run<M, NB, NT, 1, 1, false, HALF, HALF>(buf, tw, cz.H, ld, stv);
 }
 
 // Real grids: when every atom's f is a real multiple of one complex value,
@@ -134,13 +132,10 @@ k_row_czt_real(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
   __syncthreads();
   RowLoadPair<M> ld{a.fill || a.smooth_on ? a.pr : nullptr, cz.A, cz.L,
                     reinterpret_cast<const float *>(buf), mz, rs.slot};
-  fft_run<M, NB, NT, false, 1, false, 0, false, HALF, false>(buf, tw, nullptr, ld,
-                                                            NoStore());
   // the inverse transform stays in shared memory (natural order; with HALF
   // only the outputs below M/2, which hold the band); the block is
   // synchronised afterwards
-  fft_run<M, NB, NT, true, 0, true, 0, false, false, HALF>(buf, tw, cz.H, NoLoad(),
-                                                          NoStore());
+  czt_run<M, NB, NT, 1, 0, false, HALF, HALF>(buf, tw, cz.H, ld, NoStore());
   for (int f = 0; f < NB; ++f) {
     for (int j = threadIdx.x; j < nf; j += NT) {
       const int m = m_zero + j, mm = m_zero - j;  // k and -k
