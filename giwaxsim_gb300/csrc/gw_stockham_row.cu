@@ -51,14 +51,38 @@ struct RowStore {
   }
 };
 
+// Sequences and threads of a row block (and the blocks per SM that its
+// registers are sized for): half of the column kernels' and the adjoint's from
+// 512 points up, so that more blocks are resident and one's barriers, row
+// set-up and deposit hide behind the others'.  Rows of 512 / 640 / 1024 / 1280
+// / 1536 / 2048 points of real grids took 49.3 / 69.7 / 98.9 / 150 / 218 / 271
+// us in 180 slices of 110 x 110 x 40 A and the like, and take 43.9 / 61.5 /
+// 94.9 / 136 / 187 / 248; general rows of 640 / 1280 / 1536 / 2048 points 117 /
+// 260 / 381 / 468, now 107 / 245 / 338 / 440.  The general rows of 512, 768 and
+// 1024 points keep the larger block: there the smaller one won 8, 0 and 1 % with
+// 180 atoms a row and lost 7 and 4 % (512, 1024) with 80 (less L1 is left beside
+// more copies of the twiddles).
+template <int M, bool REAL>
+struct RowShape : FftShape<M> {};
+template <> struct RowShape<512, true>  { static constexpr int NB = 4, NT = 128, MINB = 8; };
+template <> struct RowShape<768, true>  { static constexpr int NB = 2, NT = 96,  MINB = 10; };
+template <> struct RowShape<1024, true> { static constexpr int NB = 2, NT = 128, MINB = 8; };
+template <bool REAL>
+struct RowShape<640, REAL>  { static constexpr int NB = 4, NT = 160, MINB = 6; };
+template <bool REAL>
+struct RowShape<1280, REAL> { static constexpr int NB = 2, NT = 160, MINB = 6; };
+template <bool REAL>
+struct RowShape<1536, REAL> { static constexpr int NB = 2, NT = 192, MINB = 5; };
+template <bool REAL>
+struct RowShape<2048, REAL> { static constexpr int NB = 2, NT = 256, MINB = 4; };
+
 // HALF: the window (L) and the band (N) both fit in M / 2, so the forward
 // transform's first pass and the inverse transform's last pass are pruned.
 template <int M, bool BIL, bool HALF>
-__global__ void __launch_bounds__(FftShape<M>::NT,
-                                  HALF ? minb_pruned_rows<M>() : FftShape<M>::MINB)
+__global__ void __launch_bounds__(RowShape<M, false>::NT, RowShape<M, false>::MINB)
 k_row_czt(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
           int nc_out, float2 *F1) {
-  constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
+  constexpr int NB = RowShape<M, false>::NB, NT = RowShape<M, false>::NT;
   constexpr int TWL = FftPlan<M>::tw_len();
   constexpr int LDM = FftPlan<M>::LDM;
   extern __shared__ float2 smem[];
@@ -111,11 +135,10 @@ struct RowLoadPair {
 };
 
 template <int M, bool HALF>
-__global__ void __launch_bounds__(FftShape<M>::NT,
-                                  HALF ? minb_pruned_rows<M>() : FftShape<M>::MINB)
+__global__ void __launch_bounds__(RowShape<M, true>::NT, RowShape<M, true>::MINB)
 k_row_czt_real(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
                int m_zero, int nf, float2 *F1) {
-  constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
+  constexpr int NB = RowShape<M, true>::NB, NT = RowShape<M, true>::NT;
   constexpr int TWL = FftPlan<M>::tw_len();
   constexpr int LDM = FftPlan<M>::LDM;
   static_assert(LDM % 2 == 0, "two rows per transform buffer");
@@ -160,7 +183,7 @@ template <int M, bool BIL, bool HALF>
 int launch_row_t(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
                  int slice0, int n_sl) {
   const int n_rows = batch_rows(P, slice0, n_sl);
-  constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
+  constexpr int NB = RowShape<M, false>::NB, NT = RowShape<M, false>::NT;
   const size_t smem = (size_t)(NB * FftPlan<M>::LDM + FftPlan<M>::tw_len()) * sizeof(float2);
   static gw::SmemRecord attr;
   GW_TRY(gw::smem_limit(attr, k_row_czt<M, BIL, HALF>, smem));
@@ -176,7 +199,7 @@ template <int M, bool HALF>
 int launch_row_real(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
                     int slice0, int n_sl) {
   const int n_rows = batch_rows(P, slice0, n_sl);
-  constexpr int NB = FftShape<M>::NB, NT = FftShape<M>::NT;
+  constexpr int NB = RowShape<M, true>::NB, NT = RowShape<M, true>::NT;
   const size_t smem = (size_t)(NB * FftPlan<M>::LDM + FftPlan<M>::tw_len()) * sizeof(float2);
   static gw::SmemRecord attr;
   GW_TRY(gw::smem_limit(attr, k_row_czt_real<M, HALF>, smem));
@@ -191,7 +214,7 @@ int launch_row_real(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
 template <int M>
 int launch_row(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
                int slice0, int n_sl) {
-  if constexpr (M <= 2048 && FftShape<M>::NB <= 16) {
+  if constexpr (M <= 2048) {
     if (P->real)
       return pruned<M>(cz) ? launch_row_real<M, true>(P, a, cz, slice0, n_sl)
                            : launch_row_real<M, false>(P, a, cz, slice0, n_sl);
