@@ -683,10 +683,10 @@ __global__ void k_col_tables(const gw_phi *ph, int g, int k0, int nc,
 
 // The gather's line table from the counts per window line: lptr, its entries
 // and the heavy lines, so that a plan's creation neither reads the column
-// tables back nor sorts them on the host (403^3 at 360 angles: @HOST@ against
-// @DEV@ us).  Two launches of a block scan each (line_sums: a block's totals;
-// line_ptrs: the totals before it, then its own lines), kLineBlock lines a
-// block.  line_ptrs leaves line l's start in lptr[l + 1]; line_scatter counts
+// tables back nor sorts them on the host (creation of a plan of 403^3 voxels at
+// 360 angles 2.0 -> 0.68 ms).  Two launches of a block scan each (line_sums: a
+// block's totals; line_ptrs: the totals before it, then its own lines),
+// kLineBlock lines a block.  line_ptrs leaves line l's start in lptr[l + 1]; line_scatter counts
 // it up to the line's end while it takes the keys phi Nc + m in any order, and
 // line_entries puts each entry at its key's rank in the line: table order.
 constexpr int kLineBlock = 1024;
