@@ -187,11 +187,11 @@ __device__ __forceinline__ bool fast_index(const OrientFast &T, const DetArgs &a
 // When every orientation keeps the same axis at a fixed index (the plane
 // rotated about its own normal, the reference's psi rotations), all samples
 // lie in one plane of I(q).  The plane is copied to a compact nu x nv array
-// (u, v the two free axes in memory order) and each block gathers from it:
-// from shared memory when the plane fits, else from global memory through
-// L1.  Blocks own 16 x 32 pixel tiles, so that per orientation a block's
-// samples cover a compact patch of the plane.  Indices, worklist decisions
-// and the per-pixel accumulation order are those of the general mode; only
+// (u, v the two free axes in memory order) and each block gathers from it
+// through L1 (a copy of the plane in shared memory, where it fits, holds one
+// block an SM: 91 rotations of 500 px in 203^2 59 us, without it 50).  A
+// block's tile keeps its samples of one orientation within a compact patch of
+// the plane.  Indices, worklist decisions and the per-pixel accumulation order are those of the general mode; only
 // the order in which k_detector_fix atomically adds the replayed samples
 // differs (it is scheduling order in both).
 struct PlaneArgs {
@@ -211,13 +211,41 @@ struct __align__(16) PlaneOrient {
   float w, pad;
 };
 static_assert(sizeof(PlaneOrient) == 48, "three 16-byte words per orientation");
-constexpr int kPlTW = 32, kPlTH = 32, kPlThreads = 512;
+// First worklist slot of this lane's need set bits: one add per warp, as a
+// pixel on an index' edge is uncertain at every orientation and an add and its
+// answer per sample were the longest warp's time (203 x 203 pixels in
+// 101^3, 720 orientations, some pixels at q = 0: 688 us so, now 215).  All lanes
+// call.
+__device__ __forceinline__ int worklist_slots(unsigned need, int *wl_count) {
+  const int lane = threadIdx.x & 31, n = __popc(need);
+  int end = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += v;
+  }
+  int base = 0;
+  if (lane == 31) base = atomicAdd(wl_count, end);
+  return __shfl_sync(0xffffffffu, base, 31) + end - n;
+}
+
+// A block owns a tile of 16 x 16 pixels, a thread two pixels kPlRows rows apart,
+// a warp 8 x 4 and the same kPlRows below: small blocks, as a detector has few
+// tiles and the last ones set the time (general mode, 2880 orientations of 500
+// px 1.37 ms with 32 x 32 tiles, 1.20 with 16 x 16; 300 orientations of 500 px in
+// 351^3 0.21 and 0.15 ms, but 0.30 with 16 x 8).  The samples of kPlBatch
+// orientations are loaded before the first is used: 300 of 351^3 155 us with 2
+// at a time, 153 with 4, 144 with 8; 91 rotations of 1000 px in the plane of
+// 403^2 122 -> 108 us against one load at a time, 181 of 100 px 38 -> 25.
+constexpr int kPlTile = 16, kPlThreads = 128, kPlRows = 8, kPlBatch = 8;
+static_assert(kPlTile * kPlTile == 2 * kPlThreads, "two pixels a thread");
+__device__ __forceinline__ int tile_col(int t) { return t / 32 % 2 * 8 + t % 8; }
+__device__ __forceinline__ int tile_row(int t) { return t / 64 * 4 + t % 32 / 8; }
+
 // A compile-time bool as a value (selects a lambda's instantiation).
 template <bool B>
 struct BoolC {
   static constexpr bool value = B;
 };
-constexpr size_t kPlaneSmemMax = 200 * 1024;
 
 __global__ void k_plane_extract(DetArgs a, PlaneArgs pa, float *P) {
   const int64_t n = (int64_t)pa.nu * pa.nv;
@@ -258,23 +286,16 @@ __device__ __forceinline__ bool plane_index(const PlaneOrient &T, float2 n1,
   return (fmaxf(lo.x, 0.f) >= fl.x) & (fmaxf(lo.y, 0.f) >= fl.y);
 }
 
-template <bool SMEM, bool ZX>
+template <bool ZX>
 __global__ void __launch_bounds__(kPlThreads)
 k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
                  double *acc_out, int2 *wl, int *wl_count, int wl_cap) {
-  extern __shared__ float s_plane[];
   __shared__ PlaneOrient s_ot[kDetChunk];
-  constexpr int KP = kPlTH * kPlTW / kPlThreads;  // pixels per thread
+  constexpr int KP = 2;  // pixels per thread
   const float2 n1 = make_float2((float)(pa.nu - 1), (float)(pa.nv - 1));
-  const int tiles_x = (a.nh + kPlTW - 1) / kPlTW;
-  const int j = (blockIdx.x % tiles_x) * kPlTW + (threadIdx.x % kPlTW);
-  const int ib = (blockIdx.x / tiles_x) * kPlTH + threadIdx.x / kPlTW;
-  const float *src = pa.P;
-  if (SMEM) {
-    const int n = pa.nu * pa.nv;
-    for (int t = threadIdx.x; t < n; t += kPlThreads) s_plane[t] = pa.P[t];
-    src = s_plane;
-  }
+  const int tiles_x = (a.nh + kPlTile - 1) / kPlTile;
+  const int j = (blockIdx.x % tiles_x) * kPlTile + tile_col(threadIdx.x);
+  const int ib = (blockIdx.x / tiles_x) * kPlTile + tile_row(threadIdx.x);
   int pix[KP];
   bool valid[KP];
   float xf[KP], yf[KP], zf[KP];
@@ -282,7 +303,7 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
   float part[KP];
 #pragma unroll
   for (int k = 0; k < KP; ++k) {
-    const int i = ib + k * (kPlThreads / kPlTW);
+    const int i = ib + k * kPlRows;
     valid[k] = i < a.nv && j < a.nh;
     pix[k] = valid[k] ? i * a.nh + j : 0;
     double x0 = 0.0, y0 = 0.0, z0 = 0.0;
@@ -291,6 +312,7 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
     acc[k] = 0.0;
     part[k] = 0.f;
   }
+  const unsigned vmask = (valid[0] ? 0x55555555u : 0u) | (valid[1] ? 0xaaaaaaaau : 0u);
   // tiles wholly inside the detector (all but the last tile row and
   // column) run the loop without the per-pixel validity tests
   auto orient_loop = [&](auto all_valid) {
@@ -308,35 +330,55 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
         // bit (oo - g0) KP + k: a sample whose index is not certain in
         // float32, replayed in float64 after the group
         unsigned need_bits = 0;
-  #pragma unroll 2
-        for (int oo = g0; oo < ge; ++oo) {
-          // three 16-byte loads; each holds two (u, v) pairs
-          const float4 *q = reinterpret_cast<const float4 *>(s_ot + oo);
-          const float4 q0 = q[0], q1 = q[1], q2 = q[2];
-          PlaneOrient T;
-          T.x = make_float2(q0.x, q0.y);
-          T.y = make_float2(q0.z, q0.w);
-          T.z = make_float2(q1.x, q1.y);
-          T.c = make_float2(q1.z, q1.w);
-          T.d = make_float2(q2.x, q2.y);
-          T.w = q2.z;
+        for (int oo = g0; oo < ge; oo += kPlBatch) {
+          // every index is clamped, so the samples of kPlBatch orientations are
+          // loaded unconditionally, all in flight at once
+          int at[kPlBatch][KP];
+          float w[kPlBatch], v[kPlBatch][KP];
+          unsigned ok = 0;
   #pragma unroll
-          for (int k = 0; k < KP; ++k) {
-            int iu, iv;
-            const bool ok = plane_index<ZX>(T, n1, make_float2(xf[k], xf[k]),
-                                            make_float2(yf[k], yf[k]),
-                                            make_float2(zf[k], zf[k]), iu, iv);
-            if ((AV || valid[k]) && ok)
-              part[k] = fmaf(SMEM ? src[iu * pa.nv + iv] : __ldg(src + iu * pa.nv + iv), T.w,
-                             part[k]);
-            need_bits |= (unsigned)((AV || valid[k]) && !ok) << ((oo - g0) * KP + k);
+          for (int b = 0; b < kPlBatch; ++b) {
+            // three 16-byte loads; each holds two (u, v) pairs
+            const float4 *q = reinterpret_cast<const float4 *>(s_ot + min(oo + b, ge - 1));
+            const float4 q0 = q[0], q1 = q[1], q2 = q[2];
+            PlaneOrient T;
+            T.x = make_float2(q0.x, q0.y);
+            T.y = make_float2(q0.z, q0.w);
+            T.z = make_float2(q1.x, q1.y);
+            T.c = make_float2(q1.z, q1.w);
+            T.d = make_float2(q2.x, q2.y);
+            w[b] = q2.z;
+  #pragma unroll
+            for (int k = 0; k < KP; ++k) {
+              int iu, iv;
+              const bool in = plane_index<ZX>(T, n1, make_float2(xf[k], xf[k]),
+                                              make_float2(yf[k], yf[k]),
+                                              make_float2(zf[k], zf[k]), iu, iv);
+              at[b][k] = iu * pa.nv + iv;
+              ok |= (unsigned)in << (b * KP + k);
+            }
           }
+  #pragma unroll
+          for (int b = 0; b < kPlBatch; ++b)
+  #pragma unroll
+            for (int k = 0; k < KP; ++k) v[b][k] = __ldg(pa.P + at[b][k]);
+          // (no samples of pixels outside the detector or past the group)
+          unsigned want = (1u << (min(kPlBatch, ge - oo) * KP)) - 1u;
+          if (!AV) want &= vmask;
+          need_bits |= (want & ~ok) << ((oo - g0) * KP);
+          ok &= want;
+  #pragma unroll
+          for (int b = 0; b < kPlBatch; ++b)
+  #pragma unroll
+            for (int k = 0; k < KP; ++k)
+              if (ok >> (b * KP + k) & 1u) part[k] = fmaf(v[b][k], w[b], part[k]);
         }
         // the group's uncertain samples go to the worklist (replayed exactly
         // by k_detector_fix), or, once it is full, are replayed here into the
         // float64 accumulator
         if (__any_sync(0xffffffffu, need_bits != 0)) {
-          while (need_bits) {
+          int slot = worklist_slots(need_bits, wl_count);
+          for (; need_bits; ++slot) {
             const int b = __ffs(need_bits) - 1;
             need_bits &= need_bits - 1;
             const int k = b % KP, o = c0 + g0 + b / KP;
@@ -344,7 +386,6 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
   #pragma unroll
             for (int q = 1; q < KP; ++q)
               if (k == q) px = pix[q];
-            const int slot = atomicAdd(wl_count, 1);
             if (slot < wl_cap) {
               wl[slot] = make_int2(px, o);
             } else {
@@ -364,8 +405,8 @@ k_detector_plane(DetArgs a, const PlaneOrient *ot, PlaneArgs pa,
       }
     }
   };
-  const int tile_i = (blockIdx.x / tiles_x) * kPlTH, tile_j = (blockIdx.x % tiles_x) * kPlTW;
-  if (tile_i + kPlTH <= a.nv && tile_j + kPlTW <= a.nh) orient_loop(BoolC<true>{});
+  const int tile_i = (blockIdx.x / tiles_x) * kPlTile, tile_j = (blockIdx.x % tiles_x) * kPlTile;
+  if (tile_i + kPlTile <= a.nv && tile_j + kPlTile <= a.nh) orient_loop(BoolC<true>{});
   else orient_loop(BoolC<false>{});
 #pragma unroll
   for (int k = 0; k < KP; ++k)
@@ -385,27 +426,26 @@ struct __align__(16) GenOrient {
 };
 static_assert(sizeof(GenOrient) == 96, "six 16-byte words per orientation");
 
-// Every orientation's samples of a 32 x 32 pixel tile, two pixels a thread,
-// gathered from the whole I(q).  The indices, certainty tests and order of
-// the sums are those of fast_index with each floor taken by one addition
-// rounded toward minus infinity (as in plane_index); an index is the 32-bit
-// sum of the rounded additions' bit patterns less a constant, which is exact
-// modulo 2^32 (I(q) has fewer than 2^32 elements).  Tiles keep a block's
-// samples of one orientation within a small patch of the volume.
-// 2880 orientations of 500 x 500 pixels in 203^3: 4.75 ms with one axis at a
-// time, rows of 512 pixels a block and 64-bit indices, 1.37 ms so.
+// Every orientation's samples of a pixel tile, two pixels a thread, gathered
+// from the whole I(q).  The indices, certainty tests and order of the sums are
+// those of fast_index with each floor taken by one addition rounded toward
+// minus infinity (as in plane_index); an index is the 32-bit sum of the rounded
+// additions' bit patterns less a constant, which is exact modulo 2^32 (I(q) has
+// fewer than 2^32 elements).  Tiles keep a block's samples of one orientation
+// within a small patch of the volume.  Bound by issue.  2880 orientations of
+// 500 x 500 pixels in 203^3: 4.75 ms with one axis at a time, rows of 512
+// pixels a block and 64-bit indices, 1.20 ms so.
 template <bool ZX, bool KAHAN>
 __global__ void __launch_bounds__(kPlThreads)
 k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, int *wl_count,
                    int wl_cap) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
   constexpr int KP = 2;
-  static_assert(kPlTH * kPlTW == KP * kPlThreads, "two pixels a thread");
   static_assert(kDetFlush * KP <= 32, "a group's uncertain samples fit one mask");
   __shared__ GenOrient s_ot[kDetChunk];
-  const int tiles_x = (a.nh + kPlTW - 1) / kPlTW;
-  const int j = (blockIdx.x % tiles_x) * kPlTW + (threadIdx.x % kPlTW);
-  const int ib = (blockIdx.x / tiles_x) * kPlTH + threadIdx.x / kPlTW;
+  const int tiles_x = (a.nh + kPlTile - 1) / kPlTile;
+  const int j = (blockIdx.x % tiles_x) * kPlTile + tile_col(threadIdx.x);
+  const int ib = (blockIdx.x / tiles_x) * kPlTile + tile_row(threadIdx.x);
   const float mx = (float)(a.nx - 1), my = (float)(a.ny - 1), mz = (float)(a.nz - 1);
   const unsigned nx = a.nx, nz = a.nz;
   const unsigned base = (0x4B400000u * nx + 0x4B400000u) * nz + 0x4B400000u;
@@ -415,7 +455,7 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
   double acc[KP];
 #pragma unroll
   for (int k = 0; k < KP; ++k) {
-    const int i = ib + k * (kPlThreads / kPlTW);
+    const int i = ib + k * kPlRows;
     valid[k] = i < a.nv && j < a.nh;
     pix[k] = valid[k] ? i * a.nh + j : 0;
     double x0 = 0.0, y0 = 0.0, z0 = 0.0;
@@ -424,6 +464,7 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
     acc[k] = 0.0;
     part[k] = kc[k] = 0.f;
   }
+  const unsigned vmask = (valid[0] ? 0x55555555u : 0u) | (valid[1] ? 0xaaaaaaaau : 0u);
   const float2 px = make_float2(xf[0], xf[1]), py = make_float2(yf[0], yf[1]),
                pz = make_float2(zf[0], zf[1]);
   const float2 mg = make_float2(kMagic, kMagic);
@@ -446,48 +487,66 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
     for (int g0 = 0; g0 < nc; g0 += kDetFlush) {
       const int ge = min(g0 + kDetFlush, nc);
       unsigned need = 0;  // bit (oo - g0) KP + k: an uncertain sample
-#pragma unroll 2
-      for (int oo = g0; oo < ge; ++oo) {
-        const float4 *q = reinterpret_cast<const float4 *>(s_ot + oo);
-        const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
-        const float w = s_ot[oo].w.x;
-        const float2 cx = make_float2(q0.x, q0.y), cy = make_float2(q0.z, q0.w),
-                     cz = make_float2(q1.x, q1.y), cc = make_float2(q1.z, q1.w),
-                     cd = make_float2(q2.x, q2.y);
-        // z axis of both pixels
-        float2 t = __ffma2_rn(make_float2(q3.x, q3.y), py,
-                              __ffma2_rn(make_float2(q3.z, q3.w), pz, make_float2(q4.x, q4.y)));
-        if (!ZX) t = __ffma2_rn(make_float2(q2.z, q2.w), px, t);
-        const float2 zd = make_float2(q4.z, q4.w);
-        const float2 zhi = __fadd2_rn(t, zd), zlo = f2_sub(t, zd);
-        const float2 zr = __fadd2_rd(
-            make_float2(fminf(fmaxf(zhi.x, 0.f), mz), fminf(fmaxf(zhi.y, 0.f), mz)), mg);
-        const float2 zfl = f2_sub(zr, mg);
+      for (int oo = g0; oo < ge; oo += kPlBatch) {
+        // every index is clamped, so the samples of kPlBatch orientations are
+        // loaded unconditionally, all in flight at once
+        unsigned at[kPlBatch][KP], ok = 0;
+        float w[kPlBatch], v[kPlBatch][KP];
 #pragma unroll
-        for (int k = 0; k < KP; ++k) {
-          const float2 yy = make_float2(yf[k], yf[k]), zz = make_float2(zf[k], zf[k]);
-          float2 u = __ffma2_rn(cy, yy, __ffma2_rn(cz, zz, cc));
-          if (!ZX) u = __ffma2_rn(cx, make_float2(xf[k], xf[k]), u);
-          const float2 hi = __fadd2_rn(u, cd), lo = f2_sub(u, cd);
-          const float2 r = __fadd2_rd(
-              make_float2(fminf(fmaxf(hi.x, 0.f), mx), fminf(fmaxf(hi.y, 0.f), my)), mg);
-          const float2 fl = f2_sub(r, mg);
-          const bool ok = (fmaxf(lo.x, 0.f) >= fl.x) & (fmaxf(lo.y, 0.f) >= fl.y) &
-                          (fmaxf(k ? zlo.y : zlo.x, 0.f) >= (k ? zfl.y : zfl.x));
-          const unsigned idx = (__float_as_uint(r.y) * nx + __float_as_uint(r.x)) * nz +
-                               __float_as_uint(k ? zr.y : zr.x) - base;
-          if (valid[k] && ok) add(k, __ldg(a.iq + idx), w);
-          need |= (unsigned)(valid[k] && !ok) << ((oo - g0) * KP + k);
+        for (int b = 0; b < kPlBatch; ++b) {
+          const float4 *q = reinterpret_cast<const float4 *>(s_ot + min(oo + b, ge - 1));
+          const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
+          w[b] = q[5].x;
+          const float2 cx = make_float2(q0.x, q0.y), cy = make_float2(q0.z, q0.w),
+                       cz = make_float2(q1.x, q1.y), cc = make_float2(q1.z, q1.w),
+                       cd = make_float2(q2.x, q2.y);
+          // z axis of both pixels
+          float2 t = __ffma2_rn(make_float2(q3.x, q3.y), py,
+                                __ffma2_rn(make_float2(q3.z, q3.w), pz, make_float2(q4.x, q4.y)));
+          if (!ZX) t = __ffma2_rn(make_float2(q2.z, q2.w), px, t);
+          const float2 zd = make_float2(q4.z, q4.w);
+          const float2 zhi = __fadd2_rn(t, zd), zlo = f2_sub(t, zd);
+          const float2 zr = __fadd2_rd(
+              make_float2(fminf(fmaxf(zhi.x, 0.f), mz), fminf(fmaxf(zhi.y, 0.f), mz)), mg);
+          const float2 zfl = f2_sub(zr, mg);
+#pragma unroll
+          for (int k = 0; k < KP; ++k) {
+            const float2 yy = make_float2(yf[k], yf[k]), zz = make_float2(zf[k], zf[k]);
+            float2 u = __ffma2_rn(cy, yy, __ffma2_rn(cz, zz, cc));
+            if (!ZX) u = __ffma2_rn(cx, make_float2(xf[k], xf[k]), u);
+            const float2 hi = __fadd2_rn(u, cd), lo = f2_sub(u, cd);
+            const float2 r = __fadd2_rd(
+                make_float2(fminf(fmaxf(hi.x, 0.f), mx), fminf(fmaxf(hi.y, 0.f), my)), mg);
+            const float2 fl = f2_sub(r, mg);
+            const bool in = (fmaxf(lo.x, 0.f) >= fl.x) & (fmaxf(lo.y, 0.f) >= fl.y) &
+                            (fmaxf(k ? zlo.y : zlo.x, 0.f) >= (k ? zfl.y : zfl.x));
+            at[b][k] = (__float_as_uint(r.y) * nx + __float_as_uint(r.x)) * nz +
+                       __float_as_uint(k ? zr.y : zr.x) - base;
+            ok |= (unsigned)in << (b * KP + k);
+          }
         }
+#pragma unroll
+        for (int b = 0; b < kPlBatch; ++b)
+#pragma unroll
+          for (int k = 0; k < KP; ++k) v[b][k] = __ldg(a.iq + at[b][k]);
+        // (no samples of pixels outside the detector or past the group)
+        const unsigned want = vmask & ((1u << (min(kPlBatch, ge - oo) * KP)) - 1u);
+        need |= (want & ~ok) << ((oo - g0) * KP);
+        ok &= want;
+#pragma unroll
+        for (int b = 0; b < kPlBatch; ++b)
+#pragma unroll
+          for (int k = 0; k < KP; ++k)
+            if (ok >> (b * KP + k) & 1u) add(k, v[b][k], w[b]);
       }
       // uncertain samples: to the worklist (k_detector_fix), or replayed
       // here once it is full
       if (__any_sync(0xffffffffu, need != 0)) {
-        while (need) {
+        int slot = worklist_slots(need, wl_count);
+        for (; need; ++slot) {
           const int b = __ffs(need) - 1;
           need &= need - 1;
           const int k = b % KP, o = c0 + g0 + b / KP, p = k ? pix[1] : pix[0];
-          const int slot = atomicAdd(wl_count, 1);
           if (slot < wl_cap) {
             wl[slot] = make_int2(p, o);
           } else {
@@ -934,6 +993,38 @@ extern "C" int gw_detector_set_iq32_device(gw_detector_plan *P, const float *iq3
   return GW_OK;
 }
 
+namespace {
+
+int tile_count(const gw_detector_plan *P) {
+  return ((P->p.n_h + kPlTile - 1) / kPlTile) * ((P->p.n_v + kPlTile - 1) / kPlTile);
+}
+
+void launch_plane(gw_detector_plan *P, const DetArgs &a) {
+  const PlaneArgs pa = P->plane;
+  const int tiles = tile_count(P);
+  auto run = [&](auto kernel) {
+    kernel<<<tiles, kPlThreads, 0, P->ctx->stream>>>(a, P->d_po, pa, P->d_acc, P->d_wl,
+                                                     P->d_wl_count, P->wl_cap);
+  };
+  P->zero_x ? run(k_detector_plane<true>) : run(k_detector_plane<false>);
+}
+
+void launch_general(gw_detector_plan *P, const DetArgs &a) {
+  const int tiles = tile_count(P);
+  auto run = [&](auto kernel) {
+    kernel<<<tiles, kPlThreads, 0, P->ctx->stream>>>(a, P->d_go, P->d_acc, P->d_wl,
+                                                     P->d_wl_count, P->wl_cap);
+  };
+  if (P->p.accum == GW_ACCUM_KAHAN32)
+    P->zero_x ? run(k_detector_general<true, true>)
+              : run(k_detector_general<false, true>);
+  else
+    P->zero_x ? run(k_detector_general<true, false>)
+              : run(k_detector_general<false, false>);
+}
+
+}  // namespace
+
 extern "C" int gw_detector_execute(gw_detector_plan *P) {
   if (!P) return gw::fail(GW_ERR_ARG, "gw_detector_execute: null plan");
   if (!P->iq && !P->plane_set)
@@ -967,43 +1058,17 @@ extern "C" int gw_detector_execute(gw_detector_plan *P) {
         }
         GW_LAUNCHED(P->ctx);
       }
-      const size_t smem = (size_t)pa.nu * pa.nv * sizeof(float);
-      const int tiles = ((P->p.n_h + kPlTW - 1) / kPlTW) * ((P->p.n_v + kPlTH - 1) / kPlTH);
       gw::KTimer tm(P->ctx, GW_K_DETECTOR);
-      if (smem <= kPlaneSmemMax) {
-        static gw::SmemRecord attr_zx, attr_gen;
-        GW_TRY(gw::smem_limit(attr_zx, k_detector_plane<true, true>, kPlaneSmemMax));
-        GW_TRY(gw::smem_limit(attr_gen, k_detector_plane<true, false>, kPlaneSmemMax));
-        if (P->zero_x)
-          k_detector_plane<true, true><<<tiles, kPlThreads, smem, P->ctx->stream>>>(
-              a, P->d_po, pa, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap);
-        else
-          k_detector_plane<true, false><<<tiles, kPlThreads, smem, P->ctx->stream>>>(
-              a, P->d_po, pa, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap);
-      } else if (P->zero_x) {
-        k_detector_plane<false, true><<<tiles, kPlThreads, 0, P->ctx->stream>>>(
-            a, P->d_po, pa, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap);
-      } else {
-        k_detector_plane<false, false><<<tiles, kPlThreads, 0, P->ctx->stream>>>(
-            a, P->d_po, pa, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap);
-      }
+      launch_plane(P, a);
       GW_LAUNCHED(P->ctx);
     } else {
       gw::KTimer tm(P->ctx, GW_K_DETECTOR);
-      const int tiles = ((P->p.n_h + kPlTW - 1) / kPlTW) * ((P->p.n_v + kPlTH - 1) / kPlTH);
-      const bool kh = P->p.accum == GW_ACCUM_KAHAN32;
       // the 32-bit gather index holds volumes of up to 2^32 elements; larger
       // ones replay every sample
       if ((double)a.nx * a.ny * a.nz >= 4294967296.0)
         k_detector<<<(npx + 127) / 128, 128, 0, P->ctx->stream>>>(a, P->d_acc);
-#define GW_GENERAL(ZX, KH)                                             \
-  k_detector_general<ZX, KH><<<tiles, kPlThreads, 0, P->ctx->stream>>>( \
-      a, P->d_go, P->d_acc, P->d_wl, P->d_wl_count, P->wl_cap)
-      else if (P->zero_x && kh) GW_GENERAL(true, true);
-      else if (P->zero_x) GW_GENERAL(true, false);
-      else if (kh) GW_GENERAL(false, true);
-      else GW_GENERAL(false, false);
-#undef GW_GENERAL
+      else
+        launch_general(P, a);
       GW_LAUNCHED(P->ctx);
     }
     gw::KTimer tm(P->ctx, GW_K_DET_FIX);
