@@ -493,7 +493,9 @@ def fft_passes(m):
 def shared_roof(name, info, spl, avg_ms):
     """Shared-memory traffic of a transform kernel's Stockham passes (one
     read and one write of every point per pass, forward and inverse) per
-    launch, against the nominal shared bandwidth."""
+    launch, against the nominal shared bandwidth.  (The last forward and the
+    first inverse pass share one trip in the kernels, so they move a read
+    and a write less than the passes counted here.)"""
     m = info["My"] if name == "row_czt" else info["Mz"]
     # real grids: two window rows per row transform, columns ky >= 0 only
     rows = info["Lz"] / 2 if info.get("real") else info["Lz"]
