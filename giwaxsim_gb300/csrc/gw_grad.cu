@@ -580,8 +580,12 @@ int grad_state_init(gw_voxel_plan *P) {
         (st = alloc(&G->d_G1, (size_t)P->S * P->Lz * P->Nc, &B)) ||
         (st = alloc(&G->d_sc, (size_t)P->n_slices * SC_N, &B)) ||
         (st = alloc(&G->d_amy, P->n_slices, &B)) ||
-        (st = alloc(&G->d_amz, P->n_struct, &B)))
+        (st = alloc(&G->d_amz, P->n_struct, &B))) {
+      // (a later call finds no half-made workspace)
+      grad_state_destroy(G);
+      P->grad = nullptr;
       return st;
+    }
   }
   if (G->n_atoms != P->n_atoms) {
     void *old[] = {G->d_gacc, G->d_gxyz, G->d_out_f, G->d_out_xyz};

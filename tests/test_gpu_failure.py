@@ -104,3 +104,37 @@ def test_tile_wait_timeout_reports_and_context_recovers():
     assert np.allclose(plan.iq(), ref, rtol=1e-12, atol=0)
     plan.close()
     ctx.close()
+
+
+def test_adjoint_workspace_failure_leaves_no_half_made_state():
+    """Every allocation of the adjoint's workspace fails once; each later
+    call starts again and the last one gives an untouched plan's gradients."""
+    ctx = N.Context(0)
+    xyz, _ = _case(2)
+    phis = np.array([0.0, 33.0, 90.0])
+    geom = F.VoxelGeometry(0.5, 0.15, 1.5)
+    g_iq = np.random.default_rng(5).standard_normal((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    got = []
+    for faults in (False, True):
+        plan = F.VoxelPlan(geom, [(xyz, np.full(len(xyz), 6.0 + 0j), None)], phis=phis,
+                           smooth=1.5, deposit="bilinear", real=False, ctx=ctx)
+        plan.set_atoms()
+        plan.execute()
+        failed = 0
+        while faults:
+            N.set_alloc_fault(failed)
+            try:
+                plan.backward(g_iq, want_xyz=True)
+                break
+            except N.GwError as e:
+                assert e.status == N.GW_ERR_OOM
+                failed += 1
+            finally:
+                N.set_alloc_fault(-1)
+        assert failed >= 10 * faults
+        got.append(plan.backward(g_iq, want_xyz=True))
+        plan.close()
+    for k in ("g_f", "g_xyz", "g_c"):
+        a, b = got[0][k], got[1][k]
+        assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(a)
+    ctx.close()
