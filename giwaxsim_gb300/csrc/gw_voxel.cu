@@ -1815,10 +1815,70 @@ int gather_setup(gw_voxel_plan *P) {
 
 }  // namespace
 
+namespace {
+
+// Slices per batch: the per-batch intermediates near L2 size.
+int batch_size(const gw_voxel_plan *P) {
+  const size_t per = (size_t)P->Lz * P->Nf * sizeof(float2) + (P->Ly + P->Lz) * 12;
+  const int S = P->plain ? 1
+                : P->p.batch_slices > 0 ? P->p.batch_slices
+                                        : (int)std::max<size_t>(1, (96u << 20) / per);
+  return std::min(std::min(S, P->n_slices), 4096);  // grid.y limit margin
+}
+
+// What a plan holds for the path it runs (real or general grids), as leave_real
+// exchanges it.
+struct PathParts {
+  bool real, gather, f1_tma;
+  int Nf, S, f1_box_cols, n_heavy, n_zmulti;
+  size_t bytes, path_bytes;
+  CUtensorMap f1map;
+  float2 *F1, *pr;
+  float *G;
+  int *lptr, *zptr, *zrows, *heavy, *zmulti;
+  int2 *lent;
+  std::vector<int> h_heavy;
+
+  explicit PathParts(const gw_voxel_plan *P)
+      : real(P->real), gather(P->gather), f1_tma(P->f1_tma), Nf(P->Nf), S(P->S),
+        f1_box_cols(P->f1_box_cols), n_heavy(P->n_heavy), n_zmulti(P->n_zmulti),
+        bytes(P->bytes), path_bytes(P->path_bytes), f1map(P->f1map), F1(P->d_F1),
+        pr(P->d_pr), G(P->d_G), lptr(P->d_lptr), zptr(P->d_zptr), zrows(P->d_zrows),
+        heavy(P->d_heavy), zmulti(P->d_zmulti), lent(P->d_lent), h_heavy(P->h_heavy) {}
+  void restore(gw_voxel_plan *P) const {
+    P->real = real; P->gather = gather; P->f1_tma = f1_tma;
+    P->Nf = Nf; P->S = S; P->f1_box_cols = f1_box_cols;
+    P->n_heavy = n_heavy; P->n_zmulti = n_zmulti;
+    P->bytes = bytes; P->path_bytes = path_bytes; P->f1map = f1map;
+    P->d_F1 = F1; P->d_pr = pr; P->d_G = G; P->d_lptr = lptr; P->d_zptr = zptr;
+    P->d_zrows = zrows; P->d_heavy = heavy; P->d_zmulti = zmulti; P->d_lent = lent;
+    P->h_heavy = h_heavy;
+  }
+  void free() const {
+    void *ptrs[] = {F1, pr, G, lptr, zptr, zrows, heavy, zmulti, lent};
+    for (void *q : ptrs) gw::dev_free(q);
+  }
+};
+
+// F1 and, on real grids, the row kernel's table, the tensor map, then the
+// gather's tables (the column and row tables are made).
+int path_buffers(gw_voxel_plan *P) {
+  const size_t before = P->bytes;
+  GW_TRY(alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &P->bytes));
+  if (P->real) GW_TRY(alloc(&P->d_pr, (size_t)P->n_slices * P->Ly, &P->bytes));
+  GW_TRY(col_map_dispatch(P));
+  GW_TRY(gather_setup(P));
+  P->path_bytes = P->bytes - before;
+  return GW_OK;
+}
+
+}  // namespace
+
 // Per-shell f values and the adjoint need the general path: a plan made with
 // real_grids refuses them where its window is at most half the transform
 // buffer.  A wider window takes them (such plans run them on the general
-// path): the plan leaves the real path for good.
+// path): the plan leaves the real path for good.  The general path's buffers
+// are made beside the present ones; where that fails, the plan is as it was.
 int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   if (!P->real) return GW_OK;
   if (2 * P->Ly <= fft_ldm(P->My))
@@ -1832,11 +1892,8 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
     for (int t = 0; t < P->n_out; ++t) GW_TRY(enqueue_gather(P, 2, t));
   }
   GW_CUDA(cudaStreamSynchronize(P->ctx->stream));  // no pass reads the buffers
-  if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
-  if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
-  void *drop[] = {P->d_F1, P->d_pr, P->d_heavy, P->d_zmulti, P->d_lptr, P->d_lent,
-                  P->d_zptr, P->d_zrows, P->d_G};
-  for (void *q : drop) gw::dev_free(q);
+  const PathParts now(P);
+  P->bytes -= P->path_bytes;
   P->d_F1 = nullptr;
   P->d_pr = nullptr;
   P->d_heavy = P->d_zmulti = P->d_lptr = P->d_zptr = P->d_zrows = nullptr;
@@ -1844,11 +1901,22 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   P->d_G = nullptr;
   P->gather = false;
   P->n_heavy = P->n_zmulti = 0;
+  P->h_heavy.clear();
   P->real = false;
   P->Nf = P->Nc;
-  GW_TRY(alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &P->bytes));
-  GW_TRY(col_map_dispatch(P));
-  return gather_setup(P);
+  P->S = batch_size(P);
+  int st = path_buffers(P);
+  if (st == GW_OK && cudaStreamSynchronize(P->ctx->stream) != cudaSuccess) st = GW_ERR_CUDA;
+  if (st != GW_OK) {
+    PathParts(P).free();
+    now.restore(P);
+    cudaGetLastError();  // (reported; not the next launch's)
+    return st;
+  }
+  if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
+  if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
+  now.free();
+  return GW_OK;
 }
 
 extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
@@ -2050,15 +2118,7 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
   P->real = want_real && P->My <= 2048 &&
             p->transform_y != GW_TRANSFORM_FUSED && p->transform_z != GW_TRANSFORM_FUSED;
   P->Nf = P->real ? P->Nc - P->m_zero : P->Nc;
-  // batch size: keep the per-batch intermediates near L2 size
-  {
-    const size_t per = (size_t)P->Lz * P->Nf * sizeof(float2) +
-                       (P->Ly + P->Lz) * 12;
-    int S = p->batch_slices > 0 ? p->batch_slices
-                                : (int)std::max<size_t>(1, (96u << 20) / per);
-    if (P->plain) S = 1;
-    P->S = std::min(std::min(S, P->n_slices), 4096);  // grid.y limit margin
-  }
+  P->S = batch_size(P);
 
   int st = GW_OK;
   size_t &B = P->bytes;
@@ -2158,12 +2218,9 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_cursor, (size_t)n_struct * (g + 1), &B)) ||
       (st = alloc(&P->d_zstat, n_struct, &B)) ||
       (st = alloc(&P->d_amo, (size_t)P->n_slices * P->Ly, &B)) ||
-      (P->real && (st = alloc(&P->d_pr, (size_t)P->n_slices * P->Ly, &B))) ||
       (st = alloc(&P->d_my, (size_t)P->n_slices * P->Ly, &B)) ||
       (st = alloc(&P->d_mz, (size_t)P->n_slices * P->Lz, &B)) ||
-      (st = upload(&P->d_roff, P->roff_host, &B)) ||
-      (st = alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &B)) ||
-      (st = col_map_dispatch(P))) {
+      (st = upload(&P->d_roff, P->roff_host, &B))) {
     gw_voxel_plan_destroy(P);
     return st;
   }
@@ -2185,7 +2242,7 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       return gw::cuda_fail(e, "column tables", __FILE__, __LINE__);
     }
   }
-  if ((st = gather_setup(P))) {
+  if ((st = path_buffers(P))) {
     gw_voxel_plan_destroy(P);
     return st;
   }

@@ -591,6 +591,7 @@ struct gw_voxel_plan {
   gw_structure *d_structs_shells = nullptr;  // [n_shells][n_struct]
   int64_t n_atoms = -1;
   size_t bytes = 0;
+  size_t path_bytes = 0;  // of them, what leave_real replaces (PathParts)
   std::vector<int> C1host;
   std::vector<int> h_rowofs;  // the output rows' window z (host copy)
   // device

@@ -5,6 +5,7 @@ that narrower real-grid plans refuse: per-shell f values and the adjoint."""
 import numpy as np
 import pytest
 
+from giwaxsim_gb300 import _native as N
 from giwaxsim_gb300 import forward as F
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +87,47 @@ def test_wide_plan_takes_the_adjoint_and_shells(binning, what):
             plan.close()
     for a, b in zip(got[None], got[False]):
         assert rel_l2(a, b) <= RTOL
+
+
+@pytest.mark.parametrize("binning", ["atomic", "gather"])
+def test_failed_change_of_path_leaves_the_plan(binning):
+    """Every allocation on the way to the general path fails once: the plan
+    still runs the real path (and its graph) with the same result."""
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    g_iq = np.random.default_rng(4).standard_normal((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS, binning=binning)
+    try:
+        plan.set_atoms()
+        plan.capture_graph()
+        plan.execute()
+        before, ref = plan.info(), plan.iq().copy()
+        assert before["real"] == 1
+        failed = 0
+        while True:
+            N.set_alloc_fault(failed)
+            try:
+                plan.backward(g_iq)
+            except N.GwError as e:
+                assert e.status == N.GW_ERR_OOM
+            finally:
+                N.set_alloc_fault(-1)
+            if not plan.info()["real"]:
+                break
+            assert plan.info() == before
+            failed += 1
+            plan.execute()
+            assert rel_l2(plan.iq(), ref) <= RTOL
+        assert failed == (1 if binning == "atomic" else 10)
+        after = plan.info()
+        if binning == "atomic":  # F1 in and out, the row table out
+            a, b = before, after
+            nf = a["Nc"] + a["k0"]  # columns ky >= 0
+            assert b["device_bytes"] - a["device_bytes"] == 8 * (
+                b["batch"] * b["Lz"] * b["Nc"] - a["batch"] * a["Lz"] * nf
+                - a["n_slices"] * a["Ly"])
+        plan.execute()
+        assert rel_l2(plan.iq(), ref) <= RTOL
+    finally:
+        plan.close()
