@@ -618,7 +618,7 @@ extern "C" int gw_voxel_grad_buffer(gw_voxel_plan *P, double **g_iq_dev) {
 extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
                                  int32_t iq_on_device, double *g_f,
                                  double *g_xyz, double *g_sigma, double *g_c) {
-  if (P) GW_TRY(gwv::leave_real(P, "gw_voxel_backward"));
+  if (P) GW_TRY(gwv::may_leave_real(P, "gw_voxel_backward"));
   if (!P || !g_iq || !g_f)
     return gw::fail(GW_ERR_ARG, "gw_voxel_backward: null argument");
   if (P->plain)
@@ -633,6 +633,7 @@ extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
     return gw::fail(GW_ERR_ARG, "gw_voxel_backward: coordinate gradients need the bilinear deposit");
   if (P->n_atoms < 0)
     return gw::fail(GW_ERR_STATE, "gw_voxel_backward: atoms not set");
+  GW_TRY(gwv::leave_real(P));
   GW_CUDA(cudaSetDevice(P->ctx->device));
   GW_TRY(grad_state_init(P));
   gw_grad_state *G = P->grad;

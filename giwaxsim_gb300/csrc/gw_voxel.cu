@@ -1877,13 +1877,18 @@ int path_buffers(gw_voxel_plan *P) {
 // Per-shell f values and the adjoint need the general path: a plan made with
 // real_grids refuses them where its window is at most half the transform
 // buffer.  A wider window takes them (such plans run them on the general
-// path): the plan leaves the real path for good.  The general path's buffers
-// are made beside the present ones; where that fails, the plan is as it was.
-int gwv::leave_real(gw_voxel_plan *P, const char *who) {
-  if (!P->real) return GW_OK;
-  if (2 * P->Ly <= fft_ldm(P->My))
+// path): the plan leaves the real path for good, once the call's arguments and
+// the plan's state are found to allow it.  The general path's buffers are made
+// beside the present ones; where that fails, the plan is as it was.
+int gwv::may_leave_real(const gw_voxel_plan *P, const char *who) {
+  if (P->real && 2 * P->Ly <= fft_ldm(P->My))
     return gw::fail(GW_ERR_STATE, std::string(who) + ": the plan was made with real_grids; "
                                   "per-shell f values and the adjoint need real_grids 0");
+  return GW_OK;
+}
+
+int gwv::leave_real(gw_voxel_plan *P) {
+  if (!P->real) return GW_OK;
   GW_CUDA(cudaSetDevice(P->ctx->device));
   if (P->executed && gathering(P)) {
     // the last execute's results that are made on request, from its pixels
@@ -1915,6 +1920,7 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   }
   if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
   if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
+  P->graph_kernels = 0;
   now.free();
   return GW_OK;
 }
@@ -2314,7 +2320,7 @@ extern "C" int gw_voxel_set_shells(gw_voxel_plan *P, int32_t n_shells,
                                    const double *lower, const double *upper,
                                    const float *f, const double *avg_f) {
   if (!P) return gw::fail(GW_ERR_ARG, "gw_voxel_set_shells: null plan");
-  GW_TRY(gwv::leave_real(P, "gw_voxel_set_shells"));
+  GW_TRY(gwv::may_leave_real(P, "gw_voxel_set_shells"));
   auto drop = [P]() {
     gw::dev_free(P->d_shell); gw::dev_free(P->d_f_shells);
     gw::dev_free(P->d_structs_shells);
@@ -2345,6 +2351,7 @@ extern "C" int gw_voxel_set_shells(gw_voxel_plan *P, int32_t n_shells,
     if (k + 2 < n_shells && !(lower[k + 2] >= upper[k]))
       return gw::fail(GW_ERR_ARG, "gw_voxel_set_shells: a shell overlaps the one after next");
   }
+  GW_TRY(gwv::leave_real(P));
   drop();
   const int K = n_shells;
   const size_t W3 = (size_t)P->W * P->W * P->W;

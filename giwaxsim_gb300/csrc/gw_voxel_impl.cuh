@@ -716,9 +716,11 @@ int fused_col_block(const gw_voxel_plan *P);
 // I(q) grids.
 int enqueue_finalize(gw_voxel_plan *P, bool f64);
 int enqueue_gather(gw_voxel_plan *P, int mode, int t, int line_lo = 0, int line_hi = -1);
-// Takes a real-grid plan with a wide window to the general path; refuses
-// (GW_ERR_STATE) for other real-grid plans.
-int leave_real(gw_voxel_plan *P, const char *who);
+// Refuses (GW_ERR_STATE) the calls that need the general path on a real-grid
+// plan, unless its window is wide.
+int may_leave_real(const gw_voxel_plan *P, const char *who);
+// Takes a real-grid plan to the general path.
+int leave_real(gw_voxel_plan *P);
 // Number of window rows of slices [s0, s0+n).
 int batch_rows(gw_voxel_plan *P, int s0, int n);
 void grad_state_destroy(gw_grad_state *g);

@@ -131,3 +131,44 @@ def test_failed_change_of_path_leaves_the_plan(binning):
         assert rel_l2(plan.iq(), ref) <= RTOL
     finally:
         plan.close()
+
+
+def test_refused_calls_leave_the_plan():
+    """A backward or set_shells that is refused, and a clear of the shells,
+    keep a wide plan on the real path; a refusal keeps its graph too."""
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    g_iq = np.ones((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    for kw in (dict(average="separate"), dict(fill_bkg=True)):
+        plan = F.VoxelPlan(geom, [(xyz, fv, None), (xyz + 1.0, fv, None)], phis=PHIS, **kw)
+        try:
+            plan.set_atoms()
+            plan.capture_graph()
+            before = plan.info()
+            assert before["real"] == 1 and before["graph_kernels"] > 0
+            with pytest.raises(N.GwError) as e:
+                plan.backward(g_iq)
+            assert e.value.status == N.GW_ERR_ARG
+            with pytest.raises(N.GwError) as e:
+                plan.backward(g_iq, want_xyz=True)
+            assert e.value.status == N.GW_ERR_ARG
+            for lower, upper in (([1.0], [0.5]), ([0.0, 0.1], [0.5, 0.4])):
+                with pytest.raises(N.GwError) as e:
+                    plan.set_shells(geom.q, np.array(lower), np.array(upper),
+                                    np.ones((len(lower), 2 * len(xyz))), np.ones((len(lower), 2)))
+                assert e.value.status == N.GW_ERR_ARG
+            assert plan.info() == before
+            plan.execute()
+            plan.set_shells(None, None, None, None, None)
+            assert plan.info()["real"] == 1
+        finally:
+            plan.close()
+    # no atoms yet
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS)
+    try:
+        with pytest.raises(N.GwError) as e:
+            plan.backward(g_iq)
+        assert e.value.status == N.GW_ERR_STATE and plan.info()["real"] == 1
+    finally:
+        plan.close()
