@@ -633,7 +633,7 @@ extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
     return gw::fail(GW_ERR_ARG, "gw_voxel_backward: coordinate gradients need the bilinear deposit");
   if (P->n_atoms < 0)
     return gw::fail(GW_ERR_STATE, "gw_voxel_backward: atoms not set");
-  GW_TRY(gwv::leave_real(P));
+  GW_TRY(gwv::leave_real(P, "gw_voxel_backward"));
   GW_CUDA(cudaSetDevice(P->ctx->device));
   GW_TRY(grad_state_init(P));
   gw_grad_state *G = P->grad;

@@ -1762,7 +1762,7 @@ int gather_lines(gw_voxel_plan *P) {
 // Gather binning: where it applies and the pixel store fits the budget
 // (GW_GATHER_MAX_MB, default 8192), its tables and store.  The column and
 // row tables of the plan are made.
-int gather_setup(gw_voxel_plan *P) {
+int gather_setup(gw_voxel_plan *P, const char *who) {
   size_t &B = P->bytes;
   const size_t g_bytes = (size_t)P->n_slices * P->Nf * P->Nr * sizeof(float);
   const char *env = getenv("GW_GATHER_MAX_MB");
@@ -1771,7 +1771,7 @@ int gather_setup(gw_voxel_plan *P) {
   const bool can = !P->plain && P->p.accum == GW_ACCUM_FP64 && !P->fused_z &&
                    g_bytes <= cap && g_bytes / sizeof(float) < ((size_t)1 << 31);
   if (P->p.binning == GW_BINNING_GATHER && !can) {
-    return gw::fail(GW_ERR_ARG, "gw_voxel_plan_create: gather binning needs a batched, "
+    return gw::fail(GW_ERR_ARG, std::string(who) + ": gather binning needs a batched, "
                                 "float64-accumulating plan without the fused column "
                                 "kernel, and a pixel store within GW_GATHER_MAX_MB");
   }
@@ -1862,12 +1862,12 @@ struct PathParts {
 
 // F1 and, on real grids, the row kernel's table, the tensor map, then the
 // gather's tables (the column and row tables are made).
-int path_buffers(gw_voxel_plan *P) {
+int path_buffers(gw_voxel_plan *P, const char *who) {
   const size_t before = P->bytes;
   GW_TRY(alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &P->bytes));
   if (P->real) GW_TRY(alloc(&P->d_pr, (size_t)P->n_slices * P->Ly, &P->bytes));
   GW_TRY(col_map_dispatch(P));
-  GW_TRY(gather_setup(P));
+  GW_TRY(gather_setup(P, who));
   P->path_bytes = P->bytes - before;
   return GW_OK;
 }
@@ -1879,7 +1879,9 @@ int path_buffers(gw_voxel_plan *P) {
 // buffer.  A wider window takes them (such plans run them on the general
 // path): the plan leaves the real path for good, once the call's arguments and
 // the plan's state are found to allow it.  The general path's buffers are made
-// beside the present ones; where that fails, the plan is as it was.
+// beside the present ones; where that fails (gather binning asked for by name,
+// its store of twice the columns beyond GW_GATHER_MAX_MB: GW_ERR_ARG), the plan
+// is as it was.
 int gwv::may_leave_real(const gw_voxel_plan *P, const char *who) {
   if (P->real && 2 * P->Ly <= fft_ldm(P->My))
     return gw::fail(GW_ERR_STATE, std::string(who) + ": the plan was made with real_grids; "
@@ -1887,7 +1889,7 @@ int gwv::may_leave_real(const gw_voxel_plan *P, const char *who) {
   return GW_OK;
 }
 
-int gwv::leave_real(gw_voxel_plan *P) {
+int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   if (!P->real) return GW_OK;
   GW_CUDA(cudaSetDevice(P->ctx->device));
   if (P->executed && gathering(P)) {
@@ -1910,7 +1912,7 @@ int gwv::leave_real(gw_voxel_plan *P) {
   P->real = false;
   P->Nf = P->Nc;
   P->S = batch_size(P);
-  int st = path_buffers(P);
+  int st = path_buffers(P, who);
   if (st == GW_OK && cudaStreamSynchronize(P->ctx->stream) != cudaSuccess) st = GW_ERR_CUDA;
   if (st != GW_OK) {
     PathParts(P).free();
@@ -2248,7 +2250,7 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       return gw::cuda_fail(e, "column tables", __FILE__, __LINE__);
     }
   }
-  if ((st = path_buffers(P))) {
+  if ((st = path_buffers(P, "gw_voxel_plan_create"))) {
     gw_voxel_plan_destroy(P);
     return st;
   }
@@ -2351,7 +2353,7 @@ extern "C" int gw_voxel_set_shells(gw_voxel_plan *P, int32_t n_shells,
     if (k + 2 < n_shells && !(lower[k + 2] >= upper[k]))
       return gw::fail(GW_ERR_ARG, "gw_voxel_set_shells: a shell overlaps the one after next");
   }
-  GW_TRY(gwv::leave_real(P));
+  GW_TRY(gwv::leave_real(P, "gw_voxel_set_shells"));
   drop();
   const int K = n_shells;
   const size_t W3 = (size_t)P->W * P->W * P->W;

@@ -720,7 +720,7 @@ int enqueue_gather(gw_voxel_plan *P, int mode, int t, int line_lo = 0, int line_
 // plan, unless its window is wide.
 int may_leave_real(const gw_voxel_plan *P, const char *who);
 // Takes a real-grid plan to the general path.
-int leave_real(gw_voxel_plan *P);
+int leave_real(gw_voxel_plan *P, const char *who);
 // Number of window rows of slices [s0, s0+n).
 int batch_rows(gw_voxel_plan *P, int s0, int n);
 void grad_state_destroy(gw_grad_state *g);

@@ -172,3 +172,36 @@ def test_refused_calls_leave_the_plan():
         assert e.value.status == N.GW_ERR_STATE and plan.info()["real"] == 1
     finally:
         plan.close()
+
+
+def test_gather_store_too_large_for_the_general_path(monkeypatch):
+    """Gather binning asked for, with a pixel store that fits the limit with
+    the columns ky >= 0 and not with all of them: a call that needs the
+    general path is refused, again when it is repeated, and changes nothing."""
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    g_iq = np.ones((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    probe = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS, binning="atomic")
+    i = probe.info()
+    probe.close()
+    per = (i["Nc"] + i["k0"]) * i["Nr"] * 4  # bytes a slice, columns ky >= 0
+    phis = np.linspace(0.0, 179.0, int(0.9 * 2 ** 20 / per))
+    assert len(phis) * i["Nc"] * i["Nr"] * 4 > 2 ** 20
+    monkeypatch.setenv("GW_GATHER_MAX_MB", "1")
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=phis, binning="gather")
+    try:
+        plan.set_atoms()
+        plan.execute()
+        before, ref = plan.info(), plan.iq().copy()
+        assert before["real"] == 1 and before["gather"] == 1
+        for _ in range(2):
+            with pytest.raises(N.GwError) as e:
+                plan.backward(g_iq)
+            assert e.value.status == N.GW_ERR_ARG
+            assert "gw_voxel_backward" in str(e.value) and "GW_GATHER_MAX_MB" in str(e.value)
+            assert plan.info() == before
+            plan.execute()
+            assert rel_l2(plan.iq(), ref) <= RTOL
+    finally:
+        plan.close()
