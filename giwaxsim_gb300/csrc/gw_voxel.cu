@@ -1923,6 +1923,7 @@ int gwv::leave_real(gw_voxel_plan *P, const char *who) {
   if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
   if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
   P->graph_kernels = 0;
+  P->store_filled = false;  // (its sums were made above)
   now.free();
   return GW_OK;
 }
@@ -2430,6 +2431,7 @@ extern "C" int gw_voxel_execute(gw_voxel_plan *P) {
     GW_TRY(voxel_enqueue_all(P));
   }
   P->executed = true;
+  P->store_filled = gathering(P);
   P->iq64_valid = false;
   return GW_OK;
 }
@@ -2582,7 +2584,7 @@ extern "C" int gw_voxel_get_sums(gw_voxel_plan *P, double *sums) {
     for (size_t i = 0; i < W3; ++i) s[i] = (double)k[i].x - (double)k[i].y;
   } else {
     // gather binning keeps no sum grid: made from the stored pixels here
-    if (gwv::gathering(P)) GW_TRY(gwv::enqueue_gather(P, 2, 0));
+    if (P->store_filled) GW_TRY(gwv::enqueue_gather(P, 2, 0));
     GW_CUDA(cudaMemcpyAsync(s.data(), P->d_sum, W3 * sizeof(double),
                             cudaMemcpyDeviceToHost, P->ctx->stream));
     GW_TRY(gw::check_device_error(P->ctx, "voxel stage"));

@@ -670,6 +670,7 @@ struct gw_voxel_plan {
   cudaGraphExec_t gexec = nullptr;
   int64_t graph_kernels = 0;
   bool executed = false;
+  bool store_filled = false;  // d_G holds the last execute's pixels
   // d_iq64 holds the last execute's float64 I(q) (made on request)
   bool iq64_valid = false;
   gw_grad_state *grad = nullptr;  // adjoint workspace (gw_grad.cu)

@@ -205,3 +205,26 @@ def test_gather_store_too_large_for_the_general_path(monkeypatch):
             assert rel_l2(plan.iq(), ref) <= RTOL
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("binning", ["atomic", "gather"])
+def test_sums_of_the_last_execute_after_the_change_of_path(binning):
+    """sums() and iq() asked for after a backward are those of the execute
+    before it, not of the general path's empty pixel store."""
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    g_iq = np.ones((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS, binning=binning)
+    try:
+        plan.set_atoms()
+        plan.execute()
+        ref = plan.sums(), plan.iq().copy()
+        plan.execute()  # (nothing made on request yet)
+        plan.backward(g_iq)
+        assert plan.info()["real"] == 0
+        for _ in range(2):
+            assert rel_l2(plan.sums(), ref[0]) <= RTOL and rel_l2(plan.iq(), ref[1]) <= RTOL
+            plan.execute()
+    finally:
+        plan.close()
