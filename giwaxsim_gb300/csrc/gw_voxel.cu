@@ -1417,6 +1417,7 @@ int enqueue_prep(gw_voxel_plan *P) {
   cudaStream_t st = ctx->stream;
   const Scatter sc{P->d_xyz, P->d_f, P->d_zidx, P->g, P->real ? 1 : 0, P->inv_r, P->d_cursor,
                    P->d_xyz_s, P->d_xyf_s, P->d_perm, P->d_fz_s, P->d_cand};
+  P->sorted_real = P->real;
   int64_t max_atoms = 0;
   for (auto &s : P->structs) max_atoms = std::max(max_atoms, s.atom_count);
   if (max_atoms <= kPrepSmall) {
@@ -2657,6 +2658,7 @@ extern "C" int gw_voxel_debug_window(gw_voxel_plan *P, int32_t slice,
   GW_CUDA(gw::dev_malloc((void **)&d, n * sizeof(float2)));
   cudaError_t e = cudaMemsetAsync(d, 0, n * sizeof(float2), P->ctx->stream);
   SliceArgs a = slice_args(P);
+  a.real = P->sorted_real;  // (the plan may have left the real path since)
   if (e == cudaSuccess) {
     k_debug_window<<<256, 128, 0, P->ctx->stream>>>(a, slice, d);
     P->ctx->launches++;

@@ -655,6 +655,7 @@ struct gw_voxel_plan {
   float4 *d_xyf_s = nullptr;
   float *d_fz_s = nullptr;
   int *d_perm = nullptr;   // sorted position -> input atom index
+  bool sorted_real = false;    // d_xyf_s was made for real grids
   int *d_cand = nullptr;       // candidates for the y extremes (sorted positions)
   int *d_ncand = nullptr, *d_any_ext = nullptr;
   unsigned long long *d_dirs = nullptr;  // per structure: outermost atoms

@@ -228,3 +228,26 @@ def test_sums_of_the_last_execute_after_the_change_of_path(binning):
             plan.execute()
     finally:
         plan.close()
+
+
+def test_window_of_the_last_execute_after_the_change_of_path():
+    """debug_window shows the last execute's deposit, before and after
+    set_shells takes the plan to the general path."""
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    fv = fv * (3.0 - 4.0j)
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS)
+    try:
+        plan.set_atoms()
+        plan.execute()
+        assert plan.info()["real"] == 1
+        ref = plan.debug_window(1)[0].copy()
+        assert abs(ref.sum() - fv.sum()) <= RTOL * np.abs(fv).sum()
+        plan.set_shells(geom.q, np.array([0.0]), np.array([2.0]), fv[None, :], np.ones((1, 1)))
+        assert plan.info()["real"] == 0
+        assert rel_l2(plan.debug_window(1)[0], ref) <= RTOL
+        plan.execute()
+        assert rel_l2(plan.debug_window(1)[0], ref) <= RTOL
+    finally:
+        plan.close()
