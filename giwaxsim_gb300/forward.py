@@ -572,9 +572,12 @@ class VoxelPlan:
             if g_iq.shape != (self.Qc,) * 3:
                 raise ValueError("g_iq must have shape %s" % ((self.Qc,) * 3,))
             src, flag = N.ptr(g_iq), 0
-        N.check(N.lib().gw_voxel_backward(self.handle, src, flag, N.ptr(g_f),
-                                          N.ptr(g_xyz), N.ptr(g_sigma),
-                                          N.ptr(g_c)))
+        st = N.lib().gw_voxel_backward(self.handle, src, flag, N.ptr(g_f),
+                                       N.ptr(g_xyz), N.ptr(g_sigma), N.ptr(g_c))
+        # a real-grid plan that left the real path for this has no graph now
+        if self.graph_captured and self.params.real_grids:
+            self.graph_captured = self.info()["graph_kernels"] > 0
+        N.check(st)
         return dict(g_f=g_f.view(complex), g_xyz=g_xyz, g_sigma=float(g_sigma[0]),
                     g_c=g_c.view(complex))
 

@@ -251,3 +251,24 @@ def test_window_of_the_last_execute_after_the_change_of_path():
         assert rel_l2(plan.debug_window(1)[0], ref) <= RTOL
     finally:
         plan.close()
+
+
+def test_graph_captured_follows_the_change_of_path():
+    axes, box, m = CASES[1]
+    geom = F.VoxelGeometry(*axes)
+    xyz, fv = atoms(box, 3)
+    g_iq = np.ones((geom.crop_hi - geom.crop_lo + 1,) * 3)
+    plan = F.VoxelPlan(geom, [(xyz, fv, None)], phis=PHIS)
+    try:
+        plan.set_atoms()
+        plan.capture_graph()
+        with pytest.raises(N.GwError):
+            plan.backward(g_iq, want_xyz=True)  # refused
+        assert plan.graph_captured
+        plan.backward(g_iq)
+        assert not plan.graph_captured
+        plan.capture_graph()
+        plan.backward(g_iq)  # on the general path already
+        assert plan.graph_captured and plan.info()["graph_kernels"] > 0
+    finally:
+        plan.close()
