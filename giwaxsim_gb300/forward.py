@@ -176,6 +176,14 @@ def real_multiples(fv):
     return bool(abs(np.sum(f)) > 1e-3 * np.sum(np.abs(f)))
 
 
+def real_along(fv, avg):
+    """True when every f value is a real multiple of avg's phase (to the
+    float32 precision the device keeps them in)."""
+    f = np.asarray(fv, dtype=complex).ravel()
+    cross = f.imag * avg.real - f.real * avg.imag  # Im(f conj(avg))
+    return bool(np.max(np.abs(cross)) <= 1e-6 * abs(avg) * np.max(np.abs(f)))
+
+
 def coord_ranges(coords):
     """max - min of x, y and z (comparison.py:712-717), from a transposed
     copy (contiguous reductions)."""
@@ -277,7 +285,9 @@ class VoxelPlan:
     are real multiples of one complex value in a batched, nearest-bin plan
     without a fused kernel asked for; False keeps the general path (needed
     for set_shells and backward); True asks for it and refuses f values
-    that do not allow it.  binning: "auto" (gather where it applies),
+    that do not allow it.  constants (x_bound, y_bound, z_bound, average
+    voxel f per structure, in place of the computed ones) whose average has
+    another phase than the f values keep the general path.  binning: "auto" (gather where it applies),
     "atomic" or "gather" (gw_voxel_params.binning)."""
 
     def __init__(self, geom, structures, phis=None, fill_bkg=False, smooth=0,
@@ -315,7 +325,7 @@ class VoxelPlan:
         r = geom.r_voxel_size
         st = np.zeros(len(structures), dtype=_dtype_of(N.Structure))
         xyz, fs = [], []
-        all_real = True
+        all_real = along = True
         begin = 0
         for i, (coords, fv, w) in enumerate(structures):
             coords = np.ascontiguousarray(coords, dtype=np.float64)
@@ -337,6 +347,8 @@ class VoxelPlan:
                 xb, yb, zb, avg, mv = structure_constants(coords, fv, r, rg)
             # real grids take the phase of avg (a finite, nonzero value)
             all_real = all_real and bool(np.isfinite(avg) and avg != 0)
+            if constants is not None and all_real:
+                along = along and real_along(fv, avg)
             st[i] = (begin, len(coords), xb, yb, zb, avg.real, avg.imag, mv)
             begin += len(coords)
             xyz.append(coords)
@@ -386,7 +398,9 @@ class VoxelPlan:
             raise ValueError("real=True needs every structure's f values to be "
                              "real multiples of one complex value, with a finite, "
                              "nonzero average voxel f")
-        p.real_grids = int(bool(real))
+        # the real path takes the phase of the average voxel f: a caller's
+        # constants of another phase keep the general path
+        p.real_grids = int(bool(real) and along)
         p.binning = {"auto": N.GW_BINNING_AUTO, "atomic": N.GW_BINNING_ATOMIC,
                      "gather": N.GW_BINNING_GATHER}[binning]
         self.params = p
