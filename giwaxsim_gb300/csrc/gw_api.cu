@@ -61,6 +61,19 @@ int copy_stream_ready(gw_ctx *c) {
   return GW_OK;
 }
 
+int answer_ready(gw_ctx *c) {
+  GW_TRY(copy_stream_ready(c));
+  if (!c->h_answer) GW_CUDA(cudaMallocHost((void **)&c->h_answer, sizeof(int)));
+  if (!c->answer_ev)
+    GW_CUDA(cudaEventCreateWithFlags(&c->answer_ev, cudaEventDisableTiming));
+  return GW_OK;
+}
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
 int copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st) {
   // Pipelined: worker threads fault in 32 MB chunks in order while this
   // thread copies each chunk as soon as it is ready.
@@ -440,6 +453,8 @@ int gw_ctx_destroy(gw_ctx *c) {
   if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
   for (cudaEvent_t e : c->copy_ev)
     if (e) cudaEventDestroy(e);
+  if (c->answer_ev) cudaEventDestroy(c->answer_ev);
+  if (c->h_answer) cudaFreeHost(c->h_answer);
   gw::dev_free(c->d_err);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->stream) cudaStreamDestroy(c->stream);

@@ -214,6 +214,10 @@ struct gw_ctx {
   // stream's kernels (made on first use)
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t copy_ev[17] = {};
+  // a page-locked word that the device writes an answer to, and the event of
+  // the kernel that writes it (made on first use)
+  int *h_answer = nullptr;
+  cudaEvent_t answer_ev = nullptr;
 };
 
 namespace gw {
@@ -259,6 +263,10 @@ int copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
 bool host_resident(const void *p, size_t bytes);
 // the context's copy stream and events, made on first use
 int copy_stream_ready(gw_ctx *c);
+// the context's answer word, its event and the copy stream, made on first use
+int answer_ready(gw_ctx *c);
+// work put into the stream is being captured
+bool capturing(cudaStream_t st);
 
 }  // namespace gw
 

@@ -40,6 +40,21 @@ using namespace gwv;
 
 namespace {
 
+// ------------------------------------------------------------ real grids
+// *bad = 1 (in host memory) when some atom's f is not a real multiple of its
+// structure's average voxel f, to the float32 precision of f (NaN is not).
+__global__ void k_real_along(const float2 *f, const gw_structure *st, int *bad) {
+  const gw_structure s = st[blockIdx.y];
+  const float2 u = unit_phase(s);
+  bool ok = true;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < s.atom_count;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const float2 v = f[s.atom_begin + i];
+    ok = ok && fabsf(v.y * u.x - v.x * u.y) <= 1e-6f * (fabsf(v.x) + fabsf(v.y));
+  }
+  if (!ok) *bad = 1;
+}
+
 // ------------------------------------------------------------ structure prep
 // Per structure: the minimum z, and the atoms furthest out in kDirs
 // directions of the x-y plane.  Their convex polygon bounds the atoms that
@@ -1883,8 +1898,12 @@ int path_buffers(gw_voxel_plan *P, const char *who) {
 // beside the present ones; where that fails (gather binning asked for by name,
 // its store of twice the columns beyond GW_GATHER_MAX_MB: GW_ERR_ARG), the plan
 // is as it was.
+bool gwv::wide_real(const gw_voxel_plan *P) {
+  return P->real && 2 * P->Ly > fft_ldm(P->My);
+}
+
 int gwv::may_leave_real(const gw_voxel_plan *P, const char *who) {
-  if (P->real && 2 * P->Ly <= fft_ldm(P->My))
+  if (P->real && !wide_real(P))
     return gw::fail(GW_ERR_STATE, std::string(who) + ": the plan was made with real_grids; "
                                   "per-shell f values and the adjoint need real_grids 0");
   return GW_OK;
@@ -2311,11 +2330,13 @@ extern "C" int gw_voxel_set_atoms(gw_voxel_plan *P, const double *xyz,
     P->n_atoms = n;
     if (P->gexec) { cudaGraphExecDestroy(P->gexec); P->gexec = nullptr; }
     if (P->graph) { cudaGraphDestroy(P->graph); P->graph = nullptr; }
+    P->graph_kernels = 0;
   }
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   GW_CUDA(cudaMemcpyAsync(P->d_xyz, xyz, (size_t)n * 3 * sizeof(double), kind, P->ctx->stream));
   GW_CUDA(cudaMemcpyAsync(P->d_f, f, (size_t)n * sizeof(float2), kind, P->ctx->stream));
   P->f_stale = false;
+  P->f_unseen = true;
   return GW_OK;
 }
 
@@ -2419,16 +2440,62 @@ static int shell_state(gw_voxel_plan *P, const char *who) {
   return GW_OK;
 }
 
+// A wide real-grid plan takes any f values: ones that are not real multiples of
+// the structures' average voxel f take it to the general path (the real one
+// would give wrong intensities).  The first execute of new atoms has the device
+// look at them beside its pass, on the copy stream, and reads the answer when
+// the pass is launched: 5000 atoms at 24 angles take 63.5 us without it, 64
+// so, 75 with the kernel and a copy of its answer ahead of the pass, 90 when the
+// host waits before it launches.  In a stream capture, which cannot wait, the
+// caller's statement stands.
+namespace {
+struct FLook {
+  bool on = false, bad = false;
+  int begin(gw_voxel_plan *P) {
+    gw_ctx *c = P->ctx;
+    if (!P->f_unseen || !gwv::wide_real(P) || gw::capturing(c->stream)) return GW_OK;
+    GW_TRY(gw::answer_ready(c));
+    *c->h_answer = 0;
+    GW_CUDA(cudaEventRecord(c->answer_ev, c->stream));
+    GW_CUDA(cudaStreamWaitEvent(c->copy_stream, c->answer_ev, 0));
+    k_real_along<<<dim3(std::min(gwv::atom_blocks(P), 64), P->n_struct), 256, 0,
+                   c->copy_stream>>>(P->d_f, P->d_structs, c->h_answer);
+    GW_LAUNCHED(c);
+    GW_CUDA(cudaEventRecord(c->answer_ev, c->copy_stream));
+    on = true;
+    return GW_OK;
+  }
+  int end(gw_voxel_plan *P) {
+    if (!on) return GW_OK;
+    GW_CUDA(cudaEventSynchronize(P->ctx->answer_ev));
+    bad = *static_cast<volatile int *>(P->ctx->h_answer) != 0;
+    P->f_unseen = false;
+    return GW_OK;
+  }
+};
+}  // namespace
+
 extern "C" int gw_voxel_execute(gw_voxel_plan *P) {
   if (!P) return gw::fail(GW_ERR_ARG, "gw_voxel_execute: null plan");
   if (P->n_atoms < 0) return gw::fail(GW_ERR_STATE, "gw_voxel_execute: atoms not set");
   GW_TRY(shell_state(P, "gw_voxel_execute"));
   GW_CUDA(cudaSetDevice(P->ctx->device));
   gw::Range r("giwaxsim: voxel execute");
+  FLook look;
+  GW_TRY(look.begin(P));
   if (P->gexec) {
     GW_CUDA(cudaGraphLaunch(P->gexec, P->ctx->stream));
     P->ctx->launches += P->graph_kernels;
   } else {
+    GW_TRY(voxel_enqueue_all(P));
+  }
+  GW_TRY(look.end(P));
+  if (look.bad) {  // again, on the general path
+    P->executed = false;
+    if (const int st = gwv::leave_real(P, "gw_voxel_execute")) {
+      P->n_atoms = -1;  // (these atoms cannot be executed)
+      return st;
+    }
     GW_TRY(voxel_enqueue_all(P));
   }
   P->executed = true;
@@ -2456,6 +2523,10 @@ extern "C" int gw_voxel_capture_graph(gw_voxel_plan *P) {
   GW_TRY(shell_state(P, "gw_voxel_capture_graph"));
   if (P->gexec) return GW_OK;
   GW_CUDA(cudaSetDevice(P->ctx->device));
+  FLook look;
+  GW_TRY(look.begin(P));
+  GW_TRY(look.end(P));
+  if (look.bad) GW_TRY(gwv::leave_real(P, "gw_voxel_capture_graph"));
   // first-launch attributes must be set outside capture
   GW_TRY(voxel_enqueue_all(P));
   GW_CUDA(cudaStreamSynchronize(P->ctx->stream));
@@ -2606,7 +2677,8 @@ extern "C" int gw_voxel_info(gw_voxel_plan *P, int64_t *info, int32_t n) {
                        (int64_t)P->bytes, P->graph_kernels,
                        (int64_t)P->f1_tma, (int64_t)P->fused_y,
                        (int64_t)P->fused_z, (int64_t)P->real, (int64_t)P->gather,
-                       P->gather ? P->n_heavy : 0, P->gather ? P->n_zmulti : 0};
+                       P->gather ? P->n_heavy : 0, P->gather ? P->n_zmulti : 0,
+                       (int64_t)gwv::wide_real(P)};
   const int k = std::min<int>(n, (int)(sizeof v / sizeof v[0]));
   for (int i = 0; i < k; ++i) info[i] = v[i];
   return k;

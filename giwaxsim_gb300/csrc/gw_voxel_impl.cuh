@@ -658,6 +658,7 @@ struct gw_voxel_plan {
   bool sorted_real = false;    // d_xyf_s was made for real grids
   int *d_cand = nullptr;       // candidates for the y extremes (sorted positions)
   int *d_ncand = nullptr, *d_any_ext = nullptr;
+  bool f_unseen = false;       // no execute has looked at the atoms' f values
   unsigned long long *d_dirs = nullptr;  // per structure: outermost atoms
   std::vector<int> roff_host;  // per-slice first window row (n_slices+1)
   int *d_roff = nullptr;       // null when every slice has Lz rows
@@ -718,6 +719,9 @@ int fused_col_block(const gw_voxel_plan *P);
 // I(q) grids.
 int enqueue_finalize(gw_voxel_plan *P, bool f64);
 int enqueue_gather(gw_voxel_plan *P, int mode, int t, int line_lo = 0, int line_hi = -1);
+// A plan on the real path whose window is wider than half a transform buffer:
+// it takes every call and f value, on the general path where they need it.
+bool wide_real(const gw_voxel_plan *P);
 // Refuses (GW_ERR_STATE) the calls that need the general path on a real-grid
 // plan, unless its window is wide.
 int may_leave_real(const gw_voxel_plan *P, const char *who);

@@ -417,6 +417,18 @@ class VoxelPlan:
             len(self.structs), N.ptr(self.phi_tab), len(self.phi_tab),
             ctypes.byref(h)))
         self.handle = h
+        self._wide = bool(self.params.real_grids) and self.info()["wide_real"] == 1
+
+    @property
+    def graph_captured(self):
+        """A captured graph runs the executes (a wide real-grid plan drops
+        it when it goes on on the general path)."""
+        return self._graph and not (getattr(self, "_wide", False)
+                                    and self.info()["graph_kernels"] == 0)
+
+    @graph_captured.setter
+    def graph_captured(self, on):
+        self._graph = on
 
     def key(self):
         """Everything gw_voxel_plan_create receives: two plans with equal
@@ -549,7 +561,7 @@ class VoxelPlan:
         keys = ["crop", "batch", "Ly", "Lz", "Nc", "Nr", "My", "Mz", "y_lo",
                 "z_lo", "k0", "kz0", "n_slices", "device_bytes",
                 "graph_kernels", "col_tma", "fused_y", "fused_z", "real",
-                "gather", "heavy_lines", "multi_rows"]
+                "gather", "heavy_lines", "multi_rows", "wide_real"]
         return dict(zip(keys, (int(x) for x in v[:n])))
 
     def debug_deposit(self, slice_index):
@@ -586,12 +598,9 @@ class VoxelPlan:
             if g_iq.shape != (self.Qc,) * 3:
                 raise ValueError("g_iq must have shape %s" % ((self.Qc,) * 3,))
             src, flag = N.ptr(g_iq), 0
-        st = N.lib().gw_voxel_backward(self.handle, src, flag, N.ptr(g_f),
-                                       N.ptr(g_xyz), N.ptr(g_sigma), N.ptr(g_c))
-        # a real-grid plan that left the real path for this has no graph now
-        if self.graph_captured and self.params.real_grids:
-            self.graph_captured = self.info()["graph_kernels"] > 0
-        N.check(st)
+        N.check(N.lib().gw_voxel_backward(self.handle, src, flag, N.ptr(g_f),
+                                          N.ptr(g_xyz), N.ptr(g_sigma),
+                                          N.ptr(g_c)))
         return dict(g_f=g_f.view(complex), g_xyz=g_xyz, g_sigma=float(g_sigma[0]),
                     g_c=g_c.view(complex))
 

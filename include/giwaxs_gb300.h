@@ -163,10 +163,11 @@ typedef struct gw_voxel_params {
                            bands are made symmetric.  Used in batched,
                            nearest-bin plans with the Stockham kernels (not
                            with GW_TRANSFORM_FUSED) with row transforms up
-                           to 2048 points; no shells, no backward, but a
-                           plan whose window is wider than half a transform
-                           buffer takes them and goes on on the general
-                           path.  gw_voxel_info reports whether it runs.
+                           to 2048 points; no shells, no backward, no other
+                           f values later, but a plan whose window is wider
+                           than half a transform buffer takes them and goes
+                           on on the general path.  gw_voxel_info reports
+                           whether it runs.
                            0: the general path.                            */
   int32_t binning;      /* how |F|^2 pixels reach the voxel sums.
                            GW_BINNING_ATOMIC: float64 atomic adds as the
@@ -214,7 +215,11 @@ int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
 int gw_voxel_plan_destroy(gw_voxel_plan *plan);
 /* Atoms: xyz (n,3) float64, f (n,2) float32 complex scattering factor
  * (Z + f' + i f'', times any per-atom weight).  on_device: 0 host, 1 device
- * (device pointers are copied into the plan). */
+ * (device pointers are copied into the plan).  f values that are not real
+ * multiples of the structures' average voxel f take a wide real-grid plan
+ * (gw_voxel_info's wide_real) to the general path at the next execute, which
+ * waits until the device has looked at them (not while the stream is being
+ * captured: the caller's statement of real_grids stands there). */
 int gw_voxel_set_atoms(gw_voxel_plan *plan, const double *xyz, const float *f,
                        int64_t n_atoms, int32_t on_device);
 /* Multi-q atomic form factors (voxelgrids.py:650-707, aff_num_qs > 1).
@@ -271,8 +276,9 @@ int gw_voxel_get_sums(gw_voxel_plan *plan, double *sums);
  * fused chirp-z kernel runs along that axis), real (1 when the real-grid
  * path runs), gather (1 when the gather binning runs), heavy_lines (gather:
  * window lines summed by a whole block each), multi_rows (gather: window z
- * with more than one output row)].  Returns the number written (at most
- * n). */
+ * with more than one output row), wide_real (1 while a real-grid plan may
+ * still change to the general path, see real_grids)].  Returns the number
+ * written (at most n). */
 int gw_voxel_info(gw_voxel_plan *plan, int64_t *info, int32_t n);
 /* Deposit indices of one slice (after execute): y,z voxel index per atom of
  * that slice's structure, -1 where the reference's valid_mask drops it

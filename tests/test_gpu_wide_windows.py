@@ -272,3 +272,65 @@ def test_graph_captured_follows_the_change_of_path():
         assert plan.graph_captured and plan.info()["graph_kernels"] > 0
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("which,capture", [(0, False), (1, False), (1, True)])
+def test_other_f_values_on_the_device(which, capture):
+    """Device f values that are not real multiples of the average voxel f
+    take a wide plan to the general path; multiples keep it and its graph."""
+    torch = pytest.importorskip("torch")
+    axes, box, m = CASES[2]
+    geom = F.VoxelGeometry(*axes)
+    (xyz, fv), (xyz2, fv2) = atoms(box, 3), atoms(0.9 * box, 4, 2500)
+    items = [(xyz, fv, None), (xyz2, fv2 * 1j, None)]
+    other = [fv.copy(), fv2 * 1j]
+    other[which][7::11] *= 1.0 - 0.01j
+    other = np.concatenate(other).astype(np.complex64)
+    got = []
+    for real in (None, False):
+        plan = F.VoxelPlan(geom, items, phis=PHIS, smooth=1.0, real=real)
+        try:
+            x = torch.as_tensor(plan.xyz).cuda()
+            good = torch.as_tensor(plan.f).cuda() * 1.5
+            bad = torch.as_tensor(other.view(np.float32)).cuda()
+            torch.cuda.synchronize()
+            plan.set_atoms(x.data_ptr(), good.data_ptr(), on_device=True)
+            plan.capture_graph()
+            plan.set_atoms(x.data_ptr(), good.data_ptr(), on_device=True)
+            plan.execute()
+            assert plan.info()["real"] == (real is None) and plan.graph_captured
+            got.append([plan.iq().copy()])
+            if real is None:
+                # set and not executed: nothing happens
+                plan.set_atoms(x.data_ptr(), bad.data_ptr(), on_device=True)
+                plan.set_atoms(x.data_ptr(), good.data_ptr(), on_device=True)
+                plan.execute()
+                assert plan.info()["real"] == 1 and rel_l2(plan.iq(), got[-1][0]) <= RTOL
+                plan.set_atoms(x.data_ptr(), bad.data_ptr(), on_device=True)
+                N.set_alloc_fault(0)
+                try:
+                    with pytest.raises(N.GwError) as e:
+                        plan.execute()
+                    assert e.value.status == N.GW_ERR_OOM
+                finally:
+                    N.set_alloc_fault(-1)
+                for call in (plan.execute, plan.iq, plan.capture_graph):
+                    with pytest.raises(N.GwError) as e:
+                        call()
+                    assert e.value.status == N.GW_ERR_STATE and plan.info()["real"] == 1
+            plan.set_atoms(x.data_ptr(), bad.data_ptr(), on_device=True)
+            if capture:
+                plan.capture_graph()
+                assert plan.info()["real"] == 0
+            plan.execute()
+            assert plan.info()["real"] == 0
+            assert plan.graph_captured == (real is False or capture)
+            got[-1].append(plan.iq().copy())
+            plan.set_atoms(x.data_ptr(), good.data_ptr(), on_device=True)
+            plan.execute()
+            got[-1].append(plan.iq().copy())
+        finally:
+            plan.close()
+    for a, b in zip(*got):
+        assert rel_l2(a, b) <= RTOL
+    assert rel_l2(got[1][1], got[1][0]) > 100 * RTOL
