@@ -34,6 +34,8 @@
 #include <vector>
 
 #include "gw_tma.cuh"
+#include <cooperative_groups.h>
+
 #include "gw_voxel_impl.cuh"
 
 using namespace gwv;
@@ -434,90 +436,155 @@ __device__ __forceinline__ void y_block_reduce(T (&lo)[S], T (&hi)[S]) {
   }
 }
 
-// The extremes of the block's slices, then, per slice, its background
-// constants and the extents of the valid atoms (voxelgrids.py:346-349): y
-// indices grow with y (the floor division is monotone), so when every atom is
-// valid the extents are (0, index of max y, 0, largest occupied z row);
-// otherwise k_ext_exact computes them atom by atom.  Bound by the candidates'
-// gathers from L2.  Over all atoms, with a reset and the extents in launches
-// of their own, 16 boxes of 57,000 atoms at 180 angles each took 389 us, one of
-// 13,713 at 180 angles 27 us and one of 264,424 at 720 angles 332 us; this and
-// k_ext_exact take 31, 7 and 14 us (the candidate test costs k_zscatter 2-6 us
-// a box of these).
-template <int S>
-__global__ void __launch_bounds__(256) k_yext(SliceArgs a, int slice0, int n) {
-  __shared__ float s_lo[S], s_hi[S];
-  const int first = slice0 + blockIdx.x * S;
-  const int ns = min(S, slice0 + n - first);
-  double c[S], sn[S];
+// A structure of more than `share` candidates (a hollow one: most atoms are) has
+// its slices' candidates shared by the blocks of a cluster (y_share).
+__device__ __forceinline__ bool y_shared(const SliceArgs &a, int sl, int share) {
+  return a.ncand[sl / a.n_phi] > share;
+}
+
+// The candidates i0, i0 + stride, .. of those of slices first .. first + ns - 1
+// that are shared (or are not), kYBatch of them at a time so that their gathers
+// are in flight together: each(sorted position, atom, first, end slice).  Where
+// most atoms are candidates, all atoms are taken instead, in order (coalesced,
+// without the list).
+constexpr int kYBatch = 4;
+template <class Each>
+__device__ __forceinline__ void y_candidates(const SliceArgs &a, int first, int ns, int share,
+                                             bool shared, int i0, int stride, Each each) {
+  for (int kb = 0, ke; kb < ns; kb = ke) {
+    ke = y_run_end(a, first, kb, ns);
+    if (y_shared(a, first + kb, share) != shared) continue;
+    const int t = (first + kb) / a.n_phi;
+    const int begin = (int)a.st[t].atom_begin, atoms = (int)a.st[t].atom_count;
+    const int *cand = a.cand + begin;
+    const int listed = a.ncand[t];
+    const bool all = 2 * (int64_t)listed > atoms;
+    const int nc = all ? atoms : listed;
+    int i = i0;
+    for (; i + (kYBatch - 1) * stride < nc; i += kYBatch * stride) {
+      int pos[kYBatch];
+      float4 q[kYBatch];
+#pragma unroll
+      for (int b = 0; b < kYBatch; ++b) pos[b] = all ? begin + i + b * stride : cand[i + b * stride];
+#pragma unroll
+      for (int b = 0; b < kYBatch; ++b) q[b] = a.xyf_s[pos[b]];
+#pragma unroll
+      for (int b = 0; b < kYBatch; ++b) each(pos[b], q[b], kb, ke);
+    }
+    for (; i < nc; i += stride) {
+      const int pos = all ? begin + i : cand[i];
+      each(pos, a.xyf_s[pos], kb, ke);
+    }
+  }
+}
+
+// The extremes of those of slices first .. first + ns - 1 (at most S) that are
+// SHARED by the cluster's blocks (or are not), then, per slice, its background constants and the extents of the valid atoms
+// (voxelgrids.py:346-349): y indices grow with y (the floor division is
+// monotone), so when every atom is valid the extents are (0, index of max y, 0,
+// largest occupied z row); otherwise ext_exact computes them atom by atom.
+template <int S, bool SHARED>
+__device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns, int share) {
+  namespace cg = cooperative_groups;
+  __shared__ unsigned s_f[2][S];
+  __shared__ float s_b[2][S];
+  __shared__ unsigned long long s_d[2][S];
+  int rank = 0, blocks = 1;
+  if constexpr (SHARED) {
+    rank = cg::this_cluster().block_rank();
+    blocks = cg::this_cluster().num_blocks();
+  }
+  float cf[S], sf[S];
   unsigned flo[S], fhi[S];  // ordered: min of (y'+d), max of (y'-d)
 #pragma unroll
   for (int k = 0; k < S; ++k) {
-    const int p = (first + min(k, ns - 1)) % a.n_phi;
-    c[k] = a.ph[p].cos_phi;
-    sn[k] = a.ph[p].sin_phi;
+    const gw_phi &ph = a.ph[(first + min(k, ns - 1)) % a.n_phi];
+    cf[k] = (float)ph.cos_phi;
+    sf[k] = (float)ph.sin_phi;
     flo[k] = ~0u;
     fhi[k] = 0u;
   }
-  for (int kb = 0; kb < ns;) {
-    const int ke = y_run_end(a, first, kb, ns);
-    const int t = (first + kb) / a.n_phi;
-    const int *cand = a.cand + a.st[t].atom_begin;
-    const int nc = a.ncand[t];
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-      const float4 q = a.xyf_s[cand[i]];
+  const int i0 = rank * blockDim.x + threadIdx.x, stride = blocks * blockDim.x;
+  y_candidates(a, first, ns, share, SHARED, i0, stride, [&](int, float4 q, int kb, int ke) {
 #pragma unroll
-      for (int k = 0; k < S; ++k) {
-        if (k < kb || k >= ke) continue;
-        float l, h;
-        y_interval(q, (float)c[k], (float)sn[k], l, h);
-        flo[k] = min(flo[k], flt_ord(h));
-        fhi[k] = max(fhi[k], flt_ord(l));
-      }
+    for (int k = 0; k < S; ++k) {
+      if (k < kb || k >= ke) continue;
+      float l, h;
+      y_interval(q, cf[k], sf[k], l, h);
+      flo[k] = min(flo[k], flt_ord(h));
+      fhi[k] = max(fhi[k], flt_ord(l));
     }
-    kb = ke;
-  }
+  });
   y_block_reduce<S>(flo, fhi);
   if (threadIdx.x == 0)
 #pragma unroll
     for (int k = 0; k < S; ++k) {
-      s_lo[k] = ord_flt(flo[k]);
-      s_hi[k] = ord_flt(fhi[k]);
+      s_f[0][k] = flo[k];
+      s_f[1][k] = fhi[k];
     }
+  if constexpr (SHARED) cg::this_cluster().sync();
+  else __syncthreads();
+  if (threadIdx.x < S) {
+    unsigned l = s_f[0][threadIdx.x], h = s_f[1][threadIdx.x];
+    if constexpr (SHARED)
+      for (int b = 0; b < blocks; ++b) {
+        const unsigned *f = cg::this_cluster().map_shared_rank(&s_f[0][0], b);
+        l = min(l, f[threadIdx.x]);
+        h = max(h, f[S + threadIdx.x]);
+      }
+    s_b[0][threadIdx.x] = ord_flt(l);
+    s_b[1][threadIdx.x] = ord_flt(h);
+  }
   __syncthreads();
+  float blo[S], bhi[S];
   unsigned long long lo[S], hi[S];
 #pragma unroll
   for (int k = 0; k < S; ++k) {
+    blo[k] = s_b[0][k];
+    bhi[k] = s_b[1][k];
     lo[k] = ~0ULL;
     hi[k] = 0ULL;
   }
-  for (int kb = 0; kb < ns;) {
-    const int ke = y_run_end(a, first, kb, ns);
-    const int t = (first + kb) / a.n_phi;
-    const int *cand = a.cand + a.st[t].atom_begin;
-    const int nc = a.ncand[t];
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-      const int pos = cand[i];
-      const float4 q = a.xyf_s[pos];
+  y_candidates(a, first, ns, share, SHARED, i0, stride, [&](int pos, float4 q, int kb, int ke) {
 #pragma unroll
-      for (int k = 0; k < S; ++k) {
-        if (k < kb || k >= ke) continue;
-        float l, h;
-        y_interval(q, (float)c[k], (float)sn[k], l, h);
-        if (l <= s_lo[k] || h >= s_hi[k]) {
-          const unsigned long long v = dbl_ord(rot_y(a.xyz_s + 3 * (size_t)pos, c[k], sn[k]));
-          lo[k] = min(lo[k], v);
-          hi[k] = max(hi[k], v);
-        }
+    for (int k = 0; k < S; ++k) {
+      if (k < kb || k >= ke) continue;
+      float l, h;
+      y_interval(q, cf[k], sf[k], l, h);
+      if (l <= blo[k] || h >= bhi[k]) {
+        const gw_phi &ph = a.ph[(first + k) % a.n_phi];
+        const unsigned long long v =
+            dbl_ord(rot_y(a.xyz_s + 3 * (size_t)pos, ph.cos_phi, ph.sin_phi));
+        lo[k] = min(lo[k], v);
+        hi[k] = max(hi[k], v);
       }
     }
-    kb = ke;
-  }
+  });
   y_block_reduce<S>(lo, hi);
+  if constexpr (SHARED) {
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < S; ++k) {
+        s_d[0][k] = lo[k];
+        s_d[1][k] = hi[k];
+      }
+    cg::this_cluster().sync();
+    if (rank == 0 && threadIdx.x == 0)
+      for (int b = 1; b < blocks; ++b) {
+        const unsigned long long *d = cg::this_cluster().map_shared_rank(&s_d[0][0], b);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          lo[k] = min(lo[k], d[k]);
+          hi[k] = max(hi[k], d[S + k]);
+        }
+      }
+    cg::this_cluster().sync();  // (its shared memory stays until it is read)
+    if (rank != 0) return;
+  }
   if (threadIdx.x != 0) return;
 #pragma unroll
   for (int k = 0; k < S; ++k) {
-    if (k >= ns) continue;
+    if (k >= ns || y_shared(a, first + k, share) != SHARED) continue;
     const int sl = first + k, t = sl / a.n_phi;
     a.ymin_ord[sl] = lo[k];
     // background constant C = avg_voxel_f * max_voxels (voxelgrids.py:358,365):
@@ -549,15 +616,33 @@ __global__ void __launch_bounds__(256) k_yext(SliceArgs a, int slice0, int n) {
   }
 }
 
-// The extents of slice sl's valid atoms, this block's share of the atoms.
-__device__ __forceinline__ void ext_exact(const SliceArgs &a, int sl) {
+// The slices whose candidates are not shared; k_yrest does the others.  Bound by
+// the candidates' gathers from L2: a block of S = 4 slices reuses each of them,
+// S = 1 keeps multiprocessors busy while four would leave some idle (180 slices:
+// 12.3 us at four a block, 5.3 at one; 2880: 29.7 at four).
+// Over all atoms, with a reset and the extents in launches of their own, 16 boxes
+// of 57,000 atoms at 180 angles each took 389 us, one of 13,713 at 180 angles 27
+// us and one of 264,424 at 720 angles 332 us; this and the extents take 39, 10 and
+// 26 us from cold caches (the candidate test costs k_zscatter 2-6 us a box of
+// these).
+template <int S>
+__global__ void __launch_bounds__(256) k_yext(SliceArgs a, int slice0, int n, int share) {
+  const int first = slice0 + blockIdx.x * S, ns = min(S, slice0 + n - first);
+  int shared = 0;
+  for (int k = 0; k < ns; ++k) shared += y_shared(a, first + k, share);
+  if (shared && threadIdx.x == 0) *a.any_ext = 1;
+  if (shared < ns) y_extents<S, false>(a, first, ns, share);
+}
+
+// The extents of slice sl's valid atoms: share `part` of `parts` of the atoms.
+__device__ __forceinline__ void ext_exact(const SliceArgs &a, int sl, int part, int parts) {
   const int t = sl / a.n_phi, p = sl % a.n_phi;
   const gw_structure s = a.st[t];
   const double c = a.ph[p].cos_phi, sn = a.ph[p].sin_phi;
   const double ymin = ord_dbl(a.ymin_ord[sl]);
   int ymn = INT_MAX, ymx = -1, zmn = INT_MAX, zmx = -1;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-       i < s.atom_count; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = part * (int64_t)blockDim.x + threadIdx.x;
+       i < s.atom_count; i += (int64_t)parts * blockDim.x) {
     const int64_t at = s.atom_begin + i;
     const double y = GW_DSUB(rot_y(a.xyz + 3 * at, c, sn), ymin);
     const int yi = (int)floor_div_exact(y, a.r, a.inv_r);
@@ -583,7 +668,34 @@ __device__ __forceinline__ void ext_exact(const SliceArgs &a, int sl) {
 __global__ void k_ext_exact(SliceArgs a, int slice0, int n) {
   if (!*a.any_ext) return;
   for (int sl = slice0 + blockIdx.y; sl < slice0 + n; sl += gridDim.y)
-    if (a.extflag[sl]) ext_exact(a, sl);
+    if (a.extflag[sl]) ext_exact(a, sl, blockIdx.x, gridDim.x);
+}
+
+// The same for plans with a structure of more atoms than `share`, after the
+// extremes of the slices whose candidates are shared: a cluster takes S slices at
+// a time.  A tube of 264,000 atoms at 24 / 180 / 720 angles: 81 / 135 / 388 us
+// over all atoms, 903 / 906 / 1260 with one block for a slice (or four) that
+// gathers one candidate at a time, 51 / 116 / 307 so.
+constexpr int kYBlocks = 8;
+template <int S>
+__global__ void __launch_bounds__(256) __cluster_dims__(kYBlocks, 1, 1)
+k_yrest(SliceArgs a, int slice0, int n, int share) {
+  namespace cg = cooperative_groups;
+  if (!*a.any_ext) return;  // (set before this launch; the same for every block)
+  const int rank = cg::this_cluster().block_rank();
+  for (int first = slice0 + blockIdx.x / kYBlocks * S; first < slice0 + n;
+       first += gridDim.x / kYBlocks * S) {
+    const int ns = min(S, slice0 + n - first);
+    bool shared = false;
+    for (int k = 0; k < ns; ++k) shared |= y_shared(a, first + k, share);
+    if (shared) {
+      y_extents<S, true>(a, first, ns, share);
+      __threadfence();
+      cg::this_cluster().sync();  // (the flags are written, shared memory is free)
+    }
+    for (int k = 0; k < ns; ++k)
+      if (__ldcg(a.extflag + first + k)) ext_exact(a, first + k, rank, kYBlocks);
+  }
 }
 
 // Per-slice profiles: fill_bkg column term (minus the background) and the
@@ -1493,20 +1605,35 @@ SliceArgs profile_view(const SliceArgs &a, int s0) {
   return v;
 }
 
+// Candidates of a structure that one block still takes alone, with n slices at
+// once: the fewer blocks the slices give, the sooner a cluster shares them (tubes:
+// 57,000 atoms at 180 angles 46 us shared, 212 not; 14,000 at 720 angles 72 and 52,
+// at 2880 235 and 101).
+static int y_share(const gw_ctx *ctx, int n) {
+  return n > 16 * ctx->sm_count ? INT_MAX : n > 4 * ctx->sm_count ? 16384 : 4096;
+}
+
 int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n) {
   gw_ctx *ctx = P->ctx;
   cudaStream_t st = ctx->stream;
+  const int share = y_share(ctx, n);
+  int64_t max_atoms = 0;
+  for (auto &s : P->structs) max_atoms = std::max(max_atoms, s.atom_count);
   {
     gw::KTimer tm(ctx, GW_K_DEPOSIT);
-    // four slices a block reuse each candidate, once there are blocks enough
-    // (180 slices: 12.3 us at four a block, 5.3 at one; 2880: 29.7 at four)
-    if (n > 4 * ctx->sm_count) k_yext<4><<<(n + 3) / 4, 256, 0, st>>>(a, s0, n);
-    else k_yext<1><<<n, 256, 0, st>>>(a, s0, n);
+    // four slices a block once there are blocks enough
+    if (n > 4 * ctx->sm_count) k_yext<4><<<(n + 3) / 4, 256, 0, st>>>(a, s0, n, share);
+    else k_yext<1><<<n, 256, 0, st>>>(a, s0, n, share);
     GW_LAUNCHED(ctx);
   }
   {
     gw::KTimer tm(ctx, GW_K_DEPOSIT);
-    k_ext_exact<<<dim3(std::min(atom_blocks(P), 16), std::min(n, 64)), 256, 0, st>>>(a, s0, n);
+    if (max_atoms <= share)
+      k_ext_exact<<<dim3(std::min(atom_blocks(P), 16), std::min(n, 64)), 256, 0, st>>>(a, s0, n);
+    else if (n > ctx->sm_count)  // (clusters of four slices each fill the GPU)
+      k_yrest<4><<<std::min((n + 3) / 4, 128) * kYBlocks, 256, 0, st>>>(a, s0, n, share);
+    else
+      k_yrest<1><<<std::min(n, 128) * kYBlocks, 256, 0, st>>>(a, s0, n, share);
     GW_LAUNCHED(ctx);
   }
   if (a.fill || a.smooth_on) {
