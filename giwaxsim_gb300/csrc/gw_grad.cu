@@ -696,7 +696,7 @@ extern "C" int gw_voxel_backward(gw_voxel_plan *P, const double *g_iq,
     }
     if (P->bil) {
       gw::KTimer tm(ctx, GW_K_MISC);
-      k_argmin_y<<<dim3(std::min(nblk_at, 2), nb), 256, 0, st>>>(a, c0, P->d_perm, G->d_amy);
+      k_argmin_y<<<dim3(std::min(nblk_at, 16), nb), 256, 0, st>>>(a, c0, P->d_perm, G->d_amy);
       GW_LAUNCHED(ctx);
     }
   }
