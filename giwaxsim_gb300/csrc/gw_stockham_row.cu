@@ -76,6 +76,18 @@ struct RowShape<1536, REAL> { static constexpr int NB = 2, NT = 192, MINB = 5; }
 template <bool REAL>
 struct RowShape<2048, REAL> { static constexpr int NB = 2, NT = 256, MINB = 4; };
 
+// Real rows of the short lengths in launches of fewer than four blocks a
+// multiprocessor: blocks of a fraction of the rows, so that the deposit, a chain
+// of loads and shared atomics, runs on more multiprocessors.  Whole passes, 128
+// points, 24 slices of 63 rows: 50.1 -> 46.0 us; 256 points, 24 of 158 rows 60.1
+// -> 56.1, 60 of them 60.9 -> 56.2 (180 with the smaller blocks too: 68.4 -> 72.7
+// of 108 rows).  No difference from 512 points up.
+template <int M> struct RowSmall { static constexpr int NB = 0; };
+template <> struct RowSmall<64>  { static constexpr int NB = 8, NT = 32, MINB = 16; };
+template <> struct RowSmall<128> { static constexpr int NB = 4, NT = 32, MINB = 16; };
+template <> struct RowSmall<256> { static constexpr int NB = 2, NT = 32, MINB = 16; };
+template <> struct RowSmall<384> { static constexpr int NB = 2, NT = 64, MINB = 16; };
+
 // HALF: the window (L) and the band (N) both fit in M / 2, so the forward
 // transform's first pass and the inverse transform's last pass are pruned.
 template <int M, bool BIL, bool HALF>
@@ -134,11 +146,11 @@ struct RowLoadPair {
   }
 };
 
-template <int M, bool HALF>
-__global__ void __launch_bounds__(RowShape<M, true>::NT, RowShape<M, true>::MINB)
+template <int M, bool HALF, class Shape>
+__global__ void __launch_bounds__(Shape::NT, Shape::MINB)
 k_row_czt_real(SliceArgs a, CztArgs cz, int slice0, int n_sl, int n_rows,
                int m_zero, int nf, float2 *F1) {
-  constexpr int NB = RowShape<M, true>::NB, NT = RowShape<M, true>::NT;
+  constexpr int NB = Shape::NB, NT = Shape::NT;
   constexpr int TWL = FftPlan<M>::tw_len();
   constexpr int LDM = FftPlan<M>::LDM;
   static_assert(LDM % 2 == 0, "two rows per transform buffer");
@@ -195,20 +207,30 @@ int launch_row_t(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
   return GW_OK;
 }
 
-template <int M, bool HALF>
-int launch_row_real(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
-                    int slice0, int n_sl) {
+template <int M, bool HALF, class Shape>
+int launch_row_real_t(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
+                      int slice0, int n_sl) {
   const int n_rows = batch_rows(P, slice0, n_sl);
-  constexpr int NB = RowShape<M, true>::NB, NT = RowShape<M, true>::NT;
+  constexpr int NB = Shape::NB, NT = Shape::NT;
   const size_t smem = (size_t)(NB * FftPlan<M>::LDM + FftPlan<M>::tw_len()) * sizeof(float2);
   static gw::SmemRecord attr;
-  GW_TRY(gw::smem_limit(attr, k_row_czt_real<M, HALF>, smem));
+  GW_TRY(gw::smem_limit(attr, k_row_czt_real<M, HALF, Shape>, smem));
   const int blocks = (n_rows + 2 * NB - 1) / (2 * NB);
   gw::KTimer tm(P->ctx, GW_K_ROW);
-  k_row_czt_real<M, HALF><<<blocks, NT, smem, P->ctx->stream>>>(
+  k_row_czt_real<M, HALF, Shape><<<blocks, NT, smem, P->ctx->stream>>>(
       a, cz, slice0, n_sl, n_rows, P->m_zero, P->Nf, P->d_F1);
   GW_LAUNCHED(P->ctx);
   return GW_OK;
+}
+
+template <int M, bool HALF>
+int launch_row_real(gw_voxel_plan *P, const SliceArgs &a, const CztArgs &cz,
+                    int slice0, int n_sl) {
+  if constexpr (RowSmall<M>::NB > 0) {
+    if (batch_rows(P, slice0, n_sl) < 4 * P->ctx->sm_count * 2 * RowShape<M, true>::NB)
+      return launch_row_real_t<M, HALF, RowSmall<M>>(P, a, cz, slice0, n_sl);
+  }
+  return launch_row_real_t<M, HALF, RowShape<M, true>>(P, a, cz, slice0, n_sl);
 }
 
 template <int M>

@@ -334,3 +334,65 @@ def test_other_f_values_on_the_device(which, capture):
     for a, b in zip(*got):
         assert rel_l2(a, b) <= RTOL
     assert rel_l2(got[1][1], got[1][0]) > 100 * RTOL
+
+
+# (r, dq, max_q), box edge; transform lengths from 64 to 384, wide and narrow
+SHORT = [((0.5, 0.15, 0.5), 8.0), ((0.4, 0.1, 0.6), 22.0), ((0.5, 0.15, 1.5), 13.0),
+         ((0.3, 0.08, 0.4), 45.0), ((0.3, 0.06, 1.0), 50.0)]
+
+
+@pytest.mark.parametrize("axes,box", SHORT)
+@pytest.mark.parametrize("accum", ["fp64", "kahan32"])
+def test_row_blocks_of_both_sizes(axes, box, accum):
+    """Real rows in the smaller blocks (launches that would not fill the GPU)
+    and in the others, several structures of uneven height (row pairs across two
+    slices, an odd number of rows), plain and from a graph, against the general
+    path."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    geom = F.VoxelGeometry(*axes)
+    items = [(xyz * [1.0, 1.0, z], fv, None) for (xyz, fv), z in
+             ((atoms(box, 5), 1.0), (atoms(0.8 * box, 6, 90), 2.7), (atoms(0.9 * box, 7, 411), 0.31))]
+    probe = F.VoxelPlan(geom, items, phis=PHIS)
+    rows = probe.info()["Lz"]
+    assert probe.info()["real"] == 1
+    probe.close()
+    # at most 16 sequences of two rows a block: four blocks a multiprocessor
+    enough = 4 * sms * 2 * 16 // rows + 1
+    for n_phi in (3, enough):
+        phis = np.linspace(0.0, 178.0, n_phi)
+        out = []
+        for real in (None, False):
+            plan = F.VoxelPlan(geom, items, phis=phis, fill_bkg=True, smooth=1.0, real=real,
+                               accum=accum)
+            try:
+                plan.set_atoms()
+                plan.execute()
+                out.append(plan.iq().copy())
+                plan.capture_graph()
+                plan.execute()
+                assert rel_l2(plan.iq(), out[-1]) <= RTOL
+            finally:
+                plan.close()
+        assert rel_l2(*out) <= RTOL
+
+
+@pytest.mark.parametrize("axes,box,m", CASES)
+def test_wide_windows_of_uneven_structures(axes, box, m):
+    """Row pairs across two slices, Kahan sums and a captured graph at every
+    length."""
+    geom = F.VoxelGeometry(*axes)
+    items = [(xyz * [1.0, 1.0, z], fv, None) for (xyz, fv), z in
+             ((atoms(box, 5), 1.0), (atoms(0.8 * box, 6, 90), 2.7))]
+    out = []
+    for real in (None, False):
+        plan = F.VoxelPlan(geom, items, phis=PHIS, smooth=1.5, real=real, accum="kahan32")
+        try:
+            plan.set_atoms()
+            plan.capture_graph()
+            plan.execute()
+            assert plan.info()["real"] == (real is None)
+            out.append(plan.iq().copy())
+        finally:
+            plan.close()
+    assert rel_l2(*out) <= RTOL
