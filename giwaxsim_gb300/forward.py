@@ -19,6 +19,7 @@ same float64 arithmetic per atom and per pixel:
 import atexit
 import ctypes
 import warnings
+from itertools import islice
 
 import numpy as np
 from numpy.fft import fftfreq, fftshift
@@ -831,18 +832,20 @@ def orientation_matrices(corners, psis, psi_weights, phis, phi_weights, thetas,
     An axis depends on the rotations before it only, so the matrices of one
     axis are made for all its angles at once; identity matrices are left
     out, which changes no bit."""
-    n1, n2, n3 = (min(len(a), len(w)) for a, w in
-                  ((psis, psi_weights), (phis, phi_weights), (thetas, theta_weights)))
+    # any iterables, as zip takes them
+    psi_weights, phi_weights, theta_weights = ws = [
+        list(islice(w, len(a))) for w, a in ((psi_weights, psis), (phi_weights, phis),
+                                             (theta_weights, thetas))]
+    n1, n2, n3 = (len(w) for w in ws)
     psis, phis, thetas = psis[:n1], phis[:n2], thetas[:n3]
     if n1 * n2 * n3 == 0:
         return np.zeros(0, np.int32), np.zeros((0, 3, 3)), np.zeros(0)
-    a, b, c = (np.asarray(v)[:n] for v, n in ((psi_weights, n1), (phi_weights, n2),
-                                              (theta_weights, n3)))
-    if a.dtype == b.dtype == c.dtype == np.float64:
+    if all(type(v) in (float, np.float64) for w in ws for v in w):
+        a, b, c = (np.array(w) for w in ws)
         w = a[:, None, None] * b[None, :, None] * c[None, None, :]
     else:  # other types multiply element by element in their own precision
-        w = np.array([p * h * t for p in psi_weights[:n1] for h in phi_weights[:n2]
-                      for t in theta_weights[:n3]], dtype=np.float64)
+        w = np.array([p * h * t for p in psi_weights for h in phi_weights
+                      for t in theta_weights], dtype=np.float64)
     # a zero angle about an axis of finite direction is the identity exactly:
     # the trailing axes whose angles are all zero need no corners
     p = corners.pts

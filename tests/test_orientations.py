@@ -63,3 +63,25 @@ def test_degenerate_plane_and_unequal_lists():
     n, m, w = F.orientation_matrices(F.PlaneCorners(h, h), [1.0, 2.0, 3.0], [0.5, 0.5],
                                      [0.0], [1.0], [], [])
     assert len(n) == len(m) == len(w) == 0
+
+
+def test_weights_of_any_iterable():
+    """Weights as zip takes them: generators, longer and mixed lists."""
+    h = np.linspace(-1, 1, 5)
+    c = F.PlaneCorners(h, h)
+    psis, phis, thetas = [0.0, 10.0, 20.0], [5.0, 6.0], [0.0, 1.0]
+    pw = [0.25, np.float32(0.1), 0.65]
+    hw, tw = (np.float32(0.3), 0.7, 0.9), [1, 2]
+    ref = one_by_one(c, psis, pw, phis, hw, thetas, tw)
+    got = F.orientation_matrices(c, psis, (w for w in pw), phis, hw, thetas, iter(tw))
+    for a, b in zip(got, ref):
+        assert np.array_equal(a, b)
+
+    def forever():
+        while True:
+            yield 0.5
+
+    ref = one_by_one(c, psis, [0.5] * 3, phis, [0.5] * 2, thetas, [0.5] * 2)
+    got = F.orientation_matrices(c, psis, forever(), phis, forever(), thetas, [0.5] * 9)
+    for a, b in zip(got, ref):
+        assert np.array_equal(a, b)
