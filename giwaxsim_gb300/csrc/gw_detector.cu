@@ -145,7 +145,8 @@ __global__ void k_det_debug(DetArgs a, int o, int64_t *idx) {
 // k_detector_fix replays with the exact float64 chain.
 struct OrientFast {
   // an axis whose coordinate is exactly +-0 for every pixel has A = 0, b =
-  // its (clipped) index + 0.5 and d = 0: it gathers that index, certainly
+  // its (clipped) index + 0.5 and d = 0: it gathers that index, certainly (d is
+  // infinite, and every sample replayed, for an index of 2^22 or more)
   float A[9];
   float b[3];
   float d[3];
@@ -872,7 +873,8 @@ extern "C" int gw_detector_plan_create(gw_ctx *ctx, const gw_detector_params *p,
           fix[3 * o + c] = (int)k;
           for (int j = 0; j < 3; ++j) ot[o].A[3 * c + j] = 0.f;
           ot[o].b[c] = (float)k + 0.5f;
-          ot[o].d[c] = 0.f;
+          // (beyond 2^22 the float32 floors are not exact: always replayed)
+          ot[o].d[c] = k < 4194304.0 ? 0.f : INFINITY;
         }
       }
       ot[o].w = (float)weights[o];

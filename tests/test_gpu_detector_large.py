@@ -1,0 +1,44 @@
+"""The detector gather at the limits of its index arithmetic: an axis fixed at
+an index beyond the float32 floors' range, a plane whose line pitch a 2-D copy
+does not take, and a volume of more than 2^32 elements, against the exact path
+(float64 indices of every sample)."""
+import numpy as np
+import pytest
+
+from giwaxsim_gb300 import forward as F
+
+pytestmark = pytest.mark.gpu
+
+
+def plans(shape, q, psis, phis=(0.0,), **kw):
+    """The fast and the exact plan; q: (x, y, z) axes of an I(q) of shape
+    (ny, nx, nz)."""
+    one = lambda a: np.full(len(a), 1.0 / len(a))  # noqa: E731
+    for exact in (False, True):
+        yield F.DetectorPlan(shape, *q, 64, 1.0, (), (), psis, one(psis), phis, one(phis), [0.0],
+                             [1.0], mirror=False, exact=exact, **kw)
+
+
+@pytest.mark.parametrize("kw", [dict(plane=False), dict(accum="kahan32"), dict()])
+def test_fixed_axis_beyond_the_exact_floors(kw):
+    """x = 0 lies at index 4,500,001 of the x axis; the adjoint too."""
+    n, dq = 4500010, 1e-4
+    qx = (np.arange(n) - 4500001.5) * dq
+    shape = (2, n, 2)
+    iq = np.random.default_rng(1).random(shape)
+    psis = np.linspace(0.0, 90.0, 7)
+    g = np.random.default_rng(2).standard_normal((64, 64))
+    img, adj = [], []
+    # (dq is the z axis': 2 voxels a side along y and z)
+    qz = np.array([-dq, 0.0])
+    for plan in plans(shape, (qx, qz, qz), psis, **kw):
+        try:
+            plan.set_iq(iq)
+            plan.execute()
+            img.append(plan.result())
+            adj.append(plan.backward(g))
+        finally:
+            plan.close()
+    assert np.allclose(img[0], img[1], rtol=1e-6, atol=0)
+    assert np.array_equal(adj[0] != 0, adj[1] != 0)
+    assert np.allclose(adj[0], adj[1], rtol=1e-9, atol=1e-15)
