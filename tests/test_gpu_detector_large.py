@@ -42,3 +42,31 @@ def test_fixed_axis_beyond_the_exact_floors(kw):
     assert np.allclose(img[0], img[1], rtol=1e-6, atol=0)
     assert np.array_equal(adj[0] != 0, adj[1] != 0)
     assert np.allclose(adj[0], adj[1], rtol=1e-9, atol=1e-15)
+
+
+def test_plane_of_lines_far_apart():
+    """nx nz float64 values between the lines of the plane: more bytes than the
+    pitch of a 2-D copy holds."""
+    ny, nx, nz = 3, 16385, 16390
+    assert nx * nz * 8 > 2 ** 31
+    iq = np.zeros((ny, nx, nz))  # (only the plane's pages are ever touched)
+    fixed = 7
+    iq[:, fixed, :] = np.random.default_rng(3).random((ny, nz))
+    dq = 1e-4
+    qx = (np.arange(nx) - fixed - 0.5) * dq
+    qy = np.array([-1.5, -0.5, 0.5]) * dq
+    qz = (np.arange(nz) - nz / 2) * dq
+    psis = np.linspace(0.0, 90.0, 5)
+    w = np.full(5, 0.2)
+    plan = F.DetectorPlan(iq.shape, qx, qy, qz, 64, 1.0, (), (), psis, w, [0.0], [1.0], [0.0],
+                          [1.0], mirror=False)
+    try:
+        plan.set_iq(iq)
+        plan.execute()
+        img = plan.result()
+        idx = [plan.debug_indices(o) for o in range(5)]
+    finally:
+        plan.close()
+    want = sum(0.2 * iq.reshape(-1)[i] for i in idx).reshape(64, 64)
+    want = np.where(want <= 0, 1e-6, want) * 1e-6
+    assert np.allclose(img, want, rtol=1e-6, atol=0)
