@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gw_common.cuh"
@@ -436,8 +437,10 @@ static_assert(sizeof(GenOrient) == 96, "six 16-byte words per orientation");
 // fewer than 2^32 elements).  Tiles keep a block's samples of one orientation
 // within a small patch of the volume.  Bound by issue.  2880 orientations of
 // 500 x 500 pixels in 203^3: 4.75 ms with one axis at a time, rows of 512
-// pixels a block and 64-bit indices, 1.20 ms so.
-template <bool ZX, bool KAHAN>
+// pixels a block and 64-bit indices, 1.20 ms so.  WIDE: 64-bit indices, for I(q)
+// of 2^32 elements and more (320 orientations of 500 x 500 pixels in 1626^3: 0.63 ms
+// so, 8.30 with every sample's exact index; in 1600^3 0.56).
+template <bool ZX, bool KAHAN, bool WIDE>
 __global__ void __launch_bounds__(kPlThreads)
 k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, int *wl_count,
                    int wl_cap) {
@@ -450,7 +453,8 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
   const int ib = (blockIdx.x / tiles_x) * kPlTile + tile_row(threadIdx.x);
   const float mx = (float)(a.nx - 1), my = (float)(a.ny - 1), mz = (float)(a.nz - 1);
   const unsigned nx = a.nx, nz = a.nz;
-  const unsigned base = (0x4B400000u * nx + 0x4B400000u) * nz + 0x4B400000u;
+  constexpr unsigned kBits = 0x4B400000u;  // kMagic's
+  const unsigned base = (kBits * nx + kBits) * nz + kBits;
   int pix[KP];
   bool valid[KP];
   float xf[KP], yf[KP], zf[KP], part[KP], kc[KP];
@@ -492,7 +496,8 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
       for (int oo = g0; oo < ge; oo += kPlBatch) {
         // every index is clamped, so the samples of kPlBatch orientations are
         // loaded unconditionally, all in flight at once
-        unsigned at[kPlBatch][KP], ok = 0;
+        std::conditional_t<WIDE, int64_t, unsigned> at[kPlBatch][KP];
+        unsigned ok = 0;
         float w[kPlBatch], v[kPlBatch][KP];
 #pragma unroll
         for (int b = 0; b < kPlBatch; ++b) {
@@ -522,8 +527,12 @@ k_detector_general(DetArgs a, const GenOrient *ot, double *acc_out, int2 *wl, in
             const float2 fl = f2_sub(r, mg);
             const bool in = (fmaxf(lo.x, 0.f) >= fl.x) & (fmaxf(lo.y, 0.f) >= fl.y) &
                             (fmaxf(k ? zlo.y : zlo.x, 0.f) >= (k ? zfl.y : zfl.x));
-            at[b][k] = (__float_as_uint(r.y) * nx + __float_as_uint(r.x)) * nz +
-                       __float_as_uint(k ? zr.y : zr.x) - base;
+            const unsigned ry = __float_as_uint(r.y), rx = __float_as_uint(r.x),
+                           rz = __float_as_uint(k ? zr.y : zr.x);
+            if constexpr (WIDE)
+              at[b][k] = ((int64_t)(ry - kBits) * nx + (rx - kBits)) * nz + (rz - kBits);
+            else
+              at[b][k] = (ry * nx + rx) * nz + rz - base;
             ok |= (unsigned)in << (b * KP + k);
           }
         }
@@ -1051,12 +1060,19 @@ void launch_general(gw_detector_plan *P, const DetArgs &a) {
     kernel<<<tiles, kPlThreads, 0, P->ctx->stream>>>(a, P->d_go, P->d_acc, P->d_wl,
                                                      P->d_wl_count, P->wl_cap);
   };
-  if (P->p.accum == GW_ACCUM_KAHAN32)
-    P->zero_x ? run(k_detector_general<true, true>)
-              : run(k_detector_general<false, true>);
-  else
-    P->zero_x ? run(k_detector_general<true, false>)
-              : run(k_detector_general<false, false>);
+  const bool kahan = P->p.accum == GW_ACCUM_KAHAN32;
+  // (the 32-bit gather index holds volumes of fewer than 2^32 elements)
+  if ((double)a.nx * a.ny * a.nz >= 4294967296.0) {
+    if (kahan) P->zero_x ? run(k_detector_general<true, true, true>)
+                         : run(k_detector_general<false, true, true>);
+    else P->zero_x ? run(k_detector_general<true, false, true>)
+                   : run(k_detector_general<false, false, true>);
+  } else {
+    if (kahan) P->zero_x ? run(k_detector_general<true, true, false>)
+                         : run(k_detector_general<false, true, false>);
+    else P->zero_x ? run(k_detector_general<true, false, false>)
+                   : run(k_detector_general<false, false, false>);
+  }
 }
 
 }  // namespace
@@ -1099,12 +1115,7 @@ extern "C" int gw_detector_execute(gw_detector_plan *P) {
       GW_LAUNCHED(P->ctx);
     } else {
       gw::KTimer tm(P->ctx, GW_K_DETECTOR);
-      // the 32-bit gather index holds volumes of up to 2^32 elements; larger
-      // ones replay every sample
-      if ((double)a.nx * a.ny * a.nz >= 4294967296.0)
-        k_detector<<<(npx + 127) / 128, 128, 0, P->ctx->stream>>>(a, P->d_acc);
-      else
-        launch_general(P, a);
+      launch_general(P, a);
       GW_LAUNCHED(P->ctx);
     }
     gw::KTimer tm(P->ctx, GW_K_DET_FIX);

@@ -70,3 +70,34 @@ def test_plane_of_lines_far_apart():
     want = sum(0.2 * iq.reshape(-1)[i] for i in idx).reshape(64, 64)
     want = np.where(want <= 0, 1e-6, want) * 1e-6
     assert np.allclose(img, want, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("accum", ["fp64", "kahan32"])
+@pytest.mark.parametrize("phis", [(0.0,), (0.0, 25.0, 71.0)])
+def test_volume_of_more_than_32_bit_indices(accum, phis):
+    """2^32 elements and more, the samples at the volume's end; the gather and
+    the exact path on the same device array."""
+    torch = pytest.importorskip("torch")
+    n = 1626
+    assert n ** 3 > 2 ** 32
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs a 17 GB array")
+    iq = torch.empty((n, n, n), dtype=torch.float32, device="cuda")
+    line = torch.arange(n * n, device="cuda", dtype=torch.int64).reshape(n, n)
+    for y in range(n):
+        iq[y] = ((line + 977 * y) % 1009).float()
+    torch.cuda.synchronize()
+    dq = 0.002
+    q = (np.arange(n) - 0.8 * n) * dq  # q = 0 (and the pixels) towards the end
+    img = []
+    for plan in plans((n, n, n), (q, q, q), np.linspace(0.0, 80.0, 5), phis, accum=accum,
+                      plane=False):
+        try:
+            plan.set_iq_device32(iq.data_ptr())
+            plan.execute()
+            img.append(plan.result())
+        finally:
+            plan.close()
+    del iq
+    torch.cuda.empty_cache()
+    assert np.allclose(img[0], img[1], rtol=1e-5, atol=0)
