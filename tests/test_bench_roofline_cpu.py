@@ -60,3 +60,16 @@ def test_traffic_table_covers_the_bench_plans():
         for k in ("row_czt", "col_czt_bin"):
             assert ("si-100A", k, 1280, 1024, real) in bench.NCU_TRAFFIC
             assert bench.NCU_TRAFFIC[("si-100A", k, 1280, 1024, real)] > 0
+
+
+def test_shared_roof_moves_one_trip_less():
+    """The bandwidth is of the bytes the Stockham kernels move: the last
+    forward and the first inverse pass are one trip (five of three passes a
+    side); the fused kernels keep the count of the passes."""
+    r = bench.shared_roof("row_czt", INFO, 180, 0.5)
+    moved = 180 * 207 * 5 * 1280 * 16
+    assert r["moved_bytes_per_launch"] == moved == r["bytes_per_launch"] * 5 / 6
+    assert abs(r["achieved"] * 1e12 * 0.5e-3 / moved - 1) < 1e-12
+    assert abs(r["frac"] * r["peak"] / r["achieved"] - 1) < 1e-12
+    c = bench.shared_roof("col_czt_bin", dict(INFO, fused_z=1), 180, 0.25)
+    assert c["moved_bytes_per_launch"] == c["bytes_per_launch"]
