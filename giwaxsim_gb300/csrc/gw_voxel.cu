@@ -1598,9 +1598,12 @@ int enqueue_prep(gw_voxel_plan *P) {
 // (the setup kernels and the row stage index them by batch slot).
 SliceArgs profile_view(const SliceArgs &a, int s0) {
   SliceArgs v = a;
-  v.amo = a.amo + (size_t)s0 * a.Ly;
-  if (a.pr) v.pr = a.pr + (size_t)s0 * a.Ly;
-  v.my = a.my + (size_t)s0 * a.Ly;
+  if (a.pr) {  // real grids
+    v.pr = a.pr + (size_t)s0 * a.Ly;
+  } else {
+    v.amo = a.amo + (size_t)s0 * a.Ly;
+    v.my = a.my + (size_t)s0 * a.Ly;
+  }
   v.mz = a.mz + (size_t)s0 * a.Lz;
   return v;
 }
@@ -1976,8 +1979,8 @@ struct PathParts {
   int Nf, S, f1_box_cols, n_heavy, n_zmulti;
   size_t bytes, path_bytes;
   CUtensorMap f1map;
-  float2 *F1, *pr;
-  float *G;
+  float2 *F1, *pr, *amo;
+  float *G, *my;
   int *lptr, *zptr, *zrows, *heavy, *zmulti;
   int2 *lent;
   std::vector<int> h_heavy;
@@ -1986,29 +1989,38 @@ struct PathParts {
       : real(P->real), gather(P->gather), f1_tma(P->f1_tma), Nf(P->Nf), S(P->S),
         f1_box_cols(P->f1_box_cols), n_heavy(P->n_heavy), n_zmulti(P->n_zmulti),
         bytes(P->bytes), path_bytes(P->path_bytes), f1map(P->f1map), F1(P->d_F1),
-        pr(P->d_pr), G(P->d_G), lptr(P->d_lptr), zptr(P->d_zptr), zrows(P->d_zrows),
-        heavy(P->d_heavy), zmulti(P->d_zmulti), lent(P->d_lent), h_heavy(P->h_heavy) {}
+        pr(P->d_pr), amo(P->d_amo), G(P->d_G), my(P->d_my), lptr(P->d_lptr), zptr(P->d_zptr),
+        zrows(P->d_zrows), heavy(P->d_heavy), zmulti(P->d_zmulti), lent(P->d_lent),
+        h_heavy(P->h_heavy) {}
   void restore(gw_voxel_plan *P) const {
     P->real = real; P->gather = gather; P->f1_tma = f1_tma;
     P->Nf = Nf; P->S = S; P->f1_box_cols = f1_box_cols;
     P->n_heavy = n_heavy; P->n_zmulti = n_zmulti;
     P->bytes = bytes; P->path_bytes = path_bytes; P->f1map = f1map;
-    P->d_F1 = F1; P->d_pr = pr; P->d_G = G; P->d_lptr = lptr; P->d_zptr = zptr;
-    P->d_zrows = zrows; P->d_heavy = heavy; P->d_zmulti = zmulti; P->d_lent = lent;
+    P->d_F1 = F1; P->d_pr = pr; P->d_amo = amo; P->d_my = my; P->d_G = G;
+    P->d_lptr = lptr; P->d_zptr = zptr; P->d_zrows = zrows;
+    P->d_heavy = heavy; P->d_zmulti = zmulti; P->d_lent = lent;
     P->h_heavy = h_heavy;
   }
   void free() const {
-    void *ptrs[] = {F1, pr, G, lptr, zptr, zrows, heavy, zmulti, lent};
+    void *ptrs[] = {F1, pr, amo, my, G, lptr, zptr, zrows, heavy, zmulti, lent};
     for (void *q : ptrs) gw::dev_free(q);
   }
 };
 
-// F1 and, on real grids, the row kernel's table, the tensor map, then the
-// gather's tables (the column and row tables are made).
+// F1, the slices' fill and y smoothing profiles (real grids: the row kernel's table
+// of both), the tensor map, then the gather's tables (the column and row tables are
+// made).
 int path_buffers(gw_voxel_plan *P, const char *who) {
   const size_t before = P->bytes;
   GW_TRY(alloc(&P->d_F1, (size_t)P->S * P->Lz * P->Nf, &P->bytes));
-  if (P->real) GW_TRY(alloc(&P->d_pr, (size_t)P->n_slices * P->Ly, &P->bytes));
+  const size_t profile = (size_t)P->n_slices * P->Ly;
+  if (P->real) {
+    GW_TRY(alloc(&P->d_pr, profile, &P->bytes));
+  } else {
+    GW_TRY(alloc(&P->d_amo, profile, &P->bytes));
+    GW_TRY(alloc(&P->d_my, profile, &P->bytes));
+  }
   GW_TRY(col_map_dispatch(P));
   GW_TRY(gather_setup(P, who));
   P->path_bytes = P->bytes - before;
@@ -2373,8 +2385,6 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_rowstart, (size_t)n_struct * (g + 2), &B)) ||
       (st = alloc(&P->d_cursor, (size_t)n_struct * (g + 1), &B)) ||
       (st = alloc(&P->d_zstat, n_struct, &B)) ||
-      (st = alloc(&P->d_amo, (size_t)P->n_slices * P->Ly, &B)) ||
-      (st = alloc(&P->d_my, (size_t)P->n_slices * P->Ly, &B)) ||
       (st = alloc(&P->d_mz, (size_t)P->n_slices * P->Lz, &B)) ||
       (st = upload(&P->d_roff, P->roff_host, &B))) {
     gw_voxel_plan_destroy(P);

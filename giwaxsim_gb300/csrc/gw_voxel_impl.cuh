@@ -269,12 +269,11 @@ __device__ __forceinline__ RowConst row_const(const SliceArgs &a, int slot,
 struct RowValueArgs {
   const float2 *amo;
   const float *my;
-  const float2 *pr;
   int fill, smooth_on, y_lo, g, Ly;
 };
 
 __device__ __forceinline__ RowValueArgs row_value_args(const SliceArgs &a) {
-  return RowValueArgs{a.amo, a.my, a.pr, a.fill, a.smooth_on, a.y_lo, a.g, a.Ly};
+  return RowValueArgs{a.amo, a.my, a.fill, a.smooth_on, a.y_lo, a.g, a.Ly};
 }
 
 __device__ __forceinline__ float2 d_value_row(const RowValueArgs &a,

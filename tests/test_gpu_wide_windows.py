@@ -119,14 +119,14 @@ def test_failed_change_of_path_leaves_the_plan(binning):
             failed += 1
             plan.execute()
             assert rel_l2(plan.iq(), ref) <= RTOL
-        assert failed == (1 if binning == "atomic" else 10)
+        assert failed == (3 if binning == "atomic" else 12)
         after = plan.info()
-        if binning == "atomic":  # F1 in and out, the row table out
+        if binning == "atomic":  # F1 in and out, the row table out, the profiles in
             a, b = before, after
             nf = a["Nc"] + a["k0"]  # columns ky >= 0
             assert b["device_bytes"] - a["device_bytes"] == 8 * (
                 b["batch"] * b["Lz"] * b["Nc"] - a["batch"] * a["Lz"] * nf
-                - a["n_slices"] * a["Ly"])
+                - a["n_slices"] * a["Ly"]) + 12 * a["n_slices"] * a["Ly"]
         plan.execute()
         assert rel_l2(plan.iq(), ref) <= RTOL
     finally:
