@@ -34,8 +34,6 @@
 #include <vector>
 
 #include "gw_tma.cuh"
-#include <cooperative_groups.h>
-
 #include "gw_voxel_impl.cuh"
 
 using namespace gwv;
@@ -437,18 +435,17 @@ __device__ __forceinline__ void y_block_reduce(T (&lo)[S], T (&hi)[S]) {
 }
 
 // A structure of more than `share` candidates (a hollow one: most atoms are) has
-// its slices' candidates shared by the blocks of a cluster (y_share).
+// its slices' candidates shared by several blocks (y_share).
 __device__ __forceinline__ bool y_shared(const SliceArgs &a, int sl, int share) {
   return a.ncand[sl / a.n_phi] > share;
 }
 
 // The candidates i0, i0 + stride, .. of those of slices first .. first + ns - 1
-// that are shared (or are not), kYBatch of them at a time so that their gathers
-// are in flight together: each(sorted position, atom, first, end slice).  Where
-// most atoms are candidates, all atoms are taken instead, in order (coalesced,
-// without the list).
-constexpr int kYBatch = 4;
-template <class Each>
+// that are shared (or are not), B of them at a time so that their gathers are in
+// flight together: each(sorted position, atom, first, end slice).  Where most atoms
+// are candidates, all atoms are taken instead, in order (coalesced, without the
+// list).
+template <int B, class Each>
 __device__ __forceinline__ void y_candidates(const SliceArgs &a, int first, int ns, int share,
                                              bool shared, int i0, int stride, Each each) {
   for (int kb = 0, ke; kb < ns; kb = ke) {
@@ -460,40 +457,33 @@ __device__ __forceinline__ void y_candidates(const SliceArgs &a, int first, int 
     const int listed = a.ncand[t];
     const bool all = 2 * (int64_t)listed > atoms;
     const int nc = all ? atoms : listed;
-    int i = i0;
-    for (; i + (kYBatch - 1) * stride < nc; i += kYBatch * stride) {
-      int pos[kYBatch];
-      float4 q[kYBatch];
+    // (past the end: the last one again, which changes no extreme)
+    for (int i = i0; i < nc; i += B * stride) {
+      int pos[B];
+      float4 q[B];
 #pragma unroll
-      for (int b = 0; b < kYBatch; ++b) pos[b] = all ? begin + i + b * stride : cand[i + b * stride];
+      for (int b = 0; b < B; ++b) {
+        const int c = min(i + b * stride, nc - 1);
+        pos[b] = all ? begin + c : cand[c];
+      }
 #pragma unroll
-      for (int b = 0; b < kYBatch; ++b) q[b] = a.xyf_s[pos[b]];
+      for (int b = 0; b < B; ++b) q[b] = a.xyf_s[pos[b]];
 #pragma unroll
-      for (int b = 0; b < kYBatch; ++b) each(pos[b], q[b], kb, ke);
-    }
-    for (; i < nc; i += stride) {
-      const int pos = all ? begin + i : cand[i];
-      each(pos, a.xyf_s[pos], kb, ke);
+      for (int b = 0; b < B; ++b) each(pos[b], q[b], kb, ke);
     }
   }
 }
 
-// The extremes of those of slices first .. first + ns - 1 (at most S) that are
-// SHARED by the cluster's blocks (or are not), then, per slice, its background constants and the extents of the valid atoms
-// (voxelgrids.py:346-349): y indices grow with y (the floor division is
-// monotone), so when every atom is valid the extents are (0, index of max y, 0,
-// largest occupied z row); otherwise ext_exact computes them atom by atom.
-template <int S, bool SHARED>
-__device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns, int share) {
-  namespace cg = cooperative_groups;
-  __shared__ unsigned s_f[2][S];
+// Block `rank` of `blocks` over its share of the candidates of those of slices
+// first .. first + ns - 1 (at most S) that are shared (or are not): the least and
+// the largest y' of the share, in thread 0 (~0 and 0 without a candidate).
+template <int S>
+__device__ __forceinline__ void y_extremes(const SliceArgs &a, int first, int ns, int share,
+                                           bool shared, int rank, int blocks,
+                                           unsigned long long (&lo)[S],
+                                           unsigned long long (&hi)[S]) {
+  constexpr int kB = 2;
   __shared__ float s_b[2][S];
-  __shared__ unsigned long long s_d[2][S];
-  int rank = 0, blocks = 1;
-  if constexpr (SHARED) {
-    rank = cg::this_cluster().block_rank();
-    blocks = cg::this_cluster().num_blocks();
-  }
   float cf[S], sf[S];
   unsigned flo[S], fhi[S];  // ordered: min of (y'+d), max of (y'-d)
 #pragma unroll
@@ -505,7 +495,7 @@ __device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns,
     fhi[k] = 0u;
   }
   const int i0 = rank * blockDim.x + threadIdx.x, stride = blocks * blockDim.x;
-  y_candidates(a, first, ns, share, SHARED, i0, stride, [&](int, float4 q, int kb, int ke) {
+  y_candidates<kB>(a, first, ns, share, shared, i0, stride, [&](int, float4 q, int kb, int ke) {
 #pragma unroll
     for (int k = 0; k < S; ++k) {
       if (k < kb || k >= ke) continue;
@@ -519,25 +509,11 @@ __device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns,
   if (threadIdx.x == 0)
 #pragma unroll
     for (int k = 0; k < S; ++k) {
-      s_f[0][k] = flo[k];
-      s_f[1][k] = fhi[k];
+      s_b[0][k] = ord_flt(flo[k]);
+      s_b[1][k] = ord_flt(fhi[k]);
     }
-  if constexpr (SHARED) cg::this_cluster().sync();
-  else __syncthreads();
-  if (threadIdx.x < S) {
-    unsigned l = s_f[0][threadIdx.x], h = s_f[1][threadIdx.x];
-    if constexpr (SHARED)
-      for (int b = 0; b < blocks; ++b) {
-        const unsigned *f = cg::this_cluster().map_shared_rank(&s_f[0][0], b);
-        l = min(l, f[threadIdx.x]);
-        h = max(h, f[S + threadIdx.x]);
-      }
-    s_b[0][threadIdx.x] = ord_flt(l);
-    s_b[1][threadIdx.x] = ord_flt(h);
-  }
   __syncthreads();
   float blo[S], bhi[S];
-  unsigned long long lo[S], hi[S];
 #pragma unroll
   for (int k = 0; k < S; ++k) {
     blo[k] = s_b[0][k];
@@ -545,7 +521,7 @@ __device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns,
     lo[k] = ~0ULL;
     hi[k] = 0ULL;
   }
-  y_candidates(a, first, ns, share, SHARED, i0, stride, [&](int pos, float4 q, int kb, int ke) {
+  y_candidates<kB>(a, first, ns, share, shared, i0, stride, [&](int pos, float4 q, int kb, int ke) {
 #pragma unroll
     for (int k = 0; k < S; ++k) {
       if (k < kb || k >= ke) continue;
@@ -561,59 +537,40 @@ __device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns,
     }
   });
   y_block_reduce<S>(lo, hi);
-  if constexpr (SHARED) {
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int k = 0; k < S; ++k) {
-        s_d[0][k] = lo[k];
-        s_d[1][k] = hi[k];
-      }
-    cg::this_cluster().sync();
-    if (rank == 0 && threadIdx.x == 0)
-      for (int b = 1; b < blocks; ++b) {
-        const unsigned long long *d = cg::this_cluster().map_shared_rank(&s_d[0][0], b);
-#pragma unroll
-        for (int k = 0; k < S; ++k) {
-          lo[k] = min(lo[k], d[k]);
-          hi[k] = max(hi[k], d[S + k]);
-        }
-      }
-    cg::this_cluster().sync();  // (its shared memory stays until it is read)
-    if (rank != 0) return;
+}
+
+// One thread, from the extremes of slice sl's y': its background constants and the
+// extents of the valid atoms (voxelgrids.py:346-349): y indices grow with y (the
+// floor division is monotone), so when every atom is valid the extents are (0, index
+// of max y, 0, largest occupied z row); otherwise (true) ext_exact computes them
+// atom by atom.
+__device__ __forceinline__ bool y_finish(const SliceArgs &a, int sl, unsigned long long lo,
+                                         unsigned long long hi) {
+  const int t = sl / a.n_phi;
+  a.ymin_ord[sl] = lo;
+  // background constant C = avg_voxel_f * max_voxels (voxelgrids.py:358,365):
+  // Cbg is what the transformed window excludes (batched mode), Cd what
+  // stays inside it
+  const gw_structure s = a.st[t];
+  double cr = GW_DMUL(s.avg_f_re, s.max_voxels), ci = GW_DMUL(s.avg_f_im, s.max_voxels);
+  if (a.real) {  // real grids are in units of the structure's phase
+    cr = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im) * s.max_voxels;
+    ci = 0.0;
   }
-  if (threadIdx.x != 0) return;
-#pragma unroll
-  for (int k = 0; k < S; ++k) {
-    if (k >= ns || y_shared(a, first + k, share) != SHARED) continue;
-    const int sl = first + k, t = sl / a.n_phi;
-    a.ymin_ord[sl] = lo[k];
-    // background constant C = avg_voxel_f * max_voxels (voxelgrids.py:358,365):
-    // Cbg is what the transformed window excludes (batched mode), Cd what
-    // stays inside it
-    const gw_structure s = a.st[t];
-    double cr = GW_DMUL(s.avg_f_re, s.max_voxels), ci = GW_DMUL(s.avg_f_im, s.max_voxels);
-    if (a.real) {  // real grids are in units of the structure's phase
-      cr = sqrt(s.avg_f_re * s.avg_f_re + s.avg_f_im * s.avg_f_im) * s.max_voxels;
-      ci = 0.0;
-    }
-    const float2 cf = make_float2((float)cr, (float)ci);
-    const bool bg = !a.plain && (a.fill || a.smooth_on);
-    // the q = 0 pixel is by far the largest
-    const double g2 = (double)a.g * (double)a.g;
-    const double dr = bg ? cr * g2 : 0.0, di = bg ? ci * g2 : 0.0;
-    a.sdc[sl] = make_float4((float)dr, (float)di, (float)(dr - (float)dr), (float)(di - (float)di));
-    a.sconst[sl] = bg ? make_float4(cf.x, cf.y, 0.f, 0.f) : make_float4(0.f, 0.f, cf.x, cf.y);
-    const double Y = floor_div_exact(GW_DSUB(ord_dbl(hi[k]), ord_dbl(lo[k])), a.r, a.inv_r);
-    const int2 zs = a.zstat[t];
-    if (Y < (double)a.g && zs.y) {
-      a.ext[sl] = make_int4(0, (int)Y, 0, zs.x);
-      a.extflag[sl] = 0;
-    } else {
-      a.ext[sl] = make_int4(INT_MAX, -1, INT_MAX, -1);
-      a.extflag[sl] = 1;
-      *a.any_ext = 1;
-    }
-  }
+  const float2 cf = make_float2((float)cr, (float)ci);
+  const bool bg = !a.plain && (a.fill || a.smooth_on);
+  // the q = 0 pixel is by far the largest
+  const double g2 = (double)a.g * (double)a.g;
+  const double dr = bg ? cr * g2 : 0.0, di = bg ? ci * g2 : 0.0;
+  a.sdc[sl] = make_float4((float)dr, (float)di, (float)(dr - (float)dr), (float)(di - (float)di));
+  a.sconst[sl] = bg ? make_float4(cf.x, cf.y, 0.f, 0.f) : make_float4(0.f, 0.f, cf.x, cf.y);
+  const double Y = floor_div_exact(GW_DSUB(ord_dbl(hi), ord_dbl(lo)), a.r, a.inv_r);
+  const int2 zs = a.zstat[t];
+  const bool in = Y < (double)a.g && zs.y;
+  a.ext[sl] = in ? make_int4(0, (int)Y, 0, zs.x) : make_int4(INT_MAX, -1, INT_MAX, -1);
+  a.extflag[sl] = !in;
+  if (!in) *a.any_ext = 1;
+  return !in;
 }
 
 // The slices whose candidates are not shared; k_yrest does the others.  Bound by
@@ -622,16 +579,27 @@ __device__ __forceinline__ void y_extents(const SliceArgs &a, int first, int ns,
 // 12.3 us at four a block, 5.3 at one; 2880: 29.7 at four).
 // Over all atoms, with a reset and the extents in launches of their own, 16 boxes
 // of 57,000 atoms at 180 angles each took 389 us, one of 13,713 at 180 angles 27
-// us and one of 264,424 at 720 angles 332 us; this and the extents take 39, 10 and
-// 26 us from cold caches (the candidate test costs k_zscatter 2-6 us a box of
-// these).
+// us and one of 264,424 at 720 angles 332 us; this and the extents take 33, 10 and 20 us
+// from cold caches (the candidate test costs k_zscatter 2-6 us a box of these).
 template <int S>
 __global__ void __launch_bounds__(256) k_yext(SliceArgs a, int slice0, int n, int share) {
   const int first = slice0 + blockIdx.x * S, ns = min(S, slice0 + n - first);
-  int shared = 0;
-  for (int k = 0; k < ns; ++k) shared += y_shared(a, first + k, share);
-  if (shared && threadIdx.x == 0) *a.any_ext = 1;
-  if (shared < ns) y_extents<S, false>(a, first, ns, share);
+  unsigned long long lo[S], hi[S];
+  y_extremes<S>(a, first, ns, share, false, 0, 1, lo, hi);
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int k = 0; k < S; ++k) {
+    if (k >= ns) continue;
+    const int sl = first + k;
+    if (y_shared(a, sl, share)) {  // (k_yrest adds its blocks' extremes up)
+      a.ymin_ord[sl] = ~0ULL;
+      a.ymax_ord[sl] = 0ULL;
+      a.ydone[sl] = 0;
+      *a.any_ext = 1;
+    } else {
+      y_finish(a, sl, lo[k], hi[k]);
+    }
+  }
 }
 
 // The extents of slice sl's valid atoms: share `part` of `parts` of the atoms.
@@ -671,30 +639,48 @@ __global__ void k_ext_exact(SliceArgs a, int slice0, int n) {
     if (a.extflag[sl]) ext_exact(a, sl, blockIdx.x, gridDim.x);
 }
 
-// The same for plans with a structure of more atoms than `share`, after the
-// extremes of the slices whose candidates are shared: a cluster takes S slices at
-// a time.  A tube of 264,000 atoms at 24 / 180 / 720 angles: 81 / 135 / 388 us
-// over all atoms, 903 / 906 / 1260 with one block for a slice (or four) that
-// gathers one candidate at a time, 51 / 116 / 307 so.
+// The same for plans with a structure of more atoms than `share`, and the extremes
+// of the slices whose candidates are shared: kYBlocks blocks take S slices at a time;
+// the last of them to add its extremes finishes the slices.  A tube of 264,000 atoms
+// at 24 / 180 / 720 angles: 81 / 135 / 388 us over all atoms, 903 / 906 / 1260 with
+// one block for a slice (or four) that gathers one candidate at a time, 64 / 120 /
+// 303 so.
 constexpr int kYBlocks = 8;
 template <int S>
-__global__ void __launch_bounds__(256) __cluster_dims__(kYBlocks, 1, 1)
-k_yrest(SliceArgs a, int slice0, int n, int share) {
-  namespace cg = cooperative_groups;
-  if (!*a.any_ext) return;  // (set before this launch; the same for every block)
-  const int rank = cg::this_cluster().block_rank();
-  for (int first = slice0 + blockIdx.x / kYBlocks * S; first < slice0 + n;
-       first += gridDim.x / kYBlocks * S) {
+__global__ void __launch_bounds__(256) k_yrest(SliceArgs a, int slice0, int n, int share) {
+  if (!*a.any_ext) return;
+  __shared__ bool s_flag[S];
+  const int rank = blockIdx.x;
+  for (int first = slice0 + blockIdx.y * S; first < slice0 + n; first += gridDim.y * S) {
     const int ns = min(S, slice0 + n - first);
     bool shared = false;
     for (int k = 0; k < ns; ++k) shared |= y_shared(a, first + k, share);
     if (shared) {
-      y_extents<S, true>(a, first, ns, share);
-      __threadfence();
-      cg::this_cluster().sync();  // (the flags are written, shared memory is free)
+      unsigned long long lo[S], hi[S];
+      y_extremes<S>(a, first, ns, share, true, rank, kYBlocks, lo, hi);
+      if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          s_flag[k] = false;
+          if (k >= ns || !y_shared(a, first + k, share)) continue;
+          const int sl = first + k;
+          atomicMin(a.ymin_ord + sl, lo[k]);
+          atomicMax(a.ymax_ord + sl, hi[k]);
+          __threadfence();
+          if (atomicAdd(a.ydone + sl, 1) == kYBlocks - 1) {
+            __threadfence();
+            s_flag[k] = y_finish(a, sl, __ldcg(a.ymin_ord + sl), __ldcg(a.ymax_ord + sl));
+          }
+        }
+      }
+      __syncthreads();
+      for (int k = 0; k < ns; ++k)
+        if (s_flag[k]) ext_exact(a, first + k, 0, 1);
+      __syncthreads();
     }
     for (int k = 0; k < ns; ++k)
-      if (__ldcg(a.extflag + first + k)) ext_exact(a, first + k, rank, kYBlocks);
+      if (a.extflag[first + k] && !y_shared(a, first + k, share))
+        ext_exact(a, first + k, rank, kYBlocks);
   }
 }
 
@@ -1527,6 +1513,7 @@ SliceArgs slice_args(gw_voxel_plan *P) {
   a.roff = P->d_roff;
   a.zstat = P->d_zstat; a.extflag = P->d_extflag;
   a.ph = P->d_phis; a.clbase = P->d_clbase; a.ymin_ord = P->d_ymin;
+  a.ymax_ord = P->d_ymax; a.ydone = P->d_ydone;
   a.ext = P->d_ext; a.amo = P->d_amo; a.my = P->d_my; a.pr = P->d_pr;
   a.mz = P->d_mz; a.gw = P->d_gw; a.sconst = P->d_sconst; a.sdc = P->d_sdc; a.err = P->ctx->d_err;
   return a;
@@ -1609,11 +1596,14 @@ SliceArgs profile_view(const SliceArgs &a, int s0) {
 }
 
 // Candidates of a structure that one block still takes alone, with n slices at
-// once: the fewer blocks the slices give, the sooner a cluster shares them (tubes:
-// 57,000 atoms at 180 angles 46 us shared, 212 not; 14,000 at 720 angles 72 and 52,
-// at 2880 235 and 101).
+// once: the fewer blocks the slices give, the sooner several share them (tubes, all
+// set-up launches: 57,000 atoms at 180 angles 54 us shared, 212 not; whole passes of
+// 5,000 at 180 angles 81 and 65, of 14,000 at 720 212 and 199, at 2880 717 and 579).
 static int y_share(const gw_ctx *ctx, int n) {
-  return n > 16 * ctx->sm_count ? INT_MAX : n > 4 * ctx->sm_count ? 16384 : 4096;
+  return n > 16 * ctx->sm_count  ? INT_MAX
+         : n > 4 * ctx->sm_count ? 16384
+         : n > ctx->sm_count     ? 8192
+                                 : 4096;
 }
 
 int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n) {
@@ -1633,10 +1623,10 @@ int enqueue_slice_setup(gw_voxel_plan *P, const SliceArgs &a, int s0, int n) {
     gw::KTimer tm(ctx, GW_K_DEPOSIT);
     if (max_atoms <= share)
       k_ext_exact<<<dim3(std::min(atom_blocks(P), 16), std::min(n, 64)), 256, 0, st>>>(a, s0, n);
-    else if (n > ctx->sm_count)  // (clusters of four slices each fill the GPU)
-      k_yrest<4><<<std::min((n + 3) / 4, 128) * kYBlocks, 256, 0, st>>>(a, s0, n, share);
+    else if (n > ctx->sm_count)  // (groups of four slices fill the GPU)
+      k_yrest<4><<<dim3(kYBlocks, std::min((n + 3) / 4, 128)), 256, 0, st>>>(a, s0, n, share);
     else
-      k_yrest<1><<<std::min(n, 128) * kYBlocks, 256, 0, st>>>(a, s0, n, share);
+      k_yrest<1><<<dim3(kYBlocks, std::min(n, 128)), 256, 0, st>>>(a, s0, n, share);
     GW_LAUNCHED(ctx);
   }
   if (a.fill || a.smooth_on) {
@@ -2379,6 +2369,7 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_iq64, P->iq_stride * P->n_out, &B)) ||
       (st = alloc(&P->d_iq32, P->iq_stride * P->n_out, &B)) ||
       (st = alloc(&P->d_dirs, (size_t)n_struct * kDirs, &B)) ||
+      (st = alloc(&P->d_ymax, P->n_slices, &B)) || (st = alloc(&P->d_ydone, P->n_slices, &B)) ||
       (st = alloc(&P->d_ncand, n_struct, &B)) || (st = alloc(&P->d_any_ext, 1, &B)) ||
       (st = alloc(&P->d_extflag, P->n_slices, &B)) ||
       (st = alloc(&P->d_zhist, (size_t)n_struct * (g + 1), &B)) ||
@@ -2428,7 +2419,8 @@ extern "C" int gw_voxel_plan_destroy(gw_voxel_plan *P) {
                   P->d_C2, P->d_sum, P->d_sumk, P->d_f0, P->d_iq64,
                   P->d_iq32, P->d_F1, P->d_amo, P->d_my, P->d_mz,
                   P->d_sconst, P->d_sdc, P->d_xyz_s, P->d_xyf_s, P->d_fz_s,
-                  P->d_perm, P->d_cand, P->d_dirs, P->d_ncand, P->d_any_ext, P->d_roff, P->d_zhist, P->d_rowstart,
+                  P->d_perm, P->d_cand, P->d_dirs, P->d_ncand, P->d_ymax, P->d_ydone,
+                  P->d_any_ext, P->d_roff, P->d_zhist, P->d_rowstart,
                   P->d_cursor, P->d_zstat, P->d_extflag,
                   P->d_shell, P->d_f_shells, P->d_structs_shells, P->d_zf0,
                   P->d_fty, P->d_ftz, P->d_G, P->d_lptr, P->d_lent, P->d_zptr,

@@ -50,7 +50,8 @@ struct SliceArgs {
   const gw_structure *st;
   const gw_phi *ph;
   const double *clbase;  // per slice
-  unsigned long long *ymin_ord;
+  unsigned long long *ymin_ord, *ymax_ord;
+  int *ydone;            // per slice: blocks of k_yrest that added their extremes
   int *extflag;          // per slice: 1 = extents need the exact pass
   int *any_ext;          // some slice of the pass needs it
   int4 *ext;  // y_min, y_max, z_min, z_max (valid atoms)
@@ -657,6 +658,8 @@ struct gw_voxel_plan {
   bool sorted_real = false;    // d_xyf_s was made for real grids
   int *d_cand = nullptr;       // candidates for the y extremes (sorted positions)
   int *d_ncand = nullptr, *d_any_ext = nullptr;
+  unsigned long long *d_ymax = nullptr;  // with d_ydone: k_yrest
+  int *d_ydone = nullptr;
   bool f_unseen = false;       // no execute has looked at the atoms' f values
   unsigned long long *d_dirs = nullptr;  // per structure: outermost atoms
   std::vector<int> roff_host;  // per-slice first window row (n_slices+1)

@@ -1,7 +1,7 @@
 """The y extremes at the block shapes the other tests do not reach: four
 slices a block (more slices than four a multiprocessor) with blocks that hold
 the slices of two or three structures and a partial last one, and a slice's
-candidates shared by a cluster of blocks (hollow structures: most atoms are
+candidates shared by several blocks (hollow structures: most atoms are
 candidates), with structures on both sides of the line in one plan.  Deposit
 indices bit-exact against the oracle."""
 import numpy as np
@@ -20,8 +20,9 @@ def structure(shape, n):
         return rng.uniform(0.0, 1.0, (n, 3)) * [14.0, 11.0, 9.0] + [40.0, -50.0, 7.0]
     if shape == "tall":  # higher and wider than the grid: atoms outside it
         return rng.uniform(0.0, 1.0, (n, 3)) * [30.0, 45.0, 60.0]
-    a = rng.uniform(0.0, 2 * np.pi, n)  # tube: every atom on the hull
-    return np.stack([6.0 * np.cos(a), 6.0 * np.sin(a), rng.uniform(0.0, 9.0, n)], axis=1)
+    a = rng.uniform(0.0, 2 * np.pi, n)  # tube: every atom on the hull; pipe: wider
+    R0 = 6.0 if shape == "tube" else 25.0  # than the grid
+    return np.stack([R0 * np.cos(a), R0 * np.sin(a), rng.uniform(0.0, 9.0, n)], axis=1)
 
 
 def multiprocessors():
@@ -34,6 +35,7 @@ def multiprocessors():
     [("box", 700), ("tube", 2500), ("box", 9001), ("box", 5)],   # many-block preparation
     [("tube", 4096), ("box", 6000), ("tube", 4097), ("tube", 12301), ("box", 40)],
     [("box", 50), ("tube", 17001), ("tall", 16385)],
+    [("pipe", 17003), ("box", 5000), ("pipe", 300)],
     [("tube", 4097)]])
 @pytest.mark.parametrize("per_sm", [0, 2, 4])
 def test_blocks_of_slices_vs_oracle(shapes, per_sm):
