@@ -418,14 +418,16 @@ class VoxelPlan:
             len(self.structs), N.ptr(self.phi_tab), len(self.phi_tab),
             ctypes.byref(h)))
         self.handle = h
-        self._wide = bool(self.params.real_grids) and self.info()["wide_real"] == 1
 
     @property
     def graph_captured(self):
         """A captured graph runs the executes (a wide real-grid plan drops
         it when it goes on on the general path)."""
-        return self._graph and not (getattr(self, "_wide", False)
-                                    and self.info()["graph_kernels"] == 0)
+        if self._graph and getattr(getattr(self, "params", None), "real_grids", 0):
+            v = (ctypes.c_int64 * 15)()  # (the last one: graph_kernels)
+            N.lib().gw_voxel_info(self.handle, v, 15)
+            return v[14] > 0
+        return self._graph
 
     @graph_captured.setter
     def graph_captured(self, on):
