@@ -2369,7 +2369,6 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_iq64, P->iq_stride * P->n_out, &B)) ||
       (st = alloc(&P->d_iq32, P->iq_stride * P->n_out, &B)) ||
       (st = alloc(&P->d_dirs, (size_t)n_struct * kDirs, &B)) ||
-      (st = alloc(&P->d_ymax, P->n_slices, &B)) || (st = alloc(&P->d_ydone, P->n_slices, &B)) ||
       (st = alloc(&P->d_ncand, n_struct, &B)) || (st = alloc(&P->d_any_ext, 1, &B)) ||
       (st = alloc(&P->d_extflag, P->n_slices, &B)) ||
       (st = alloc(&P->d_zhist, (size_t)n_struct * (g + 1), &B)) ||
@@ -2377,7 +2376,8 @@ extern "C" int gw_voxel_plan_create(gw_ctx *ctx, const gw_voxel_params *p,
       (st = alloc(&P->d_cursor, (size_t)n_struct * (g + 1), &B)) ||
       (st = alloc(&P->d_zstat, n_struct, &B)) ||
       (st = alloc(&P->d_mz, (size_t)P->n_slices * P->Lz, &B)) ||
-      (st = upload(&P->d_roff, P->roff_host, &B))) {
+      (st = upload(&P->d_roff, P->roff_host, &B)) ||
+      (st = alloc(&P->d_ymax, P->n_slices, &B)) || (st = alloc(&P->d_ydone, P->n_slices, &B))) {
     gw_voxel_plan_destroy(P);
     return st;
   }
