@@ -2598,7 +2598,7 @@ struct FLook {
     if (!on) return GW_OK;
     GW_CUDA(cudaEventSynchronize(P->ctx->answer_ev));
     bad = *static_cast<volatile int *>(P->ctx->h_answer) != 0;
-    P->f_unseen = false;
+    P->f_unseen = bad;  // (asked again should the change of path fail)
     return GW_OK;
   }
 };

@@ -320,6 +320,18 @@ def test_other_f_values_on_the_device(which, capture):
                     assert e.value.status == N.GW_ERR_STATE and plan.info()["real"] == 1
             plan.set_atoms(x.data_ptr(), bad.data_ptr(), on_device=True)
             if capture:
+                if real is None:
+                    N.set_alloc_fault(0)
+                    try:
+                        with pytest.raises(N.GwError) as e:
+                            plan.capture_graph()
+                        assert e.value.status == N.GW_ERR_OOM
+                        with pytest.raises(N.GwError) as e:
+                            plan.execute()  # (looks again)
+                        assert e.value.status == N.GW_ERR_OOM
+                    finally:
+                        N.set_alloc_fault(-1)
+                    plan.set_atoms(x.data_ptr(), bad.data_ptr(), on_device=True)
                 plan.capture_graph()
                 assert plan.info()["real"] == 0
             plan.execute()
