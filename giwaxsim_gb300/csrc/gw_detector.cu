@@ -976,7 +976,8 @@ extern "C" int gw_detector_plan_destroy(gw_detector_plan *P) {
 // its lines are nz contiguous elements, and one 2-D copy takes them alone.
 // 403^3 float64 from pageable memory, x fixed: 1.3 of 524 MB, a call of
 // detectormaker_fitting (1000 px, 91 psi) without the 3.0 ms of upload and
-// conversion (8.6 -> 0.63 ms with the orientation matrices made at once).
+// conversion (8.6 ms before, 0.6 to 1.2 by host with the orientation matrices made
+// at once).
 static int set_iq_plane(gw_detector_plan *P, const double *iq, int32_t on_device) {
   const PlaneArgs &pa = P->plane;
   const size_t nx = P->p.iq_shape[1], nz = P->p.iq_shape[2];
