@@ -13,7 +13,6 @@
 // rotations (angle 0) are dropped by the host, which leaves every bit
 // unchanged.
 #include <algorithm>
-#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -986,14 +985,9 @@ static int set_iq_plane(gw_detector_plan *P, const double *iq, int32_t on_device
   const size_t pitch = (pa.fa == 0 ? nx * nz : nz) * sizeof(double);
   if (!P->d_plane64)
     GW_CUDA(gw::dev_malloc((void **)&P->d_plane64, (size_t)pa.nu * line));
-  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (pitch <= INT_MAX) {
-    GW_CUDA(cudaMemcpy2DAsync(P->d_plane64, line, src, pitch, line, pa.nu, kind, P->ctx->stream));
-  } else {  // (more than a 2-D copy's pitch: line by line)
-    for (int u = 0; u < pa.nu; ++u)
-      GW_CUDA(cudaMemcpyAsync(P->d_plane64 + (size_t)u * pa.nv, src + u * (pitch / sizeof(double)),
-                              line, kind, P->ctx->stream));
-  }
+  GW_CUDA(cudaMemcpy2DAsync(P->d_plane64, line, src, pitch, line, pa.nu,
+                            on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                            P->ctx->stream));
   // the caller's array is free to change on return
   if (!on_device) GW_CUDA(cudaStreamSynchronize(P->ctx->stream));
   P->iq = nullptr;

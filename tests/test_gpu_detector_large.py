@@ -1,6 +1,6 @@
 """The detector gather at the limits of its index arithmetic: an axis fixed at
-an index beyond the float32 floors' range, a plane whose line pitch a 2-D copy
-does not take, and a volume of more than 2^32 elements, against the exact path
+an index beyond the float32 floors' range, a plane of lines more than 2^31 bytes
+apart, and a volume of more than 2^32 elements, against the exact path
 (float64 indices of every sample)."""
 import numpy as np
 import pytest
@@ -45,8 +45,8 @@ def test_fixed_axis_beyond_the_exact_floors(kw):
 
 
 def test_plane_of_lines_far_apart():
-    """nx nz float64 values between the lines of the plane: more bytes than the
-    pitch of a 2-D copy holds."""
+    """nx nz float64 values between the lines of the plane: more bytes than
+    cudaDeviceProp::memPitch, which the plane's 2-D copy takes all the same."""
     ny, nx, nz = 3, 16385, 16390
     assert nx * nz * 8 > 2 ** 31
     iq = np.zeros((ny, nx, nz))  # (only the plane's pages are ever touched)
